@@ -192,22 +192,43 @@ int validate_geom(const jpet_strip_geom* geom, std::string& msg) {
   return JPET_OK;
 }
 
+// The widest in-ellipse row is 2 * 3 sigma_z / sqrt(2) / pixel (+ rounding).
+int widest_row(const DevGeom& g) {
+  const double half = 3.0 * g.sigma_z / std::sqrt(2.0) / g.pixel_width;
+  return 2 * static_cast<int>(half) + 3;
+}
+
+// The batch-union kernel's batch shape for events of the given box rows (99.9 %
+// of them) and widest in-ellipse row, and what a CTA of that shape can hold: the
+// pixels of its windows (the largest that still let ctas_per_sm CTAs share an
+// SM's shared memory) and its largest chunk.  The smallest shape that leaves the
+// union of a batch a few rows and columns beyond its events' own; an explicit
+// CTA size selects the 64-row shapes.
+struct UnionLimits {
+  int shape, window_px, ctas_per_sm, max_chunk;
+};
+UnionLimits union_limits(const jpet_strip_opts& o, int rows, int widest) {
+  const UnionLimits m{kUnion64x32, 6144, 2, 2048};
+  if (o.block_threads == 128) return UnionLimits{kUnion64x32n4, 6144, 4, 2048};
+  if (o.block_threads == 256) return m;
+  if (rows <= 30 && widest <= 13) return UnionLimits{kUnion32x16, 3328, 5, 1024};
+  if (rows <= 30 && widest <= 28) return UnionLimits{kUnion32x32, 3328, 4, 1024};
+  return m;
+}
+
 // Window sizing: the largest box dimension that covers all but a tiny tail of
 // the events (the tail takes the global-memory path), then the largest square
 // tile whose window (tile + box) fits the shared-memory budget.
 void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
                    const std::vector<int32_t>& hh, int64_t n_nonempty, int n_sms, int n_y,
-                   int n_z, Tiling& t) {
+                   int n_z, int widest, Tiling& t) {
   // window pixels per array (rho, out): 12288 (~100 KiB per CTA, 2 CTAs per SM)
   // for 256-thread CTAs; 6144 (~55 KiB, 4 CTAs per SM) for the row-owned
-  // kernel's 128-thread CTAs and for the batch-union kernel (~76 KiB with its
-  // batch records, ~100 KiB with the compensation window, 2 CTAs of 256
-  // threads per SM)
+  // kernel's 128-thread CTAs; the batch-union kernel's from its batch shape
   const bool fast = o.mode == JPET_MODE_CPU_REFERENCE &&
                     (o.variant == JPET_VARIANT_FAST || o.variant == JPET_VARIANT_ROWS);
   const bool union_k = fast && o.variant == JPET_VARIANT_FAST;
   const bool rows4 = fast && o.block_threads != 256;
-  const int budget_px = (rows4 || union_k) ? 6144 : 12288;
   auto pct = [&](const std::vector<int32_t>& h, double keep) {
     int64_t tail = static_cast<int64_t>(std::floor((1.0 - keep) * n_nonempty));
     int64_t acc = 0;
@@ -217,6 +238,10 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
     }
     return 1;
   };
+  // batch shape of the batch-union kernel
+  const UnionLimits u = union_limits(o, pct(hh, 0.999), widest);
+  t.union_shape = u.shape;
+  const int budget_px = union_k ? u.window_px : (rows4 ? 6144 : 12288);
   int mw = std::min(255, std::max(1, pct(hw, 0.99999)));
   int mh = std::min(1024, std::max(1, pct(hh, 0.99999)));
   // shrink the box limits until at least an 8x8 tile fits
@@ -243,23 +268,22 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
   t.win_h = th + mh;
   t.n_tiles_x = (n_z + tw - 1) / tw;
   t.n_tiles_y = (n_y + th - 1) / th;
-  // events per chunk of the batch-union kernel: the largest of 2048, 1024 and
-  // 512 that still leaves at least 16 chunks per resident CTA (2 per SM).
+  // events per chunk of the batch-union kernel: the largest power of two (64 to
+  // 2048) that still leaves at least 16 chunks per resident CTA, or 4 below 512.
   // Larger chunks mean fewer chunk prologues and window flushes (2e7 events at
   // 2 mm: 13.50, 13.06, 12.88 ms per iteration with 512, 1024, 2048), but
-  // fewer chunks leave SMs idle at the end of the launch (event sets of ~8e5:
-  // 4.2e8, 4.0e8, 3.6e8 event-iterations/s).  The other kernels and the
-  // fixed-point mode (whose integer window sums must stay below 2^31) use 512.
+  // fewer chunks leave SMs idle at the end of the launch.  The fixed-point mode
+  // (whose integer window sums must stay below 2^31) takes at most 512, the
+  // other kernels 512.
   t.chunk_events = 512;
-  if (union_k && o.precision != JPET_PRECISION_FIXED) {
-    const int64_t min_chunks = 16LL * 2 * std::max(n_sms, 1);
-    t.chunk_events = 2048;
-    while (t.chunk_events > 512 && n_nonempty / t.chunk_events < min_chunks)
+  if (union_k) {
+    const int64_t resident = static_cast<int64_t>(u.ctas_per_sm) * std::max(n_sms, 1);
+    t.chunk_events = o.precision == JPET_PRECISION_FIXED ? 512 : u.max_chunk;
+    while (t.chunk_events > 64 &&
+           n_nonempty / t.chunk_events < (t.chunk_events > 512 ? 16 : 4) * resident)
       t.chunk_events /= 2;
   }
-  // the FP32 batch-union kernel (FAST variant) defaults to 256-thread CTAs
-  // (8 events per batch); the row-owned kernel to 128
-  t.threads = o.block_threads > 0 ? o.block_threads : (union_k ? 256 : (rows4 ? 128 : 256));
+  t.threads = o.block_threads > 0 ? o.block_threads : (rows4 ? 128 : 256);
   t.group = 32;
   // one spare entry per event for its widest row; a multiple of 8 entries so
   // that every event's table starts on a 16-byte boundary
@@ -271,11 +295,6 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
   t.rows_shape = kRowsShape4x1x3;
 }
 
-// The widest in-ellipse row is 2 * 3 sigma_z / sqrt(2) / pixel (+ rounding).
-int widest_row(const DevGeom& g) {
-  const double half = 3.0 * g.sigma_z / std::sqrt(2.0) / g.pixel_width;
-  return 2 * static_cast<int>(half) + 3;
-}
 int fast_width_shape(const DevGeom& g) {
   const int w = widest_row(g);
   return w <= 16 ? kShapeS : (w <= 24 ? kShapeM : kShapeL);
@@ -326,7 +345,7 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   int n_sms = 0;
   JPET_CUDA(h, cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, h->device),
             "cudaDeviceGetAttribute");
-  choose_tiling(h->opts, hw, hh, nonempty, n_sms, h->g.n_y, h->g.n_z, h->tiling);
+  choose_tiling(h->opts, hw, hh, nonempty, n_sms, h->g.n_y, h->g.n_z, widest_row(h->g), h->tiling);
   h->tiling.fast_shape = std::max(h->tiling.fast_shape, fast_width_shape(h->g));
   {
     int64_t tail = static_cast<int64_t>(std::floor(0.001 * nonempty)), acc_h = 0;
@@ -412,9 +431,9 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
       JPET_CUDA(h, h->batches.alloc(static_cast<size_t>(acc)), "cudaMalloc(batches)");
       JPET_CUDA(h, h->ev_const.alloc(static_cast<size_t>(acc) * union_event_bytes()),
                 "cudaMalloc(event constants)");
-      JPET_CUDA(h, h->union_rows.alloc(static_cast<size_t>(acc) * union_row_words()),
+      JPET_CUDA(h, h->union_rows.alloc(static_cast<size_t>(acc) * union_row_words(t)),
                 "cudaMalloc(union rows)");
-      JPET_CUDA(h, h->event_rows.alloc(static_cast<size_t>(acc) * union_row_words()),
+      JPET_CUDA(h, h->event_rows.alloc(static_cast<size_t>(acc) * union_row_words(t)),
                 "cudaMalloc(event rows)");
       JPET_CUDA(h, launch_union_setup(h->g, h->fc, t, h->chunks.p, h->n_chunks, acc,
                                       h->sorted_geom.p, h->sorted_box.p, h->row_table.p,

@@ -44,6 +44,16 @@ struct Tiling {
   int32_t row_stride;      // entries per event in the row table (>= max_box_h, even)
   int32_t fast_shape;      // register-cache shape of the warp-per-event kernel (FastShape)
   int32_t rows_shape;      // register-cache shape of the row-owned kernel (RowsShape)
+  int32_t union_shape;     // batch shape of the batch-union kernel (UnionShape)
+};
+
+// Batch shapes of the batch-union kernel: the largest union of a batch, window
+// rows x columns (strip_union_<shape>.cu).
+enum UnionShape : int32_t {
+  kUnion64x32 = 0,    // 8 warps, 8 events
+  kUnion64x32n4 = 1,  // 4 warps, 4 events
+  kUnion32x16 = 2,    // 4 warps, 8 events
+  kUnion32x32 = 3,    // 4 warps, 8 events
 };
 
 // Register-cache shapes of the fast iteration kernel: 4 lanes per image row,
@@ -163,19 +173,34 @@ cudaError_t sort_events(const Tiling& t, int64_t n, const float4* ev_geom, const
                         int64_t n_tile_events, int64_t n_over, float4* sorted_geom,
                         short4* sorted_box, float4* over_geom, short4* over_box,
                         cudaStream_t s);
-// Batch-union kernel (strip_union.cu): per-event constants and batches of up
-// to 4 (128-thread CTAs) or 8 (256-thread CTAs) similar events per chunk
-// (set-up), and the iteration over them in every accumulation mode (precision:
-// a FastPrecision code; aux: the second image of the compensated and
-// fixed-point modes; seed: the fixed-point dither's per-iteration seed).
+// Batch-union kernel (strip_union.cuh; set-up in strip_union.cu): per-event
+// constants and batches of similar events per chunk (set-up), and the iteration
+// over them in every accumulation mode (precision: a FastPrecision code; aux: the
+// second image of the compensated and fixed-point modes; seed: the fixed-point
+// dither's per-iteration seed).
+struct UnionOps {
+  int32_t threads, events, rows, cols;  // CTA, batch, largest union
+  size_t (*smem)(const Tiling& t, int precision);
+  cudaError_t (*prepare)(const Tiling& t, int precision);
+  cudaError_t (*launch)(const DevGeom& g, const FastConst& fc, const Tiling& t,
+                        const Chunk* chunks, int32_t n_chunks, const float4* ev_geom,
+                        const short4* ev_box, const void* ev_const, const uint16_t* erows,
+                        const uint16_t* urows, const uint32_t* batches, const float* rho,
+                        float* out, AuxImage aux, DevCounters* counters, int precision,
+                        uint32_t seed, cudaStream_t s);
+};
+const UnionOps& union_ops_64x32();
+const UnionOps& union_ops_64x32n4();
+const UnionOps& union_ops_32x16();
+const UnionOps& union_ops_32x32();
+const UnionOps& union_ops(int shape);
 size_t union_event_bytes();
 size_t union_smem_bytes(const Tiling& t, int precision);
-bool union_split_exponent(const DevGeom& g, const FastConst& fc);
 cudaError_t union_prepare_kernel(const Tiling& t, int precision);
 // union_row_words(): 16-bit words per event of the union-row and event-row
 // arrays (urows: per batch, indexed by the batch word's position; erows: per
 // event), written by launch_union_setup from the row table.
-size_t union_row_words();
+size_t union_row_words(const Tiling& t);
 cudaError_t launch_union_setup(const DevGeom& g, const FastConst& fc, const Tiling& t,
                                Chunk* chunks, int32_t n_chunks, int32_t n_events,
                                const float4* ev_geom, const short4* ev_box, const uint16_t* rows,

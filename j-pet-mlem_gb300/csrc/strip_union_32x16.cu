@@ -1,0 +1,12 @@
+// Batch-union iteration (strip_union.cuh) for batches of up to
+// 32 rows x 16 columns: 5 mm pixels at sigma 10 / 42.
+#include "strip_union.cuh"
+
+namespace jpet {
+
+const UnionOps& union_ops_32x16() {
+  static const UnionOps ops = UnionHost<UShape<4, 8, 2, 1, 5>>::ops();
+  return ops;
+}
+
+}  // namespace jpet
