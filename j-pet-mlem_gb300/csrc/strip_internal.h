@@ -44,6 +44,8 @@ struct Tiling {
   int32_t row_stride;      // entries per event in the row table (>= max_box_h, even)
   int32_t fast_shape;      // register-cache shape of the warp-per-event kernel (FastShape)
   int32_t rows_shape;      // register-cache shape of the row-owned kernel (RowsShape)
+  int32_t cell_w, cell_h;  // sort order: cells of the box corner inside the tile
+  int32_t tan_shift;       // sort order: tan buckets of 2^tan_shift / 512 (64 buckets at most)
   int32_t union_shape;     // batch shape of the batch-union kernel (UnionShape)
 };
 

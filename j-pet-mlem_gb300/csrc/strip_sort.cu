@@ -4,15 +4,15 @@
 // Key, most significant first: the image tile of the box's top-left corner
 // (the tile kernels' work unit; oversize boxes and empty boxes get two keys past
 // the last tile, so they end up behind the tile events, in that order); tan in
-// buckets of 1/8; the corner's row and column inside the tile; tan quantised to
-// 12 bits.  Within a tile, consecutive events then have nearly the same box,
-// slope and in-ellipse rows, which the batch-union kernel (strip_union.cu)
-// relies on: its batches of similar events share one lane-to-pixel map, and a
-// batch's per-row union is widest where its events' slopes differ (at the box's
-// top and bottom rows).  Bucketing tan ahead of the corner trades about one
-// pixel of corner spread for a much narrower slope spread where few events share
-// a corner pixel.  The order is deterministic (the sort is stable and the input
-// order is the caller's).
+// buckets; the cell of the corner inside the tile, cell row by cell row in
+// alternating direction; tan quantised to 12 bits.  Within a tile, consecutive
+// events then have nearly the same box, slope and in-ellipse rows, which the
+// batch-union kernel (strip_union.cuh) relies on: its batches of similar events
+// share one lane-to-pixel map, and a batch's per-row union is widest where its
+// events' slopes differ (at the box's top and bottom rows) or their corners do.
+// Cell size and bucket width trade the one spread for the other and depend on
+// how many events share a corner pixel (choose_tiling).  The order is
+// deterministic (the sort is stable and the input order is the caller's).
 #include <cuda_runtime.h>
 
 #include <cub/cub.cuh>
@@ -39,12 +39,13 @@ __global__ void sort_keys_kernel(Tiling t, int64_t n, const float4* __restrict__
     tile = n_tiles;
   } else {
     tile = static_cast<uint64_t>(b.y / t.tile_h) * t.n_tiles_x + static_cast<uint64_t>(b.x / t.tile_w);
-    ry = static_cast<uint64_t>(b.y % t.tile_h) & 255u;
-    rx = static_cast<uint64_t>(b.x % t.tile_w) & 255u;
+    ry = static_cast<uint64_t>(b.y % t.tile_h / t.cell_h) & 255u;
+    rx = static_cast<uint64_t>(b.x % t.tile_w / t.cell_w) & 255u;
+    if (ry & 1u) rx = 255u - rx;
     // fminf/fmaxf drop a NaN operand, so every tan maps into [0, 4095]
     const float q = fminf(fmaxf((ev_geom[i].z + 4.0f) * 512.0f, 0.0f), 4095.0f);
     tq = static_cast<uint64_t>(q);
-    tb = tq >> 6;
+    tb = tq >> t.tan_shift;
   }
   keys[i] = (tile << 34) | (tb << 28) | (ry << 20) | (rx << 12) | tq;
   idx[i] = static_cast<int32_t>(i);

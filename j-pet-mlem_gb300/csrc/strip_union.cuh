@@ -2,23 +2,21 @@
 // default kernel of every accumulation mode), and the set-up passes that feed
 // it.
 //
-// Events are sorted by image tile, then by tan in buckets of 1/8, their box
+// Events are sorted by image tile, then by tan in buckets, the cell of their box
 // corner inside the tile and tan (strip_sort.cu), so neighbouring events in a
 // chunk have nearly the same box and the same in-ellipse rows.  At set-up,
 // union_batches_kernel groups each chunk's events greedily into batches of up
-// to E consecutive events whose
-// union -- per window row, from the smallest first column (rounded down to
-// even) to the largest last column -- spans at most 64 rows and 32 columns, and
-// writes, per batch, each union row's start column and width and, per event
+// to E consecutive events whose union -- per window row, from the smallest first
+// column (rounded down to even) to the largest last column -- spans at most the
+// rows and columns of the shape (UShape; chosen from the events' boxes), and writes, per batch, each union row's start column and width and, per event
 // and union row, its in-ellipse interval relative to that start.  An event
 // that does not fit that rectangle on its own is rasterised in the reference's
 // order instead (the exact path); union_events_kernel stores each event's
 // constants (y, tan, exponent coefficients, window-relative box).
 //
-// The iteration kernel runs one CTA of NW warps per chunk (E = NW events per
-// batch), with the rho and back-projection windows of the tile in shared
-// memory.  For a batch, union row r belongs to the 4 lanes (gid) of one warp,
-// lane gl owning the pixel pairs 2 gl + 8 s (s < 4) of the row from its even
+// The iteration kernel runs one CTA of NW warps per chunk, with the rho and
+// back-projection windows of the tile in shared memory.  For a batch, union row r belongs to the 4 lanes (gid) of one warp,
+// lane gl owning the pixel pairs 2 gl + 8 s (s < SW) of the row from its even
 // start column: the SAME pixels for every event of the batch.  So rho is read
 // once per batch, each event's K rho stays in registers, and the
 // back-projection adds sum_e K_e rho inv_e to each owned pixel pair with one
@@ -40,9 +38,8 @@
 // Kernel value (src/2d/strip/gaussian_kernel.h:51-79, rewritten as in
 // strip_fast.cu): along a row the exponent of K / K_ref is p + q j + c j^2 with
 // c = kz pw^2.  With j counted from the union row's even start column and
-// jc = j - 16, K = 2^(p' + q' jc) * 2^(c jc^2); the second factor is the same
-// for every event, row and batch, so where it stays in range (|c| 16^2 <= 80,
-// e.g. 2 mm pixels at sigma_z 10: 15) it multiplies rho when rho is read
+// jc = j - kCols / 2, K = 2^(p' + q' jc) * 2^(c jc^2); the second factor is the same
+// for every event, row and batch, so where it stays in range (u_exponent_form) it multiplies rho when rho is read
 // (rho'' = rho 2^(c jc^2)) and a pixel costs one FFMA2 per pixel pair, one ex2
 // per pixel and one FMUL2; otherwise (coarse pixels, where 2^(c jc^2) would
 // underflow while 2^(p' + q' jc) overflows) the full exponent is evaluated,
@@ -50,22 +47,21 @@
 // every batch from the event's constants and the row (no per-row coefficient
 // table in memory).
 //
-// Chain form (the default where the row Gaussian spans several pixels,
-// |c| <= 0.06, e.g. 2 mm or 1 mm pixels at sigma_z = 5 pixels): along a row
+// Chain form (where the row Gaussian spans several pixels, e.g. 2 mm or 1 mm
+// pixels at sigma_z = 5 pixels: |c| = 0.058): along a row
 // K' = 2^(p' + q' jc) is geometric, so a lane evaluates two ex2 per event and
 // row (its first pixel pair) and steps to its next pair, 8 columns on, with one
 // FMUL2 by R8 = 2^(8 q') (computed once per event and row at set-up).  Every
-// K' a lane forms is a product of at most four rounded factors, within ~1e-6
-// of the direct value, and stays a normal float: a column of the union row is
-// at most ~43 pixels from the event's row peak, where 2^(c 43^2) >= 2^-111.
+// K' a lane forms is a product of at most SW rounded factors, within ~1e-6
+// of the direct value, and stays a normal float (u_exponent_form).
 // The masked K' stay in registers; the forward sum takes K' rho'' in one FFMA2
 // per pair, and the back-projection forms sum_e K'_e inv_e per pair and
 // multiplies by rho'' once per batch.
 //
 // Pixel set: exactly the reference's (gaussian_kernel.h:131-137 in its
 // rounding), from the exact per-row intervals of row_table_kernel: an event's
-// row interval [lo, hi) relative to the union start becomes a 32-bit column
-// mask (bit j = column j of the union row), tested once per pixel.
+// row interval [lo, hi) relative to the union start becomes a column mask (bit
+// j = column j of the union row), tested once per pixel.
 #pragma once
 
 #include <cuda_runtime.h>
