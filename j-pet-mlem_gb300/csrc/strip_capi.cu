@@ -203,7 +203,8 @@ int widest_row(const DevGeom& g) {
 // pixels of its windows (the largest that still let ctas_per_sm CTAs share an
 // SM's shared memory) and its largest chunk.  The smallest shape that leaves the
 // union of a batch a few rows and columns beyond its events' own; an explicit
-// CTA size selects the 64-row shapes.
+// CTA size selects the 64-row shapes.  Measured per iteration: 1e6 events of 26
+// rows x 11 columns (5 mm pixels) 552 us in the 64x32 shape, 294 in 32x16.
 struct UnionLimits {
   int shape, window_px, ctas_per_sm, max_chunk;
 };
@@ -213,6 +214,7 @@ UnionLimits union_limits(const jpet_strip_opts& o, int rows, int widest) {
   if (o.block_threads == 256) return m;
   if (rows <= 30 && widest <= 13) return UnionLimits{kUnion32x16, 3328, 5, 1024};
   if (rows <= 30 && widest <= 28) return UnionLimits{kUnion32x32, 3328, 4, 1024};
+  if (rows <= 64 && widest <= 13) return UnionLimits{kUnion64x16, 4096, 3, 1024};
   return m;
 }
 

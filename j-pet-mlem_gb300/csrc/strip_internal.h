@@ -56,6 +56,7 @@ enum UnionShape : int32_t {
   kUnion64x32n4 = 1,  // 4 warps, 4 events
   kUnion32x16 = 2,    // 4 warps, 8 events
   kUnion32x32 = 3,    // 4 warps, 8 events
+  kUnion64x16 = 5,    // 8 warps, 8 events
 };
 
 // Register-cache shapes of the fast iteration kernel: 4 lanes per image row,
@@ -154,6 +155,10 @@ cudaError_t launch_row_coefficients(const DevGeom& g, const FastConst& fc, const
                                     int32_t n_events, const float4* ev_geom,
                                     const short4* ev_box, const uint16_t* rows, float2* pq,
                                     uint32_t* row_pk, uint32_t* ev_pk, cudaStream_t s);
+// Raises a kernel's dynamic shared-memory limit to all that the current device
+// lets a CTA have: the limit belongs to the kernel, not to a handle, so it must
+// hold the largest windows of any handle (strip_kernels.cu).
+cudaError_t allow_shared_memory(const void* kernel);
 // Sets the dynamic shared-memory limit of the row-owned kernel the tiling and
 // precision select (once per event set; launch_iterate_rows only launches).
 cudaError_t rows_prepare_kernel(const Tiling& t, int precision);
@@ -183,7 +188,7 @@ cudaError_t sort_events(const Tiling& t, int64_t n, const float4* ev_geom, const
 struct UnionOps {
   int32_t threads, events, rows, cols;  // CTA, batch, largest union
   size_t (*smem)(const Tiling& t, int precision);
-  cudaError_t (*prepare)(const Tiling& t, int precision);
+  cudaError_t (*prepare)(int precision);
   cudaError_t (*launch)(const DevGeom& g, const FastConst& fc, const Tiling& t,
                         const Chunk* chunks, int32_t n_chunks, const float4* ev_geom,
                         const short4* ev_box, const void* ev_const, const uint16_t* erows,
@@ -195,6 +200,7 @@ const UnionOps& union_ops_64x32();
 const UnionOps& union_ops_64x32n4();
 const UnionOps& union_ops_32x16();
 const UnionOps& union_ops_32x32();
+const UnionOps& union_ops_64x16();
 const UnionOps& union_ops(int shape);
 size_t union_event_bytes();
 size_t union_smem_bytes(const Tiling& t, int precision);

@@ -207,6 +207,19 @@ __global__ void sensitivity_kernel(DevGeom g, int kind, float* __restrict__ out)
 // launchers
 // ---------------------------------------------------------------------------------
 
+cudaError_t allow_shared_memory(const void* kernel) {
+  int device = 0, most = 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             most - static_cast<int>(a.sharedSizeBytes));
+  return e;
+}
+
 cudaError_t launch_prep_events(const DevGeom& g, const float* z_u, const float* z_d,
                                const float* dl, int32_t stride, int64_t n, float4* ev_geom,
                                short4* ev_box, int32_t* hist_w, int32_t* hist_h,

@@ -383,8 +383,7 @@ cudaError_t launch_rows_kernel(const DevGeom& g, const FastConst& fc, const Tili
                       2ull * rows_stage_bytes(E, t.row_stride);
   auto* k = iterate_rows_kernel<NW, G, RS, SW, E, ACC, DEN64>;
   if (op == 0)  // once per event set, not per iteration
-    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem));
+    return allow_shared_memory(reinterpret_cast<const void*>(k));
   k<<<n_chunks, NW * 32, smem, s>>>(g, fc, t, chunks, ev_geom, ev_box, ev_pk, rows, pq, rho, out,
                                     aux, counters, seed);
   return cudaGetLastError();

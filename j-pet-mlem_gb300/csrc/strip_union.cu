@@ -164,6 +164,7 @@ const UnionOps& union_ops(int shape) {
     case kUnion64x32n4: return union_ops_64x32n4();
     case kUnion32x16: return union_ops_32x16();
     case kUnion32x32: return union_ops_32x32();
+    case kUnion64x16: return union_ops_64x16();
     default: return union_ops_64x32();
   }
 }
@@ -175,7 +176,7 @@ size_t union_smem_bytes(const Tiling& t, int precision) {
 }
 
 cudaError_t union_prepare_kernel(const Tiling& t, int precision) {
-  return union_ops(t.union_shape).prepare(t, precision);
+  return union_ops(t.union_shape).prepare(precision);
 }
 
 size_t union_row_words(const Tiling& t) { return union_ops(t.union_shape).rows; }

@@ -38,7 +38,8 @@
 // Kernel value (src/2d/strip/gaussian_kernel.h:51-79, rewritten as in
 // strip_fast.cu): along a row the exponent of K / K_ref is p + q j + c j^2 with
 // c = kz pw^2.  With j counted from the union row's even start column and
-// jc = j - kCols / 2, K = 2^(p' + q' jc) * 2^(c jc^2); the second factor is the same
+// jc = j - the union row's middle column (u_centre: the further from its events
+// the count starts, the more of p + q jc + c jc^2 cancels), K = 2^(p' + q' jc) * 2^(c jc^2); the second factor is the same
 // for every event, row and batch, so where it stays in range (u_exponent_form) it multiplies rho when rho is read
 // (rho'' = rho 2^(c jc^2)) and a pixel costs one FFMA2 per pixel pair, one ex2
 // per pixel and one FMUL2; otherwise (coarse pixels, where 2^(c jc^2) would
@@ -142,8 +143,8 @@ struct USmem {
   typename C::Mask mask[2][C::E][C::kRows + 4];  // columns of the union row inside the event's interval
   uint32_t urow[2][C::kRows];        // union start column | union width << 16
   __align__(16) DT den_part[2][C::E][C::kPartials];  // float, or double (FP64 denominators)
-  float gfac[C::kCols];              // 2^(c jc^2), jc = j - kCols / 2 (split exponent)
-  float cjc[C::kCols];               // c jc^2 (full exponent)
+  float gfac[2 * C::kCols];          // 2^(c jc^2), jc = index - kCols (split exponent)
+  float cjc[2 * C::kCols];           // c jc^2 (full exponent)
   uint32_t bw[4];  // the chunk's batch words and exact-path list (+ one read past the last
                    // batch): chunk_events + 4 words, the last of the allocation
 };
@@ -180,6 +181,10 @@ constexpr int kXFull = 0;   // p + q jc + c jc^2 per pixel
 constexpr int kXSplit = 1;  // 2^(c jc^2) folded into rho''
 constexpr int kXChain = 2;  // split, and K' stepped along the row by R8
 
+// The column that a union row of width wu counts jc from: its middle, even so
+// that the pairs of the jc tables stay aligned.
+__device__ __forceinline__ int u_centre(int wu) { return (wu >> 1) & ~1; }
+
 // Union rows and per-(event, row) records of one batch: 4 / RS threads per
 // union row (consecutive lanes), each handling RS E / 4 events.
 template <class C, int XM, class DT>
@@ -198,7 +203,7 @@ __device__ __forceinline__ void u_setup(const DevGeom& g, const FastConst& fc, U
   const int u = static_cast<int>(ur & 511u), wu = static_cast<int>(ur >> 9);
   if (sub == 0) S.urow[buf][r] = static_cast<uint32_t>(u) | (static_cast<uint32_t>(wu) << 16);
   const float py = g.tl_y_half_h - static_cast<float>(oy + u0 + r) * g.pixel_height;
-  const float colm = static_cast<float>(ox + u + C::kCols / 2);
+  const float colm = static_cast<float>(ox + u + u_centre(wu));
   const float kz2pw = 2.0f * fc.kz * g.pixel_width;
 #pragma unroll
   for (int k = 0; k < kEPT; ++k) {
@@ -240,18 +245,20 @@ __device__ __forceinline__ bool u_column(uint64_t m, int j) {
 template <class C, int SWN, int RSI, bool SPLIT, class DT>
 __device__ __forceinline__ void u_forward(float2 (&kr)[C::E][C::RS][C::SW], DT (&dsum)[C::E],
                                           const float* w_rho, const USmem<C, DT>& S, int buf,
-                                          int base, int r_u, const float2 (&jc2)[C::SW], int gl) {
-  float2 rr[C::SW], cq[C::SW];
+                                          int base, int r_u, int jc0, int gl) {
+  float2 rr[C::SW], cq[C::SW], jc2[C::SW];
 #pragma unroll
   for (int s = 0; s < SWN; ++s) {
     const float2 rv = *reinterpret_cast<const float2*>(w_rho + base + 8 * s);
     if (SPLIT) {
-      const float2 gv = *reinterpret_cast<const float2*>(&S.gfac[2 * gl + 8 * s]);
+      const float2 gv = *reinterpret_cast<const float2*>(&S.gfac[C::kCols + jc0 + 8 * s]);
       rr[s] = __fmul2_rn(rv, gv);
     } else {
       rr[s] = rv;
-      cq[s] = *reinterpret_cast<const float2*>(&S.cjc[2 * gl + 8 * s]);
+      cq[s] = *reinterpret_cast<const float2*>(&S.cjc[C::kCols + jc0 + 8 * s]);
     }
+    const float j0 = static_cast<float>(jc0 + 8 * s);
+    jc2[s] = make_float2(j0, j0 + 1.0f);
   }
 #pragma unroll
   for (int j = 0; j < C::E; ++j) {
@@ -280,19 +287,20 @@ template <class C, int SWN, int RSI, class DT>
 __device__ __forceinline__ void u_forward_chain(float2 (&kr)[C::E][C::RS][C::SW],
                                                 DT (&dsum)[C::E], const float* w_rho,
                                                 const USmem<C, DT>& S, int buf, int base, int r_u,
-                                                float jc0, int gl) {
+                                                int jc0, int gl) {
   float2 rr[C::SW];
+  const float jf = static_cast<float>(jc0);
 #pragma unroll
   for (int s = 0; s < SWN; ++s) {
     const float2 rv = *reinterpret_cast<const float2*>(w_rho + base + 8 * s);
-    const float2 gv = *reinterpret_cast<const float2*>(&S.gfac[2 * gl + 8 * s]);
+    const float2 gv = *reinterpret_cast<const float2*>(&S.gfac[C::kCols + jc0 + 8 * s]);
     rr[s] = __fmul2_rn(rv, gv);
   }
 #pragma unroll
   for (int j = 0; j < C::E; ++j) {
     const float4 a = S.pq[buf][j][r_u];
     const typename C::Mask m = S.mask[buf][j][r_u] >> (2 * gl);
-    const float e0 = fmaf(a.y, jc0, a.x);
+    const float e0 = fmaf(a.y, jf, a.x);
     float2 k = make_float2(ex2_approx(e0), ex2_approx(e0 + a.y));
     const float2 r8 = make_float2(a.z, a.w);
     float2 dd;
@@ -359,7 +367,7 @@ template <class C, int SWN, int RSI, int ACC>
 __device__ __forceinline__ void u_back_chain(const float2 (&kr)[C::E][C::RS][C::SW], float inv_l,
                                              const float* w_rho, const float* gfac,
                                              float* w_out, float* w_comp, int base, int wu,
-                                             int gl, float dither) {
+                                             int jc0, int gl, float dither) {
   // events outer, so that one event's 1/den is live at a time (lane j holds
   // event j's); the per-pair sums take the events in the same order as before
   float2 acc[C::SW];
@@ -377,7 +385,7 @@ __device__ __forceinline__ void u_back_chain(const float2 (&kr)[C::E][C::RS][C::
     // row's pitch plus the 64-float padding); the store is predicated on the
     // union row's width, the only pixels this row group owns
     const float2 rv = *reinterpret_cast<const float2*>(w_rho + base + 8 * s);
-    const float2 gv = *reinterpret_cast<const float2*>(gfac + 2 * gl + 8 * s);
+    const float2 gv = *reinterpret_cast<const float2*>(gfac + C::kCols + jc0 + 8 * s);
     const bool own = 2 * gl + 8 * s < wu;
     if (ACC == kAccFloat) {
       float2* op = reinterpret_cast<float2*>(w_out + base + 8 * s);
@@ -415,13 +423,12 @@ __device__ __forceinline__ void u_back(const float2 (&kr)[C::E][C::RS][C::SW],
 template <class C, int SWN, int RSI, int XM, class DT>
 __device__ __forceinline__ void u_forward_x(float2 (&kr)[C::E][C::RS][C::SW], DT (&dsum)[C::E],
                                             const float* w_rho, const USmem<C, DT>& S, int buf,
-                                            int base, int r_u, const float2 (&jc2)[C::SW],
-                                            int gl) {
+                                            int base, int r_u, int jc0, int gl) {
   if constexpr (SWN > 0) {
     if constexpr (XM == kXChain)
-      u_forward_chain<C, SWN, RSI, DT>(kr, dsum, w_rho, S, buf, base, r_u, jc2[0].x, gl);
+      u_forward_chain<C, SWN, RSI, DT>(kr, dsum, w_rho, S, buf, base, r_u, jc0, gl);
     else
-      u_forward<C, SWN, RSI, XM == kXSplit, DT>(kr, dsum, w_rho, S, buf, base, r_u, jc2, gl);
+      u_forward<C, SWN, RSI, XM == kXSplit, DT>(kr, dsum, w_rho, S, buf, base, r_u, jc0, gl);
   }
 }
 
@@ -442,9 +449,11 @@ __device__ __forceinline__ void u_sweeps(int nsw, F&& f) {
 template <class C, int SWN, int RSI, int XM, int ACC>
 __device__ __forceinline__ void u_back_x(const float2 (&kr)[C::E][C::RS][C::SW], float inv_l,
                                          const float* w_rho, const float* gfac, float* w_out,
-                                         float* w_comp, int base, int wu, int gl, float dither) {
+                                         float* w_comp, int base, int wu, int jc0, int gl,
+                                         float dither) {
   if constexpr (SWN > 0 && XM == kXChain) {
-    u_back_chain<C, SWN, RSI, ACC>(kr, inv_l, w_rho, gfac, w_out, w_comp, base, wu, gl, dither);
+    u_back_chain<C, SWN, RSI, ACC>(kr, inv_l, w_rho, gfac, w_out, w_comp, base, wu, jc0, gl,
+                                   dither);
   } else if constexpr (SWN > 0) {
     float2 inv2[C::E];
 #pragma unroll
@@ -517,17 +526,11 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
   }
   cp_async_commit();
   for (int i = threadIdx.x; i < 64; i += NW * 32) w_rho[t.win_h * pitch + i] = 0.0f;
-  if (threadIdx.x < C::kCols) {
+  if (threadIdx.x < 2 * C::kCols) {
     const float cz = fc.kz * g.pixel_width * g.pixel_width;
-    const float jc = static_cast<float>(static_cast<int>(threadIdx.x) - C::kCols / 2);
+    const float jc = static_cast<float>(static_cast<int>(threadIdx.x) - C::kCols);
     S.cjc[threadIdx.x] = cz * jc * jc;
     S.gfac[threadIdx.x] = ex2_approx(cz * jc * jc);
-  }
-  float2 jc2[SW];
-#pragma unroll
-  for (int s = 0; s < SW; ++s) {
-    const float j0 = static_cast<float>(2 * gl + 8 * s - C::kCols / 2);
-    jc2[s] = make_float2(j0, j0 + 1.0f);
   }
   unsigned long long contrib = 0;
   cp_async_wait_all();
@@ -545,7 +548,7 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
     DT dsum[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) dsum[j] = DT(0);
-    int base[RS], wu[RS], nsw[RS];
+    int base[RS], wu[RS], nsw[RS], jc0[RS];
 #pragma unroll
     for (int rs = 0; rs < RS; ++rs) {
       const int r_u = kRowsPerStep * rs + 8 * warp + gid;
@@ -553,6 +556,7 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
       const int wrow = min(u0 + r_u, t.win_h - 1);
       base[rs] = wrow * pitch + static_cast<int>(ur & 0xFFFFu) + 2 * gl;
       wu[rs] = static_cast<int>(ur >> 16);
+      jc0[rs] = 2 * gl - u_centre(wu[rs]);
       nsw[rs] = (__reduce_max_sync(kFull, static_cast<unsigned>(wu[rs])) + 7) >> 3;
     }
     // ---- forward, and the set-up of the next batch (its staged data was
@@ -565,17 +569,20 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
     // buffer from stale staged data).
     if constexpr (RS == 1) {
       u_sweeps<SW>(nsw[0], [&](auto n) {
-        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, w_rho, S, buf, base[0], 8 * warp + gid, jc2, gl);
+        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, w_rho, S, buf, base[0], 8 * warp + gid, jc0[0],
+                                                  gl);
         tot = rows_transpose_sum<E>(dsum);
         u_setup<C, XM, DT>(g, fc, S, buf ^ 1, S.bw[b + 1], ox, oy);
       });
     } else {
       u_sweeps<SW>(nsw[0], [&](auto n) {
-        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, w_rho, S, buf, base[0], 8 * warp + gid, jc2, gl);
+        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, w_rho, S, buf, base[0], 8 * warp + gid, jc0[0],
+                                                  gl);
       });
       u_sweeps<SW>(nsw[RS - 1], [&](auto n) {
         u_forward_x<C, decltype(n)::value, RS - 1, XM, DT>(kr, dsum, w_rho, S, buf, base[RS - 1],
-                                            kRowsPerStep + 8 * warp + gid, jc2, gl);
+                                            kRowsPerStep + 8 * warp + gid, jc0[RS - 1],
+                                                       gl);
       });
       if (b + 1 < nb) u_setup<C, XM, DT>(g, fc, S, buf ^ 1, S.bw[b + 1], ox, oy);
       tot = rows_transpose_sum<E>(dsum);
@@ -620,10 +627,11 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
       u_sweeps<SW>(nsw[rs], [&](auto n) {
         if (rs == 0)
           u_back_x<C, decltype(n)::value, 0, XM, ACC>(kr, inv_l, w_rho, S.gfac, w_out, w_comp, base[0], wu[0],
-                                       gl, dither);
+                                       jc0[0], gl, dither);
         else
           u_back_x<C, decltype(n)::value, RS - 1, XM, ACC>(kr, inv_l, w_rho, S.gfac, w_out, w_comp,
-                                            base[RS - 1], wu[RS - 1], gl, dither);
+                                            base[RS - 1], wu[RS - 1], jc0[RS - 1], gl,
+                                            dither);
       });
     }
   }
@@ -674,7 +682,7 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
 
 // ---- host side of one shape --------------------------------------------------------
 
-// The exponent form: 2^(c jc^2), |jc| <= kCols / 2, may multiply rho while it
+// The exponent form: 2^(c jc^2), |jc| <= kCols / 2 + 1 in a row, may multiply rho while it
 // stays a normal float with room for K' beside it (split); the chain form also
 // needs every K' a lane steps through to stay one: a column of the union row is
 // at most kCols + 3 sigma_z / (sqrt(2) pw) pixels from the event's row peak (the
@@ -682,23 +690,19 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
 template <class C>
 int u_exponent_form(const DevGeom& g, const FastConst& fc) {
   const float cz = -fc.kz * g.pixel_width * g.pixel_width;
-  const float half = 0.5f * C::kCols;
+  const float half = 0.5f * C::kCols + 1.0f;
   if (cz * half * half > 80.0f) return kXFull;
   const float d = C::kCols + 2.1213204f * g.sigma_z / g.pixel_width;
   return cz * d * d <= 111.0f ? kXChain : kXSplit;
 }
 
 template <class C, int ACC, bool DEN64>
-cudaError_t u_prepare(const Tiling& t) {
-  const int bytes = static_cast<int>(u_smem<C, ACC, DEN64>(t));
-  cudaError_t e = cudaFuncSetAttribute(iterate_union_kernel<C, kXFull, ACC, DEN64>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(iterate_union_kernel<C, kXSplit, ACC, DEN64>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(iterate_union_kernel<C, kXChain, ACC, DEN64>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+cudaError_t u_prepare() {
+  cudaError_t e = cudaSuccess;
+  for (auto* k : {iterate_union_kernel<C, kXFull, ACC, DEN64>,
+                  iterate_union_kernel<C, kXSplit, ACC, DEN64>,
+                  iterate_union_kernel<C, kXChain, ACC, DEN64>})
+    if (e == cudaSuccess) e = allow_shared_memory(reinterpret_cast<const void*>(k));
   return e;
 }
 
@@ -712,12 +716,12 @@ struct UnionHost {
       default: return u_smem<C, kAccFloat, false>(t);
     }
   }
-  static cudaError_t prepare(const Tiling& t, int precision) {
+  static cudaError_t prepare(int precision) {
     switch (precision) {
-      case kPrecisionCompensated: return u_prepare<C, kAccCompensated, false>(t);
-      case kPrecisionCompensatedDen64: return u_prepare<C, kAccCompensated, true>(t);
-      case kPrecisionFixed: return u_prepare<C, kAccFixed, false>(t);
-      default: return u_prepare<C, kAccFloat, false>(t);
+      case kPrecisionCompensated: return u_prepare<C, kAccCompensated, false>();
+      case kPrecisionCompensatedDen64: return u_prepare<C, kAccCompensated, true>();
+      case kPrecisionFixed: return u_prepare<C, kAccFixed, false>();
+      default: return u_prepare<C, kAccFloat, false>();
     }
   }
   static cudaError_t launch(const DevGeom& g, const FastConst& fc, const Tiling& t,

@@ -1,0 +1,12 @@
+// Batch-union iteration (strip_union.cuh) for batches of up to
+// 64 rows x 16 columns: narrow rows of tall boxes (4 mm pixels at sigma 7 / 44).
+#include "strip_union.cuh"
+
+namespace jpet {
+
+const UnionOps& union_ops_64x16() {
+  static const UnionOps ops = UnionHost<UShape<8, 8, 2, 1, 3>>::ops();
+  return ops;
+}
+
+}  // namespace jpet

@@ -25,6 +25,9 @@ SHAPES = {
     "30 rows x 13 columns": (131, 127, 4.0, 10.0, 41.0, 3001),
     "30 rows x 15 columns": (131, 127, 4.0, 11.5, 41.0, 3001),
     "32 rows x 13 columns": (131, 127, 4.0, 10.0, 42.0, 3001),
+    "46 rows x 11 columns": (197, 203, 4.0, 8.0, 62.0, 3001),
+    "32 rows x 9 columns, dense": (61, 67, 4.0, 7.0, 44.0, 40000),
+    "64 rows x 13 columns": (197, 203, 2.0, 5.3, 42.0, 3001),
     "24 rows x 27 columns": (131, 127, 2.3, 13.2, 18.0, 3001),
     "24 rows x 29 columns": (131, 127, 2.1, 13.2, 16.5, 3001),
     "64 rows x 23 columns": (197, 203, 2.0, 10.0, 42.0, 3001),
