@@ -271,12 +271,14 @@ int jpet_strip_reference_fp64(const jpet_strip_geom* geom, const float* d_respon
  * reconstructions (own geometry, widths, events, images) whose iterations run
  * together, one CUDA graph launch per jpet_strip_batch_iterate call.  Every
  * instance is a handle of its own (jpet_strip_batch_instance) for images,
- * counters and sensitivity maps; batches run the FP32 row-owned kernel in the
- * CPU-reference mode. */
+ * counters and sensitivity maps; batches run the FP32 batch-union kernel (FAST)
+ * or the row-owned kernel (ROWS) in the CPU-reference mode. */
 typedef struct jpet_strip_batch jpet_strip_batch_t;
 typedef struct jpet_strip_batch_plan {
-  int32_t raster_shape;          /* JPET_RASTER_* the instance runs (0 = automatic) */
-  int32_t block_threads;         /* CTA size (0 = default) */
+  int32_t raster_shape;          /* JPET_RASTER_* the instance runs (0 = automatic); with the
+                                    batch-union kernel, the one that covers its boxes */
+  int32_t block_threads;         /* CTA size (0 = default); 256 also for the batch-union
+                                    kernel's 384-thread CTAs */
   double tuned_ms_per_iteration; /* best time on the tuning prefix, -1 = not timed */
   int64_t tuned_events;          /* events of the tuning prefix */
   int32_t candidates;            /* plans timed for this instance (0 = cached plan) */
@@ -294,10 +296,11 @@ int jpet_strip_batch_instance(jpet_strip_batch_t* b, int32_t i, jpet_strip_t** h
 /* AoS responses of instance i, host memory (on_device = 0) or device memory. */
 int jpet_strip_batch_set_events(jpet_strip_batch_t* b, int32_t i, const float* aos, int64_t n,
                                 int32_t on_device);
-/* Autotuner: for every instance, times its automatic register shape and the
- * next larger one with 128- and 256-thread CTAs and two tile sides (the
- * largest square tile the CTA's window budget allows, and half of it) on the
- * first max_tune_events events (<= 0: 262144) and keeps the fastest; plans are
+/* Autotuner: for every instance, times two tile sides (the largest square tile
+ * the CTA's window budget allows, and half of it; with the row-owned kernel
+ * each with its automatic register shape and the next larger one and with 128-
+ * and 256-thread CTAs) on the first max_tune_events events (<= 0: 262144) and
+ * keeps the fastest; plans are
  * cached by grid, pixel size, widths and event-count octave.  Re-bins the
  * events with the chosen plan and resets every image to uniform 1. */
 int jpet_strip_batch_tune(jpet_strip_batch_t* b, int64_t max_tune_events);
@@ -305,7 +308,8 @@ int jpet_strip_batch_plan_of(const jpet_strip_batch_t* b, int32_t i, jpet_strip_
 /* n iterations of every instance: one graph launch (captured on first use for
  * each n), complete on return. */
 int jpet_strip_batch_iterate(jpet_strip_batch_t* b, int32_t n);
-/* Kernels per batched iteration after the first iterate (0 before). */
+/* Kernels per batched iteration (of all instances) after the first iterate (0
+ * before). */
 int jpet_strip_batch_launches_per_iteration(const jpet_strip_batch_t* b);
 
 /* ---- event generator (the phantom tool's Monte Carlo on the GPU) ----------

@@ -105,6 +105,7 @@ struct jpet_strip {
   unsigned long long total_box_pixels = 0;
   bool events_ready = false;
   int64_t iterations_done = 0;
+  uint64_t generation = 0;  // event sets prepared: what a captured graph of this handle was made for
 
   int fail(int code, const char* fmt, ...) {
     char buf[512];
@@ -330,6 +331,7 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
                    int64_t n, int32_t stride = 1) {
   cudaStream_t s = h->stream;
   h->events_ready = false;
+  ++h->generation;
   h->n_events = n;
   h->n_sorted = h->n_oversize = h->n_chunks = h->n_tiles_nonempty = 0;
   h->total_box_pixels = 0;
@@ -517,44 +519,104 @@ int upload_and_prepare(jpet_strip* h, const float* zu, const float* zd, const fl
   return prepare_events(h, d_zu, d_zd, d_dl, n);
 }
 
+// n iterations of the prepared events on stream s.
+int iterate_on(jpet_strip* h, int n, cudaStream_t s) {
+  const size_t n_pix = static_cast<size_t>(h->g.n_y) * h->g.n_z;
+  const float* sens = h->sens_pixel.p;
+  for (int it = 0; it < n; ++it) {
+    JPET_CUDA(h, cudaMemsetAsync(h->out.p, 0, n_pix * sizeof(float), s), "clear image");
+    JPET_CUDA(h, cudaMemsetAsync(h->counters.p, 0, sizeof(DevCounters), s), "clear counters");
+    const bool aux_img = h->opts.precision != JPET_PRECISION_FP32;
+    const AuxImage aux{h->out_lo.p, h->out_q.p};
+    if (h->out_lo.p)
+      JPET_CUDA(h, cudaMemsetAsync(h->out_lo.p, 0, n_pix * sizeof(float), s), "clear image");
+    if (h->out_q.p)
+      JPET_CUDA(h, cudaMemsetAsync(h->out_q.p, 0, n_pix * sizeof(unsigned long long), s),
+                "clear image");
+    if (h->use_fast) {
+      const int prec = precision_code(h->opts.precision);
+      const uint32_t seed = 0x9E3779B9u * static_cast<uint32_t>(h->iterations_done + 1);
+      if (h->use_union) {
+        JPET_CUDA(h, launch_iterate_union(h->g, h->fc, h->tiling, h->chunks.p, h->n_chunks,
+                                          h->sorted_geom.p, h->sorted_box.p, h->ev_const.p,
+                                          h->event_rows.p, h->union_rows.p, h->batches.p,
+                                          h->rho.p, h->out.p, aux, h->counters.p, prec, seed,
+                                          s),
+                  "iteration kernel launch");
+      } else if (h->opts.variant == JPET_VARIANT_WARP) {
+        JPET_CUDA(h, launch_iterate_fast(h->g, h->fc, h->tiling, h->chunks.p, h->n_chunks,
+                                         h->sorted_geom.p, h->sorted_box.p, h->row_table.p,
+                                         h->rho.p, h->out.p, aux, h->counters.p, prec,
+                                         seed, s),
+                  "iteration kernel launch");
+      } else {
+        JPET_CUDA(h, launch_iterate_rows(h->g, h->fc, h->tiling, h->chunks.p, h->n_chunks,
+                                         h->sorted_geom.p, h->sorted_box.p, h->ev_pk.p,
+                                         h->row_pk.p, h->row_pq.p, h->rho.p, h->out.p,
+                                         aux, h->counters.p, prec, seed, s),
+                  "iteration kernel launch");
+      }
+    } else {
+      JPET_CUDA(h, launch_iterate(h->g, h->tiling, h->opts.mode, h->chunks.p, h->n_chunks,
+                                  h->sorted_geom.p, h->sorted_box.p, h->rho.p, sens, h->out.p,
+                                  h->counters.p, s),
+                "iteration kernel launch");
+    }
+    JPET_CUDA(h, launch_iterate_global(h->g, h->opts.mode, h->n_oversize, h->over_geom.p,
+                                       h->over_box.p, h->rho.p, sens, h->out.p, h->counters.p, s),
+              "large-box kernel launch");
+    if (aux_img)
+      JPET_CUDA(h, launch_combine_aux(precision_code(h->opts.precision), aux, h->out.p, h->out.p,
+                                      n_pix, s),
+                "combine kernel launch");
+    std::swap(h->rho, h->out);
+    ++h->iterations_done;
+    h->counters_valid = true;
+  }
+  return JPET_OK;
+}
+
 }  // namespace
 
 // ---- access for the batch (strip_batch.cu) --------------------------------------
 namespace jpet {
 
-int handle_batch_view(jpet_strip* h, BatchInstance* v, std::string& why) {
+int handle_batch_ready(const jpet_strip* h, std::string& why) {
   if (!h->events_ready) {
     why = "events not set";
     return JPET_ERR_STATE;
   }
-  if (!h->use_fast || h->opts.variant != JPET_VARIANT_ROWS ||
+  if (!h->use_fast || h->opts.variant == JPET_VARIANT_WARP ||
       h->opts.precision != JPET_PRECISION_FP32) {
-    why = "batched instances run the FP32 row-owned kernel (CPU-reference mode, ROWS variant)";
+    why = "batched instances run the FP32 batch-union or row-owned kernel (CPU-reference mode)";
     return JPET_ERR_UNSUPPORTED;
   }
-  v->g = h->g;
-  v->fc = h->fc;
-  v->t = h->tiling;
-  v->chunks = h->chunks.p;
-  v->ev_geom = h->sorted_geom.p;
-  v->ev_box = h->sorted_box.p;
-  v->ev_pk = h->ev_pk.p;
-  v->rows = h->row_pk.p;
-  v->pq = h->row_pq.p;
-  v->img[0] = h->rho.p;
-  v->img[1] = h->out.p;
-  v->counters = h->counters.p;
-  v->over_geom = h->over_geom.p;
-  v->over_box = h->over_box.p;
-  v->n_oversize = h->n_oversize;
-  v->n_pix = static_cast<int32_t>(h->g.n_y) * h->g.n_z;
   return JPET_OK;
 }
 
-int32_t handle_n_chunks(const jpet_strip* h) { return h->n_chunks; }
-int handle_device(const jpet_strip* h) { return h->device; }
+const DevGeom& handle_geom(const jpet_strip* h) { return h->g; }
+const Tiling& handle_tiling(const jpet_strip* h) { return h->tiling; }
+uint64_t handle_generation(const jpet_strip* h) { return h->generation; }
+const float* handle_image(const jpet_strip* h) { return h->rho.p; }
+// kernels of one iteration
+int handle_launches(const jpet_strip* h) {
+  return (h->n_chunks > 0 ? 1 : 0) + (h->n_oversize > 0 ? 1 : 0);
+}
 
-// After n batched iterations: the latest image is in img[n & 1].
+// Issues n iterations on the (capturing) stream and leaves the handle as it was:
+// handle_batch_done counts them when the graph has run.
+int handle_capture_iterations(jpet_strip* h, int n, cudaStream_t s) {
+  const bool valid = h->counters_valid;
+  const int64_t done = h->iterations_done;
+  const float* image = h->rho.p;
+  const int rc = iterate_on(h, n, s);
+  if (h->rho.p != image) std::swap(h->rho, h->out);
+  h->iterations_done = done;
+  h->counters_valid = valid;
+  return rc;
+}
+
+// After n batched iterations: the latest image is in the other buffer if n is odd.
 void handle_batch_done(jpet_strip* h, int n) {
   if (n & 1) std::swap(h->rho, h->out);
   h->iterations_done += n;
@@ -792,60 +854,7 @@ int jpet_strip_iterate(jpet_strip_t* h, int n) {
   if (n < 0) return h->fail(JPET_ERR_ARGUMENT, "negative iteration count");
   if (!h->events_ready) return h->fail(JPET_ERR_STATE, "set_events has not succeeded");
   JPET_CUDA(h, cudaSetDevice(h->device), "cudaSetDevice");
-  cudaStream_t s = h->stream;
-  const size_t n_pix = static_cast<size_t>(h->g.n_y) * h->g.n_z;
-  const float* sens = h->sens_pixel.p;
-  for (int it = 0; it < n; ++it) {
-    JPET_CUDA(h, cudaMemsetAsync(h->out.p, 0, n_pix * sizeof(float), s), "clear image");
-    JPET_CUDA(h, cudaMemsetAsync(h->counters.p, 0, sizeof(DevCounters), s), "clear counters");
-    const bool aux_img = h->opts.precision != JPET_PRECISION_FP32;
-    const AuxImage aux{h->out_lo.p, h->out_q.p};
-    if (h->out_lo.p)
-      JPET_CUDA(h, cudaMemsetAsync(h->out_lo.p, 0, n_pix * sizeof(float), s), "clear image");
-    if (h->out_q.p)
-      JPET_CUDA(h, cudaMemsetAsync(h->out_q.p, 0, n_pix * sizeof(unsigned long long), s),
-                "clear image");
-    if (h->use_fast) {
-      const int prec = precision_code(h->opts.precision);
-      const uint32_t seed = 0x9E3779B9u * static_cast<uint32_t>(h->iterations_done + 1);
-      if (h->use_union) {
-        JPET_CUDA(h, launch_iterate_union(h->g, h->fc, h->tiling, h->chunks.p, h->n_chunks,
-                                          h->sorted_geom.p, h->sorted_box.p, h->ev_const.p,
-                                          h->event_rows.p, h->union_rows.p, h->batches.p,
-                                          h->rho.p, h->out.p, aux, h->counters.p, prec, seed,
-                                          s),
-                  "iteration kernel launch");
-      } else if (h->opts.variant == JPET_VARIANT_WARP) {
-        JPET_CUDA(h, launch_iterate_fast(h->g, h->fc, h->tiling, h->chunks.p, h->n_chunks,
-                                         h->sorted_geom.p, h->sorted_box.p, h->row_table.p,
-                                         h->rho.p, h->out.p, aux, h->counters.p, prec,
-                                         seed, s),
-                  "iteration kernel launch");
-      } else {
-        JPET_CUDA(h, launch_iterate_rows(h->g, h->fc, h->tiling, h->chunks.p, h->n_chunks,
-                                         h->sorted_geom.p, h->sorted_box.p, h->ev_pk.p,
-                                         h->row_pk.p, h->row_pq.p, h->rho.p, h->out.p,
-                                         aux, h->counters.p, prec, seed, s),
-                  "iteration kernel launch");
-      }
-    } else {
-      JPET_CUDA(h, launch_iterate(h->g, h->tiling, h->opts.mode, h->chunks.p, h->n_chunks,
-                                  h->sorted_geom.p, h->sorted_box.p, h->rho.p, sens, h->out.p,
-                                  h->counters.p, s),
-                "iteration kernel launch");
-    }
-    JPET_CUDA(h, launch_iterate_global(h->g, h->opts.mode, h->n_oversize, h->over_geom.p,
-                                       h->over_box.p, h->rho.p, sens, h->out.p, h->counters.p, s),
-              "large-box kernel launch");
-    if (aux_img)
-      JPET_CUDA(h, launch_combine_aux(precision_code(h->opts.precision), aux, h->out.p, h->out.p,
-                                      n_pix, s),
-                "combine kernel launch");
-    std::swap(h->rho, h->out);
-    ++h->iterations_done;
-    h->counters_valid = true;
-  }
-  return JPET_OK;
+  return iterate_on(h, n, h->stream);
 }
 
 int jpet_strip_get_image(jpet_strip_t* h, float* rho) {

@@ -257,39 +257,4 @@ cudaError_t launch_iterate_global(const DevGeom& g, int32_t semantics, int32_t n
                                   DevCounters* counters, cudaStream_t s);
 cudaError_t launch_sensitivity(const DevGeom& g, int kind, float* out, cudaStream_t s);
 
-// ---------------------------------------------------------------------------
-// Batched reconstructions (strip_batch.cu): what one handle contributes.
-// ---------------------------------------------------------------------------
-struct BatchInstance {
-  DevGeom g;
-  FastConst fc;
-  Tiling t;
-  const Chunk* chunks;
-  const float4* ev_geom;
-  const short4* ev_box;
-  const uint32_t* ev_pk;
-  const uint32_t* rows;
-  const float2* pq;
-  float* img[2];  // iteration k reads img[k & 1] and writes img[(k + 1) & 1]
-  DevCounters* counters;
-  const float4* over_geom;
-  const short4* over_box;
-  int32_t n_oversize;
-  int32_t n_pix;
-};
-struct BatchItem {
-  int32_t inst, index;  // chunk (tile kernel) or first large event (large-box kernel)
-};
-constexpr int kBatchOversizePerItem = 32;
-
-cudaError_t batch_rows_prepare(int rows_shape, int threads, size_t smem, int* blocks_per_sm);
-cudaError_t launch_batch_rows(int rows_shape, int threads, size_t smem, int grid,
-                              const BatchInstance* insts, const BatchItem* items, int32_t n_items,
-                              int32_t* next, int parity, cudaStream_t s);
-size_t rows_smem_bytes(const Tiling& t, int threads, int rows_shape);
-cudaError_t launch_batch_clear(const BatchInstance* insts, int32_t n_inst, int32_t max_pix,
-                               int parity, cudaStream_t s);
-cudaError_t launch_batch_oversize(const BatchInstance* insts, const BatchItem* items,
-                                  int32_t n_items, int parity, cudaStream_t s);
-
 }  // namespace jpet

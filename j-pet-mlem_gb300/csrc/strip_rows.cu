@@ -1,5 +1,5 @@
 // Row-owned MLEM iteration kernel for the CPU-reference semantics (the ROWS
-// variant; the precision modes and the batched reconstructions run it).
+// variant, in every precision mode).
 //
 // One CTA of NW warps (4 by default, or 8) per chunk of events of one image
 // tile, with the rho window and the back-projection window in shared memory, as
@@ -432,112 +432,6 @@ cudaError_t launch_rows_shape(const DevGeom& g, const FastConst& fc, const Tilin
                                           rho, out, aux, counters, precision, seed, s, op);
 }
 
-// ---- batched reconstructions ------------------------------------------------------
-
-// Persistent CTAs take (instance, chunk) work items from a shared counter,
-// largest first (the host sorts the items), and run the chunk with that
-// instance's geometry, tiling, events and images.
-template <int NW, int G, int RS, int SW, int E>
-__global__ void __launch_bounds__(NW * 32, (NW == 8 ? 2 : 4))
-    batch_rows_kernel(const BatchInstance* __restrict__ insts, const BatchItem* __restrict__ items,
-                      int32_t n_items, int32_t* next, int parity) {
-  __shared__ int32_t s_item;
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(next, 1);
-    __syncthreads();
-    const int32_t it = s_item;
-    __syncthreads();
-    if (it >= n_items) break;
-    const BatchItem w = items[it];
-    const BatchInstance& in = insts[w.inst];
-    rows_chunk<NW, G, RS, SW, E, kAccFloat, false>(
-        in.g, in.fc, in.t, in.chunks[w.index], in.ev_geom, in.ev_box, in.ev_pk, in.rows, in.pq,
-        in.img[parity], in.img[parity ^ 1], AuxImage{}, in.counters, 0u);
-    __syncthreads();
-  }
-}
-
-template <int NW, int G, int ROWS, int SW>
-struct BatchRows {
-  static constexpr int kPass = NW * (32 / G);
-  static constexpr int RS = (ROWS + kPass - 1) / kPass;
-  static constexpr int E = (RS * SW <= 4) ? 8 : (RS * SW <= 8 ? 4 : 2);
-  static auto kernel() { return batch_rows_kernel<NW, G, RS, SW, E>; }
-};
-
-template <int NW, int G, int ROWS, int SW>
-cudaError_t batch_rows_dispatch(int op, size_t smem, int grid, int* bps,
-                                const BatchInstance* insts, const BatchItem* items,
-                                int32_t n_items, int32_t* next, int parity, cudaStream_t s) {
-  auto* k = BatchRows<NW, G, ROWS, SW>::kernel();
-  if (op == 0) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, k, NW * 32, smem);
-  }
-  k<<<grid, NW * 32, smem, s>>>(insts, items, n_items, next, parity);
-  return cudaGetLastError();
-}
-
-template <int NW>
-cudaError_t batch_rows_shape(int shape, int op, size_t smem, int grid, int* bps,
-                             const BatchInstance* insts, const BatchItem* items, int32_t n_items,
-                             int32_t* next, int parity, cudaStream_t s) {
-  switch (shape) {
-    case kRowsShape8x1x1:
-      return batch_rows_dispatch<NW, 8, 32, 1>(op, smem, grid, bps, insts, items, n_items, next,
-                                               parity, s);
-    case kRowsShape8x1x2:
-      return batch_rows_dispatch<NW, 8, 32, 2>(op, smem, grid, bps, insts, items, n_items, next,
-                                               parity, s);
-    case kRowsShape4x1x2:
-      return batch_rows_dispatch<NW, 4, 64, 2>(op, smem, grid, bps, insts, items, n_items, next,
-                                               parity, s);
-    case kRowsShape4x1x3:
-      return batch_rows_dispatch<NW, 4, 64, 3>(op, smem, grid, bps, insts, items, n_items, next,
-                                               parity, s);
-    case kRowsShape4x1x4:
-      return batch_rows_dispatch<NW, 4, 64, 4>(op, smem, grid, bps, insts, items, n_items, next,
-                                               parity, s);
-    case kRowsShape2x1x6:
-      return batch_rows_dispatch<NW, 2, 64, 6>(op, smem, grid, bps, insts, items, n_items, next,
-                                               parity, s);
-    default:
-      return batch_rows_dispatch<NW, 4, 128, 4>(op, smem, grid, bps, insts, items, n_items, next,
-                                                parity, s);
-  }
-}
-
-__global__ void batch_clear_kernel(const BatchInstance* __restrict__ insts, int parity) {
-  const BatchInstance& in = insts[blockIdx.y];
-  float* out = in.img[parity ^ 1];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < in.n_pix; i += gridDim.x * blockDim.x)
-    out[i] = 0.0f;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *in.counters = DevCounters{};
-}
-
-// Large-box events of every instance: one warp per event, reference order,
-// global-memory atomics (as the single-handle large-box path).
-__global__ void batch_oversize_kernel(const BatchInstance* __restrict__ insts,
-                                      const BatchItem* __restrict__ items, int32_t n_items,
-                                      int parity) {
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-  for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const BatchItem w = items[it];
-    const BatchInstance& in = insts[w.inst];
-    const int end = min(in.n_oversize, w.index + kBatchOversizePerItem);
-    unsigned long long calls = 0, contrib = 0;
-    GlobalAccess acc{in.img[parity], in.img[parity ^ 1], in.g.n_z};
-    for (int e = w.index + warp; e < end; e += n_warps)
-      process_event<kCpuReference>(in.g, 32, in.over_geom[e], in.over_box[e], acc, nullptr, calls,
-                                   contrib);
-    if (lane == 0 && contrib) atomicAdd(&in.counters->n_contributing, contrib);
-    if (lane == 0 && calls) atomicAdd(&in.counters->n_kernel_calls, calls);
-  }
-}
-
 }  // namespace
 
 int rows_shape_rows(int rows_shape) {
@@ -605,52 +499,6 @@ cudaError_t launch_iterate_rows(const DevGeom& g, const FastConst& fc, const Til
 cudaError_t rows_prepare_kernel(const Tiling& t, int precision) {
   return rows_dispatch(DevGeom{}, FastConst{}, t, nullptr, 0, nullptr, nullptr, nullptr, nullptr,
                        nullptr, nullptr, nullptr, AuxImage{}, nullptr, precision, 0u, nullptr, 0);
-}
-
-size_t rows_smem_bytes(const Tiling& t, int threads, int rows_shape) {
-  const int nw = threads == 256 ? 8 : 4;
-  static const int rows_of[] = {32, 32, 64, 64, 64, 128, 64};
-  static const int g_of[] = {8, 8, 4, 4, 4, 4, 2};
-  static const int sw_of[] = {1, 2, 2, 3, 4, 4, 6};
-  const int k = (rows_shape >= 0 && rows_shape <= kRowsShape2x1x6) ? rows_shape : kRowsShape4x2x4;
-  const int pass = nw * (32 / g_of[k]);
-  const int rs = (rows_of[k] + pass - 1) / pass;
-  const int e = (rs * sw_of[k] <= 4) ? 8 : (rs * sw_of[k] <= 8 ? 4 : 2);
-  return 2ull * fast_window_floats(t) * 4 + 2ull * rows_stage_bytes(e, t.row_stride);
-}
-
-cudaError_t batch_rows_prepare(int rows_shape, int threads, size_t smem, int* blocks_per_sm) {
-  if (threads == 256)
-    return batch_rows_shape<8>(rows_shape, 0, smem, 0, blocks_per_sm, nullptr, nullptr, 0, nullptr,
-                               0, nullptr);
-  return batch_rows_shape<4>(rows_shape, 0, smem, 0, blocks_per_sm, nullptr, nullptr, 0, nullptr, 0,
-                             nullptr);
-}
-
-cudaError_t launch_batch_rows(int rows_shape, int threads, size_t smem, int grid,
-                              const BatchInstance* insts, const BatchItem* items, int32_t n_items,
-                              int32_t* next, int parity, cudaStream_t s) {
-  if (n_items <= 0) return cudaSuccess;
-  if (threads == 256)
-    return batch_rows_shape<8>(rows_shape, 1, smem, grid, nullptr, insts, items, n_items, next,
-                               parity, s);
-  return batch_rows_shape<4>(rows_shape, 1, smem, grid, nullptr, insts, items, n_items, next,
-                             parity, s);
-}
-
-cudaError_t launch_batch_clear(const BatchInstance* insts, int32_t n_inst, int32_t max_pix,
-                               int parity, cudaStream_t s) {
-  if (n_inst <= 0) return cudaSuccess;
-  const int bx = std::max(1, std::min(64, (max_pix + 255) / 256));
-  batch_clear_kernel<<<dim3(bx, n_inst), 256, 0, s>>>(insts, parity);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_batch_oversize(const BatchInstance* insts, const BatchItem* items,
-                                  int32_t n_items, int parity, cudaStream_t s) {
-  if (n_items <= 0) return cudaSuccess;
-  batch_oversize_kernel<<<std::min(n_items, 152 * 8), 256, 0, s>>>(insts, items, n_items, parity);
-  return cudaGetLastError();
 }
 
 }  // namespace jpet
