@@ -205,7 +205,10 @@ int widest_row(const DevGeom& g) {
 // SM's shared memory) and its largest chunk.  The smallest shape that leaves the
 // union of a batch a few rows and columns beyond its events' own; an explicit
 // CTA size selects the 64-row shapes.  Measured per iteration: 1e6 events of 26
-// rows x 11 columns (5 mm pixels) 552 us in the 64x32 shape, 294 in 32x16.
+// rows x 11 columns (5 mm pixels) 552 us in the 64x32 shape, 294 in 32x16; 1e6
+// events of 82 rows x 31 columns (2 mm, sigma 14 / 55), of which the 64x32
+// shape's windows and batches take one in ten, 23.0 ms there, 1.52 ms in 96x40
+// (1.64 with batches of 4 events and two CTAs per SM).
 struct UnionLimits {
   int shape, window_px, ctas_per_sm, max_chunk;
 };
@@ -216,7 +219,8 @@ UnionLimits union_limits(const jpet_strip_opts& o, int rows, int widest) {
   if (rows <= 30 && widest <= 13) return UnionLimits{kUnion32x16, 3328, 5, 1024};
   if (rows <= 30 && widest <= 28) return UnionLimits{kUnion32x32, 3328, 4, 1024};
   if (rows <= 64 && widest <= 13) return UnionLimits{kUnion64x16, 4096, 3, 1024};
-  return m;
+  if (rows <= 64 && widest <= 28) return m;
+  return UnionLimits{kUnion96x40, 10752, 1, 1024};
 }
 
 // Window sizing: the largest box dimension that covers all but a tiny tail of

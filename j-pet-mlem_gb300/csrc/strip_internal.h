@@ -56,6 +56,7 @@ enum UnionShape : int32_t {
   kUnion64x32n4 = 1,  // 4 warps, 4 events
   kUnion32x16 = 2,    // 4 warps, 8 events
   kUnion32x32 = 3,    // 4 warps, 8 events
+  kUnion96x40 = 4,    // 12 warps, 8 events
   kUnion64x16 = 5,    // 8 warps, 8 events
 };
 
@@ -200,6 +201,7 @@ const UnionOps& union_ops_64x32();
 const UnionOps& union_ops_64x32n4();
 const UnionOps& union_ops_32x16();
 const UnionOps& union_ops_32x32();
+const UnionOps& union_ops_96x40();
 const UnionOps& union_ops_64x16();
 const UnionOps& union_ops(int shape);
 size_t union_event_bytes();

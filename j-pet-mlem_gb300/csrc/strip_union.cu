@@ -164,6 +164,7 @@ const UnionOps& union_ops(int shape) {
     case kUnion64x32n4: return union_ops_64x32n4();
     case kUnion32x16: return union_ops_32x16();
     case kUnion32x32: return union_ops_32x32();
+    case kUnion96x40: return union_ops_96x40();
     case kUnion64x16: return union_ops_64x16();
     default: return union_ops_64x32();
   }
