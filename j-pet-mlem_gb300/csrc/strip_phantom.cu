@@ -26,9 +26,16 @@
 //  5. adds N(0, sigma_z) to z_u, z_d and N(0, sigma_dl) to dl (scanner.h:257-267,
 //     Box-Muller normals), with no second acceptance test.
 //
-// Detected events are written in candidate order (a count pass, a scan over
-// blocks and an ordered write pass with block-wide prefix sums), so the output
-// is deterministic as well.
+// Detected events are written in candidate order (a decision pass, a scan over
+// blocks and an ordered write pass), so the output is deterministic as well.
+//
+// Steps 1 to 4 are FP64 arithmetic by definition, and this GPU's FP64 pipe is a
+// sixty-fourth of its FP32 one.  The decision pass therefore evaluates them in
+// FP32 together with a bound on its own error, and only the candidates within
+// the bound of a decision (about 1e-4 of them) go through the FP64 arithmetic:
+// the decisions are those of the FP64 code.  It leaves one bit per candidate,
+// from which the write pass compacts each block's accepted candidates and
+// evaluates those alone in FP64, all threads busy.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -59,8 +66,10 @@ struct GenParams {
 };
 
 constexpr int kGenThreads = 256;
-constexpr int kGenRounds = 16;
+constexpr int kGenRounds = 4;  // 1024 candidates per block: small calls still spread over the SMs
 constexpr int kGenPerBlock = kGenThreads * kGenRounds;
+constexpr int kGenWords = kGenPerBlock / 32;
+constexpr int kGenMaxBlocks = 4096;  // 4 Mi candidates per pass at most
 constexpr int kGenMaxRegions = 256;
 
 __device__ __forceinline__ void philox_round(uint32_t (&x)[4], uint32_t k0, uint32_t k1) {
@@ -82,6 +91,11 @@ __device__ __forceinline__ void philox(uint32_t (&x)[4], uint32_t k0, uint32_t k
     k0 += 0x9E3779B9u;
     k1 += 0xBB67AE85u;
   }
+}
+
+__device__ __forceinline__ unsigned long long warp_add(unsigned long long v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
 // 53-bit uniform in [0, 1)
@@ -223,52 +237,394 @@ __device__ Candidate gen_candidate(const GenParams& p, const GenRegion* __restri
   return out;
 }
 
-// Block-wide exclusive prefix of a flag (kGenThreads threads); returns the
-// thread's rank and the block total.
-__device__ __forceinline__ int block_rank(bool flag, int* s_warp, int& total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned m = __ballot_sync(0xffffffffu, flag);
-  const int in_warp = __popc(m & ((1u << lane) - 1u));
-  if (lane == 0) s_warp[warp] = __popc(m);
-  __syncthreads();
-  int before = 0, sum = 0;
-#pragma unroll
-  for (int w = 0; w < kGenThreads / 32; ++w) {
-    const int v = s_warp[w];
-    before += (w < warp) ? v : 0;
-    sum += v;
-  }
-  __syncthreads();
-  total = sum;
-  return before + in_warp;
+// ---- FP64 functions of the write pass -----------------------------------------------
+//
+// The accepted candidates need eight uniforms, four square roots, three sines
+// and cosines, a tangent and two logarithms.  On ranges as plain as these (a
+// fraction of a turn, an angle below a right angle, a number in (0, 1]) the
+// textbook series take about 190 FP64 operations, all within a few units in
+// 1e-16, where the library's functions take about 1800 (2e6 events: 7.5 ms of
+// write pass with them, 1.1 ms with these).
+
+// 1 / x and sqrt(x): the FP32 value and two Newton steps (x > 0, normal, and
+// within FP32's range).
+__device__ __forceinline__ double gen_rcp(double x) {
+  double y = static_cast<double>(__frcp_rn(static_cast<float>(x)));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+__device__ __forceinline__ double gen_sqrt(double x) {
+  const double h = 0.5 * static_cast<double>(rsqrtf(static_cast<float>(x)));
+  double r = 2.0 * h * x;
+  r = fma(fma(-r, r, x), h, r);
+  return fma(fma(-r, r, x), h, r);
 }
 
-template <bool WRITE>
-__global__ void __launch_bounds__(kGenThreads) gen_kernel(
-    GenParams p, const GenRegion* __restrict__ regs_g, uint64_t cand0, int2* block_counts,
-    const long long* __restrict__ block_base, long long limit, int count_emissions,
-    long long capacity, unsigned long long* taken, float* __restrict__ out, GenImages im) {
-  __shared__ GenRegion regs[kGenMaxRegions];
-  __shared__ int s_warp[2][kGenThreads / 32];
-  for (int i = threadIdx.x; i < p.n_regions; i += blockDim.x) regs[i] = regs_g[i];
-  __syncthreads();
-  long long e_base = 0, d_base = 0;
-  if (WRITE) {
-    e_base = block_base[2 * blockIdx.x];
-    d_base = block_base[2 * blockIdx.x + 1];
+// sin r and cos r for |r| <= pi / 4 + 1e-8: their Taylor series to r^15 and r^16.
+__device__ __forceinline__ void gen_sincos_small(double r, double& sn, double& cs) {
+  const double z = r * r;
+  double a = -1.0 / 1307674368000.0;
+  a = fma(a, z, 1.0 / 6227020800.0);
+  a = fma(a, z, -1.0 / 39916800.0);
+  a = fma(a, z, 1.0 / 362880.0);
+  a = fma(a, z, -1.0 / 5040.0);
+  a = fma(a, z, 1.0 / 120.0);
+  a = fma(a, z, -1.0 / 6.0);
+  sn = fma(a * z, r, r);
+  double b = 1.0 / 20922789888000.0;
+  b = fma(b, z, -1.0 / 87178291200.0);
+  b = fma(b, z, 1.0 / 479001600.0);
+  b = fma(b, z, -1.0 / 3628800.0);
+  b = fma(b, z, 1.0 / 40320.0);
+  b = fma(b, z, -1.0 / 720.0);
+  b = fma(b, z, 1.0 / 24.0);
+  b = fma(b, z, -0.5);
+  cs = fma(b, z, 1.0);
+}
+
+// sin and cos of the turn u = u53(hi, ...): the nearest quarter turn from the
+// uniform's top bits, the rest by the series.
+__device__ __forceinline__ void gen_sincos_turn(uint32_t hi, double u, double& sn, double& cs) {
+  const uint32_t n = (hi >> 30) + ((hi >> 29) & 1u);
+  double a, b;
+  gen_sincos_small(fma(4.0, u, -static_cast<double>(n)) * 1.5707963267948966, a, b);
+  const double x = (n & 1u) ? b : a, y = (n & 1u) ? a : b;
+  sn = (n & 2u) ? -x : x;
+  cs = ((n + 1u) & 2u) ? -y : y;
+}
+
+// log x for x in (0, 1]: x = m 2^e with m in [sqrt(1/2), sqrt(2)), and log m =
+// 2 artanh((m - 1) / (m + 1)) by its series to the 21st power.
+__device__ __forceinline__ double gen_log(double x) {
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  int e = (hi >> 20) - 1023;
+  int mh = (hi & 0x000fffff) | 0x3ff00000;
+  if (mh >= 0x3ff6a09e) {  // above sqrt(2)
+    mh -= 0x00100000;
+    ++e;
   }
+  const double m = __hiloint2double(mh, lo);
+  const double s = (m - 1.0) * gen_rcp(m + 1.0), z = s * s;
+  double a = 1.0 / 21.0;
+  a = fma(a, z, 1.0 / 19.0);
+  a = fma(a, z, 1.0 / 17.0);
+  a = fma(a, z, 1.0 / 15.0);
+  a = fma(a, z, 1.0 / 13.0);
+  a = fma(a, z, 1.0 / 11.0);
+  a = fma(a, z, 1.0 / 9.0);
+  a = fma(a, z, 1.0 / 7.0);
+  a = fma(a, z, 1.0 / 5.0);
+  a = fma(a, z, 1.0 / 3.0);
+  const double s2 = 2.0 * s;
+  return fma(static_cast<double>(e), 0.69314718055994530942, fma(a * z, s2, s2));
+}
+
+// gen_candidate for a candidate known to be detected.
+__device__ __forceinline__ Candidate gen_detected(const GenParams& p,
+                                                  const GenRegion* __restrict__ regs,
+                                                  uint64_t index) {
+  const uint32_t lo = static_cast<uint32_t>(index), hi = static_cast<uint32_t>(index >> 32);
+  uint32_t r0[4] = {lo, hi, 0u, 0u};
+  uint32_t r1[4] = {lo, hi, 1u, 0u};
+  uint32_t r2[4] = {lo, hi, 2u, 0u};
+  uint32_t r3[4] = {lo, hi, 3u, 0u};
+  philox(r0, p.key0, p.key1);
+  philox(r1, p.key0, p.key1);
+  philox(r2, p.key0, p.key1);
+  philox(r3, p.key0, p.key1);
+  const double u_reg = u53(r0[0], r0[1]);
+  int k = 0;
+  while (k < p.n_regions - 1 && u_reg > regs[k].cdf) ++k;
+  const GenRegion& rg = regs[k];
+  const double u1 = u53(r0[2], r0[3]), u2 = u53(r1[0], r1[1]);
+  double px = rg.x, py = rg.y;
+  if (rg.kind == JPET_REGION_ELLIPSE) {
+    double st, ct;
+    gen_sincos_turn(r1[0], u2, st, ct);
+    const double rr = u1 > 0.0 ? gen_sqrt(u1) : 0.0;
+    const double ex = rg.a * rr * ct, ey = rg.b * rr * st;
+    px = rg.c * ex - rg.s * ey + rg.x;
+    py = rg.s * ex + rg.c * ey + rg.y;
+  } else if (rg.kind == JPET_REGION_RECTANGLE) {
+    px = rg.x + rg.a * (2.0 * u1 - 1.0);
+    py = rg.y + rg.b * (2.0 * u2 - 1.0);
+  }
+  // the angle's sine and cosine: beyond pi / 4 those of the complement, swapped
+  const double phi = p.phi_max * (2.0 * u53(r1[2], r1[3]) - 1.0);
+  const double ap = fabs(phi);
+  const bool steep = ap > 0.78539816339744831;
+  double sp, cp;
+  gen_sincos_small(steep ? (1.5707963267948966 - ap) + 6.123233995736766e-17 : ap, sp, cp);
+  if (steep) {
+    const double v = sp;
+    sp = cp;
+    cp = v;
+  }
+  if (phi < 0.0) sp = -sp;
+  const double sec = gen_rcp(cp), t = sp * sec;
+  const double zu = px + (p.R - py) * t;
+  const double zd = px - (p.R + py) * t;
+  const double dl = -2.0 * py * sec;
+  const double x0 = 1.0 - u53(r2[0], r2[1]), x1 = 1.0 - u53(r3[0], r3[1]);
+  const double l0 = -2.0 * gen_log(x0), l1 = -2.0 * gen_log(x1);
+  const double m0 = l0 > 0.0 ? gen_sqrt(l0) : 0.0, m1 = l1 > 0.0 ? gen_sqrt(l1) : 0.0;
+  double s0, c0, s1, c1;
+  gen_sincos_turn(r2[2], u53(r2[2], r2[3]), s0, c0);
+  gen_sincos_turn(r3[2], u53(r3[2], r3[3]), s1, c1);
+  Candidate out{true, true, 0.f, 0.f, 0.f, px, py, 0.f, 0.f, 0.f, 0.f, 0.f};
+  out.zu = static_cast<float>(zu + p.sigma_z * m0 * c0);
+  out.zd = static_cast<float>(zd + p.sigma_z * m0 * s0);
+  out.dl = static_cast<float>(dl + p.sigma_dl * m1 * c1);
+  out.ex_zu = static_cast<float>(zu);
+  out.ex_zd = static_cast<float>(zd);
+  out.ex_dl = static_cast<float>(dl);
+  out.dir_x = static_cast<float>(sp);
+  out.dir_y = static_cast<float>(cp);
+  return out;
+}
+
+// A region in FP32, for the decision pass.
+struct GenRegionF {
+  float x, y, a, b, s, c, A, B, C, cdf;
+  int32_t kind;
+};
+
+constexpr int kGenNo = 0, kGenEmitted = 1, kGenDetected = 2, kGenUnsure = 3;
+
+// The decision of gen_candidate (not an emission, emitted, detected) in FP32, or
+// kGenUnsure where a comparison lies within the FP32 error: e counts units of
+// 1e-6, about eight times the rounding of the few operations behind each value
+// (the library's sinf, cosf and sincospif are within 2 units in the last place).
+__device__ __forceinline__ int gen_decide(const GenParams& p, const GenRegionF* regs,
+                                          uint64_t index) {
+  const uint32_t lo = static_cast<uint32_t>(index), hi = static_cast<uint32_t>(index >> 32);
+  uint32_t r0[4] = {lo, hi, 0u, 0u};
+  uint32_t r1[4] = {lo, hi, 1u, 0u};
+  philox(r0, p.key0, p.key1);
+  philox(r1, p.key0, p.key1);
+  constexpr float e = 1e-6f, kInv32 = 2.3283064365386963e-10f;
+  const float u_reg = static_cast<float>(r0[0]) * kInv32;
+  bool unsure = false;
+  int k = 0;
+  for (int i = 0; i < p.n_regions - 1; ++i) {
+    const float d = u_reg - regs[i].cdf;
+    unsure = unsure || fabsf(d) < e;
+    k += d > 0.0f;
+  }
+  const GenRegionF rg = regs[k];
+  const float u1 = static_cast<float>(r0[2]) * kInv32, u2 = static_cast<float>(r1[0]) * kInv32;
+  float px, py;
+  if (rg.kind == JPET_REGION_ELLIPSE) {
+    const float rr = sqrtf(u1);
+    float st, ct;
+    sincospif(2.0f * u2, &st, &ct);
+    const float ex = rg.a * rr * ct, ey = rg.b * rr * st;
+    px = rg.c * ex - rg.s * ey + rg.x;
+    py = rg.s * ex + rg.c * ey + rg.y;
+  } else if (rg.kind == JPET_REGION_RECTANGLE) {
+    px = rg.x + rg.a * (2.0f * u1 - 1.0f);
+    py = rg.y + rg.b * (2.0f * u2 - 1.0f);
+  } else {
+    px = rg.x;
+    py = rg.y;
+  }
+  // error of the point: the uniforms' own rounding moves sqrt(u1) near 0 by up
+  // to sqrt(2^-25), which the 1e-3 of the axes next to the centre cover
+  const float dp = e * (8.0f * (rg.a + rg.b) + fabsf(rg.x) + fabsf(rg.y)) +
+                   (u1 < 10.0f * e ? 1e-3f * (rg.a + rg.b) : 0.0f);
+  bool inside = false;
+  if (!p.additive) {
+    for (int i = 0; i < k; ++i) {
+      const GenRegionF q = regs[i];
+      const float dx = px - q.x, dy = py - q.y;
+      const float ddp = dp + e * (fabsf(q.x) + fabsf(q.y));
+      if (q.kind == JPET_REGION_ELLIPSE) {
+        const float gx = fabsf(q.A * dx) + fabsf(q.C * dy), gy = fabsf(q.C * dx) + fabsf(q.B * dy);
+        const float m = q.A * dx * dx + 2.0f * q.C * dx * dy + q.B * dy * dy;
+        const float err = 4.0f * e * (gx * fabsf(dx) + gy * fabsf(dy)) +
+                          2.0f * ddp * (gx + gy) + ddp * ddp * (q.A + q.B + 2.0f * fabsf(q.C));
+        unsure = unsure || !(fabsf(m - 1.0f) > err);
+        inside = inside || m <= 1.0f;
+      } else {
+        const float ax = fabsf(dx) - q.a, ay = fabsf(dy) - q.b;  // a = b = 0 for a point
+        const float err = ddp + e * (q.a + q.b);
+        unsure = unsure || (ax < err && ay < err && !(ax < -err && ay < -err));
+        inside = inside || (ax <= 0.0f && ay <= 0.0f);
+      }
+    }
+  }
+  const float phi = static_cast<float>(p.phi_max) *
+                    (2.0f * (static_cast<float>(r1[2]) * kInv32) - 1.0f);
+  float sp, cp;
+  sincosf(phi, &sp, &cp);
+  const float t = sp / cp;
+  const float R = static_cast<float>(p.R), half = static_cast<float>(0.5 * p.L);
+  const float zu = px + (R - py) * t, zd = px - (R + py) * t;
+  const float err = (1.0f + fabsf(t)) * (dp + 2.0f * e * (R + fabsf(px) + fabsf(py))) +
+                    2.0f * e * (1.0f + t * t) * (R + fabsf(py)) + 2.0f * e * half;
+  const float out = fmaxf(fabsf(zu), fabsf(zd)) - half;
+  unsure = unsure || !(fabsf(out) > err);  // also where a value is not finite
+  if (unsure) return kGenUnsure;
+  return inside ? kGenNo : (out < 0.0f ? kGenDetected : kGenEmitted);
+}
+
+// Decision pass: per block of kGenPerBlock candidates, one bit per candidate in
+// words (emitted, then detected) and the two counts.  Bound by the integer
+// rounds of Philox and the region loop: 2e6 events of ten ellipses took two
+// FP64 passes of 16.5 ms each over 4 Mi candidates (count 3.6, write 12.9).
+__global__ void __launch_bounds__(kGenThreads)
+    gen_decide_kernel(GenParams p, const GenRegion* __restrict__ regs_g, uint64_t cand0,
+                      uint32_t* __restrict__ words, int2* __restrict__ block_counts) {
+  __shared__ GenRegionF regs[kGenMaxRegions];
+  __shared__ int s_count[2][kGenThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < p.n_regions; i += blockDim.x) {
+    const GenRegion g = regs_g[i];
+    GenRegionF f;
+    f.x = static_cast<float>(g.x);
+    f.y = static_cast<float>(g.y);
+    f.a = g.kind == JPET_REGION_POINT ? 0.0f : static_cast<float>(g.a);
+    f.b = g.kind == JPET_REGION_POINT ? 0.0f : static_cast<float>(g.b);
+    f.s = static_cast<float>(g.s);
+    f.c = static_cast<float>(g.c);
+    f.A = static_cast<float>(g.A);
+    f.B = static_cast<float>(g.B);
+    f.C = static_cast<float>(g.C);
+    f.cdf = static_cast<float>(g.cdf);
+    f.kind = g.kind;
+    regs[i] = f;
+  }
+  __syncthreads();
   int n_emit = 0, n_det = 0;
+  uint32_t* w = words + static_cast<size_t>(blockIdx.x) * 2 * kGenWords;
   for (int r = 0; r < kGenRounds; ++r) {
-    const uint64_t idx = cand0 + (static_cast<uint64_t>(blockIdx.x) * kGenRounds + r) * kGenThreads +
-                         threadIdx.x;
-    const Candidate c = gen_candidate(p, regs, idx);
-    if (WRITE) {
-      int te, td;
-      const int re = block_rank(c.emitted, s_warp[0], te);
-      const int rd = block_rank(c.detected, s_warp[1], td);
-      const long long ei = e_base + re, di = d_base + rd;
-      const bool take = c.detected && (count_emissions ? ei < limit : di < limit);
-      if (take && di < capacity) {
+    const int local = r * kGenThreads + threadIdx.x;
+    const uint64_t idx = cand0 + static_cast<uint64_t>(blockIdx.x) * kGenPerBlock + local;
+    int d = gen_decide(p, regs, idx);
+    if (d == kGenUnsure) {
+      const Candidate c = gen_candidate(p, regs_g, idx);
+      d = c.detected ? kGenDetected : (c.emitted ? kGenEmitted : kGenNo);
+    }
+    __syncwarp();
+    const uint32_t me = __ballot_sync(0xffffffffu, d != kGenNo);
+    const uint32_t md = __ballot_sync(0xffffffffu, d == kGenDetected);
+    if (lane == 0) {
+      w[local >> 5] = me;
+      w[kGenWords + (local >> 5)] = md;
+    }
+    n_emit += __popc(me);
+    n_det += __popc(md);
+  }
+  if (lane == 0) {
+    s_count[0][warp] = n_emit;
+    s_count[1][warp] = n_det;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int te = 0, td = 0;
+    for (int k = 0; k < kGenThreads / 32; ++k) {
+      te += s_count[0][k];
+      td += s_count[1][k];
+    }
+    block_counts[blockIdx.x] = make_int2(te, td);
+  }
+}
+
+// Exclusive sums of the block counts after the earlier passes' totals, which
+// move on by this pass: one CTA.
+__global__ void __launch_bounds__(1024)
+    gen_scan_kernel(const int2* __restrict__ counts, int blocks, longlong2* __restrict__ base,
+                    longlong2* __restrict__ totals) {
+  __shared__ long long s_e[32], s_d[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  longlong2 run = *totals;
+  __syncthreads();
+  for (int b0 = 0; b0 < blocks; b0 += 1024) {
+    const int b = b0 + threadIdx.x;
+    const int2 c = b < blocks ? counts[b] : make_int2(0, 0);
+    long long ie = c.x, id = c.y;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long ve = __shfl_up_sync(0xffffffffu, ie, o), vd = __shfl_up_sync(0xffffffffu, id, o);
+      if (lane >= o) {
+        ie += ve;
+        id += vd;
+      }
+    }
+    if (lane == 31) {
+      s_e[warp] = ie;
+      s_d[warp] = id;
+    }
+    __syncthreads();
+    long long we = 0, wd = 0, te = 0, td = 0;
+    for (int k = 0; k < 32; ++k) {
+      we += k < warp ? s_e[k] : 0;
+      wd += k < warp ? s_d[k] : 0;
+      te += s_e[k];
+      td += s_d[k];
+    }
+    if (b < blocks) base[b] = make_longlong2(run.x + we + ie - c.x, run.y + wd + id - c.y);
+    run.x += te;
+    run.y += td;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *totals = run;
+}
+
+// Write pass: the block's accepted candidates (the detected ones; with EMITTED,
+// for count images of the emissions, all emitted ones) compacted into a list,
+// each evaluated once in FP64 and written at its rank.  Bound by the FP64 pipe.
+template <bool EMITTED>
+__global__ void __launch_bounds__(kGenThreads) gen_write_kernel(
+    GenParams p, const GenRegion* __restrict__ regs_g, uint64_t cand0,
+    const uint32_t* __restrict__ words, const longlong2* __restrict__ block_base, long long limit,
+    int count_emissions, long long capacity, unsigned long long* taken, float* __restrict__ out,
+    GenImages im) {
+  __shared__ GenRegion regs[kGenMaxRegions];
+  __shared__ uint32_t w_e[kGenWords], w_d[kGenWords];
+  __shared__ int p_e[kGenWords], p_d[kGenWords];  // set bits before each word
+  __shared__ uint16_t list[kGenPerBlock];
+  static_assert(kGenWords == 32, "one word per lane");
+  const int lane = threadIdx.x & 31;
+  const longlong2 base = block_base[blockIdx.x];
+  if ((count_emissions ? base.x : base.y) >= limit) return;  // past the last event
+  for (int i = threadIdx.x; i < p.n_regions; i += blockDim.x) regs[i] = regs_g[i];
+  if (threadIdx.x < 32) {
+    const uint32_t* w = words + static_cast<size_t>(blockIdx.x) * 2 * kGenWords;
+    const uint32_t e = w[lane], d = w[kGenWords + lane];
+    int ie = __popc(e), id = __popc(d);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int ve = __shfl_up_sync(0xffffffffu, ie, o), vd = __shfl_up_sync(0xffffffffu, id, o);
+      if (lane >= o) {
+        ie += ve;
+        id += vd;
+      }
+    }
+    w_e[lane] = e;
+    w_d[lane] = d;
+    p_e[lane] = ie - __popc(e);
+    p_d[lane] = id - __popc(d);
+  }
+  __syncthreads();
+  const uint32_t* w_l = EMITTED ? w_e : w_d;
+  const int* p_l = EMITTED ? p_e : p_d;
+  for (int c = threadIdx.x; c < kGenPerBlock; c += kGenThreads) {
+    const uint32_t w = w_l[c >> 5], bit = 1u << (c & 31);
+    if (w & bit) list[p_l[c >> 5] + __popc(w & (bit - 1u))] = static_cast<uint16_t>(c);
+  }
+  __syncthreads();
+  const int n = p_l[kGenWords - 1] + __popc(w_l[kGenWords - 1]);
+  unsigned long long n_taken = 0;
+  for (int k = threadIdx.x; k < n; k += kGenThreads) {
+    const int local = list[k], word = local >> 5;
+    const uint32_t below = (1u << (local & 31)) - 1u;
+    const long long ei = base.x + p_e[word] + __popc(w_e[word] & below);
+    const long long di = base.y + p_d[word] + __popc(w_d[word] & below);
+    if (!(count_emissions ? ei < limit : di < limit)) continue;
+    const uint64_t index = cand0 + static_cast<uint64_t>(blockIdx.x) * kGenPerBlock + local;
+    const Candidate c = EMITTED ? gen_candidate(p, regs, index) : gen_detected(p, regs, index);
+    if (c.detected) {
+      ++n_taken;
+      if (di < capacity) {
         out[3 * di] = c.zu;
         out[3 * di + 1] = c.zd;
         out[3 * di + 2] = c.dl;
@@ -284,43 +640,15 @@ __global__ void __launch_bounds__(kGenThreads) gen_kernel(
           im.events[4 * di + 3] = c.dir_y;
         }
       }
-      if (c.emitted && (count_emissions ? ei < limit : di < limit)) {
-        image_add(im.emitted, im, c.px, c.py);
-        if (take) {
-          image_add(im.detected, im, c.px, c.py);
-          if (im.naive || im.tan_map) naive_add(im, c.zu, c.zd, c.dl);
-        }
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, take);
-      if ((threadIdx.x & 31) == 0 && m) atomicAdd(taken, static_cast<unsigned long long>(__popc(m)));
-      e_base += te;
-      d_base += td;
-    } else {
-      n_emit += c.emitted;
-      n_det += c.detected;
+    }
+    image_add(im.emitted, im, c.px, c.py);
+    if (c.detected) {
+      image_add(im.detected, im, c.px, c.py);
+      if (im.naive || im.tan_map) naive_add(im, c.zu, c.zd, c.dl);
     }
   }
-  if (!WRITE) {
-    int te, td;
-    for (int o = 16; o > 0; o >>= 1) {
-      n_emit += __shfl_xor_sync(0xffffffffu, n_emit, o);
-      n_det += __shfl_xor_sync(0xffffffffu, n_det, o);
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-      s_warp[0][warp] = n_emit;
-      s_warp[1][warp] = n_det;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      te = td = 0;
-      for (int w = 0; w < kGenThreads / 32; ++w) {
-        te += s_warp[0][w];
-        td += s_warp[1][w];
-      }
-      block_counts[blockIdx.x] = make_int2(te, td);
-    }
-  }
+  n_taken = warp_add(n_taken);
+  if (lane == 0 && n_taken) atomicAdd(taken, n_taken);
 }
 
 constexpr double kPi = 3.14159265358979323846;
@@ -503,78 +831,85 @@ int jpet_strip_generate(const jpet_strip_geom* geom, const jpet_strip_region* re
   p.additive = (flags & JPET_GEN_ADDITIVE) ? 1 : 0;
 
   cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
-  const int blocks = 1024;  // 4 Mi candidates per pass
-  GenRegion* d_regs = nullptr;
-  int2* d_counts = nullptr;
-  long long* d_base = nullptr;
-  unsigned long long* d_taken = nullptr;
-  auto release = [&]() {
-    cudaFree(d_regs);
-    cudaFree(d_counts);
-    cudaFree(d_base);
-    cudaFree(d_taken);
-  };
+  // one allocation: block bases, block counts, totals, counter, regions, bits
+  const size_t o_counts = kGenMaxBlocks * sizeof(longlong2);
+  const size_t o_totals = o_counts + kGenMaxBlocks * sizeof(int2);
+  const size_t o_taken = o_totals + sizeof(longlong2);
+  const size_t o_regs = o_taken + 16;
+  const size_t o_words = (o_regs + regs.size() * sizeof(GenRegion) + 15) & ~static_cast<size_t>(15);
+  unsigned char* d = nullptr;
   auto fail = [&](cudaError_t e, const char* what) {
     set_call_error(std::string("jpet_strip_generate: ") + what + ": " + cudaGetErrorString(e));
-    release();
+    cudaFree(d);
     return JPET_ERR_CUDA;
   };
-  cudaError_t e = cudaMalloc(&d_regs, regs.size() * sizeof(GenRegion));
-  if (e == cudaSuccess) e = cudaMalloc(&d_counts, blocks * sizeof(int2));
-  if (e == cudaSuccess) e = cudaMalloc(&d_base, 2 * blocks * sizeof(long long));
-  if (e == cudaSuccess) e = cudaMalloc(&d_taken, sizeof(unsigned long long));
+  const long long limit = n;
+  // a pass takes the candidates that the events still missing should need; the
+  // first assumes that every candidate counts
+  auto blocks_for = [](double candidates) {
+    return static_cast<int>(std::min<double>(kGenMaxBlocks,
+                                             std::max(1.0, std::ceil(candidates / kGenPerBlock))));
+  };
+  cudaError_t e = cudaMalloc(&d, o_words + static_cast<size_t>(kGenMaxBlocks) * 2 * kGenWords *
+                                               sizeof(uint32_t));
   if (e != cudaSuccess) return fail(e, "cudaMalloc");
+  auto* d_base = reinterpret_cast<longlong2*>(d);
+  auto* d_counts = reinterpret_cast<int2*>(d + o_counts);
+  auto* d_totals = reinterpret_cast<longlong2*>(d + o_totals);
+  auto* d_taken = reinterpret_cast<unsigned long long*>(d + o_taken);
+  auto* d_regs = reinterpret_cast<GenRegion*>(d + o_regs);
+  auto* d_words = reinterpret_cast<uint32_t*>(d + o_words);
   e = cudaMemcpyAsync(d_regs, regs.data(), regs.size() * sizeof(GenRegion),
                       cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_taken, 0, sizeof(unsigned long long), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_totals, 0, o_regs - o_totals, s);
   if (e != cudaSuccess) return fail(e, "copy regions");
-  std::vector<int2> counts(blocks);
-  std::vector<long long> base(2 * blocks);
-  long long emitted = 0, det = 0;
-  uint64_t cand0 = 0;
-  const long long limit = n;
-  int idle_passes = 0;
-  while ((detected ? det : emitted) < limit) {
-    gen_kernel<false><<<blocks, kGenThreads, 0, s>>>(p, d_regs, cand0, d_counts, nullptr, 0, 0,
-                                                     0, nullptr, nullptr, GenImages{});
+  long long have = 0;  // events (or emissions) so far
+  uint64_t cand0 = 0, idle = 0;
+  int blocks = blocks_for(static_cast<double>(limit));
+  while (have < limit) {
+    gen_decide_kernel<<<blocks, kGenThreads, 0, s>>>(p, d_regs, cand0, d_words, d_counts);
+    gen_scan_kernel<<<1, 1024, 0, s>>>(d_counts, blocks, d_base, d_totals);
     e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(e, "count kernel");
-    e = cudaMemcpyAsync(counts.data(), d_counts, blocks * sizeof(int2), cudaMemcpyDeviceToHost, s);
+    if (e != cudaSuccess) return fail(e, "decision kernel");
+    if (im.emitted)
+      gen_write_kernel<true><<<blocks, kGenThreads, 0, s>>>(
+          p, d_regs, cand0, d_words, d_base, limit, detected ? 0 : 1, capacity, d_taken,
+          d_out_aos, im);
+    else
+      gen_write_kernel<false><<<blocks, kGenThreads, 0, s>>>(
+          p, d_regs, cand0, d_words, d_base, limit, detected ? 0 : 1, capacity, d_taken,
+          d_out_aos, im);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(e, "write kernel");
+    longlong2 totals;
+    e = cudaMemcpyAsync(&totals, d_totals, sizeof(totals), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return fail(e, "count pass");
-    long long e_run = emitted, d_run = det;
-    for (int b = 0; b < blocks; ++b) {
-      base[2 * b] = e_run;
-      base[2 * b + 1] = d_run;
-      e_run += counts[b].x;
-      d_run += counts[b].y;
-    }
-    e = cudaMemcpyAsync(d_base, base.data(), 2 * blocks * sizeof(long long),
-                        cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) return fail(e, "copy block offsets");
-    gen_kernel<true><<<blocks, kGenThreads, 0, s>>>(p, d_regs, cand0, nullptr, d_base, limit,
-                                                    detected ? 0 : 1, capacity, d_taken,
-                                                    d_out_aos, im);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // the offsets are reused next pass
-    if (e != cudaSuccess) return fail(e, "write pass");
-    if ((detected ? d_run - det : e_run - emitted) == 0) {
-      if (++idle_passes > 64) {
+    if (e != cudaSuccess) return fail(e, "generation pass");
+    const long long now = detected ? totals.y : totals.x;
+    const uint64_t candidates = static_cast<uint64_t>(blocks) * kGenPerBlock;
+    idle = now == have ? idle + candidates : 0;
+    have = now;
+    cand0 += candidates;
+    if (have == 0 || idle > 0) {
+      // 2^28 candidates in a row without one
+      if (idle > 64ull * kGenMaxBlocks * kGenPerBlock) {
         set_call_error("jpet_strip_generate: the regions give no events");
-        release();
+        cudaFree(d);
         return JPET_ERR_ARGUMENT;
       }
+      blocks = std::min(kGenMaxBlocks, 4 * blocks);
     } else {
-      idle_passes = 0;
+      // the accepted share so far, with four standard deviations on top
+      const double missing = static_cast<double>(limit - have);
+      blocks = blocks_for((missing + 4.0 * std::sqrt(missing + 1.0)) *
+                          static_cast<double>(cand0) / static_cast<double>(have));
     }
-    emitted = e_run;
-    det = d_run;
-    cand0 += static_cast<uint64_t>(blocks) * kGenPerBlock;
   }
   unsigned long long taken = 0;
-  e = cudaMemcpy(&taken, d_taken, sizeof(taken), cudaMemcpyDeviceToHost);
+  e = cudaMemcpyAsync(&taken, d_taken, sizeof(taken), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail(e, "copy counter");
-  release();
+  cudaFree(d);
   if (static_cast<long long>(taken) > capacity) {
     set_call_error("jpet_strip_generate: capacity below the detected events");
     return JPET_ERR_ARGUMENT;
