@@ -845,7 +845,7 @@ int jpet_strip_generate(const jpet_strip_geom* geom, const jpet_strip_region* re
   };
   const long long limit = n;
   // a pass takes the candidates that the events still missing should need; the
-  // first assumes that every candidate counts
+  // first assumes that two in five count (a decision costs a fraction of an event)
   auto blocks_for = [](double candidates) {
     return static_cast<int>(std::min<double>(kGenMaxBlocks,
                                              std::max(1.0, std::ceil(candidates / kGenPerBlock))));
@@ -865,7 +865,7 @@ int jpet_strip_generate(const jpet_strip_geom* geom, const jpet_strip_region* re
   if (e != cudaSuccess) return fail(e, "copy regions");
   long long have = 0;  // events (or emissions) so far
   uint64_t cand0 = 0, idle = 0;
-  int blocks = blocks_for(static_cast<double>(limit));
+  int blocks = blocks_for(2.5 * static_cast<double>(limit));
   while (have < limit) {
     gen_decide_kernel<<<blocks, kGenThreads, 0, s>>>(p, d_regs, cand0, d_words, d_counts);
     gen_scan_kernel<<<1, 1024, 0, s>>>(d_counts, blocks, d_base, d_totals);
