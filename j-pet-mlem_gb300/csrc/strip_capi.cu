@@ -216,9 +216,12 @@ UnionLimits union_limits(const jpet_strip_opts& o, int rows, int widest) {
   const UnionLimits m{kUnion64x32, 6144, 2, 2048};
   if (o.block_threads == 128) return UnionLimits{kUnion64x32n4, 6144, 4, 2048};
   if (o.block_threads == 256) return m;
-  if (rows <= 30 && widest <= 13) return UnionLimits{kUnion32x16, 3328, 5, 1024};
+  // a batch's rows are wider than its events' by a column of alignment and, at
+  // the ends of the box, by the spread of slopes in half a sort bucket
+  const bool narrow = widest + 1 + rows / 8 <= 16;
+  if (rows <= 30 && narrow) return UnionLimits{kUnion32x16, 3328, 5, 1024};
   if (rows <= 30 && widest <= 28) return UnionLimits{kUnion32x32, 3328, 4, 1024};
-  if (rows <= 64 && widest <= 13) return UnionLimits{kUnion64x16, 4096, 3, 1024};
+  if (rows <= 64 && narrow) return UnionLimits{kUnion64x16, 4096, 3, 1024};
   if (rows <= 64 && widest <= 28) return m;
   return UnionLimits{kUnion96x40, 10752, 1, 1024};
 }
@@ -228,7 +231,7 @@ UnionLimits union_limits(const jpet_strip_opts& o, int rows, int widest) {
 // tile whose window (tile + box) fits the shared-memory budget.
 void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
                    const std::vector<int32_t>& hh, int64_t n_nonempty, int n_sms, int n_y,
-                   int n_z, int widest, Tiling& t) {
+                   int n_z, int widest, double tallest, Tiling& t) {
   // window pixels per array (rho, out): 12288 (~100 KiB per CTA, 2 CTAs per SM)
   // for 256-thread CTAs; 6144 (~55 KiB, 4 CTAs per SM) for the row-owned
   // kernel's 128-thread CTAs; the batch-union kernel's from its batch shape
@@ -294,7 +297,9 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
   // order of a tile's events: for the batch-union kernel, tan buckets of 1/4 and
   // corner cells of 2 rows x 1 column; single pixels where many events share one
   // and the rows are short (the union of 16-column batches has no column to
-  // spare), wider cells and buckets where few do.  Pixel slots of the unions per
+  // spare) or where the tallest events leave the batch no row to spare (8e5 events
+  // of 63.5 rows: 2.54 slots with cells of two rows, 1.77 with one), wider cells
+  // and buckets where few share a pixel.  Pixel slots of the unions per
   // evaluated pixel, against the plain row-by-row order with buckets of 1/8:
   // 6e6 events at 1 mm 2.60 -> 1.84, 2e6 at 2 mm 2.00 -> 1.72, 1e6 at 5 mm
   // 2.62 -> 2.59 (2.70 with cells of two rows), 2e4 at 5 mm 6.7 -> 3.5 (4.0 with
@@ -303,7 +308,10 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
   t.tan_shift = 6;
   if (union_k) {
     const double per_px = static_cast<double>(n_nonempty) / (static_cast<double>(n_y) * n_z);
-    t.cell_h = per_px < 2.0 ? 3 : (t.union_shape == kUnion32x16 && per_px >= 6.0 ? 1 : 2);
+    const bool row_to_spare = tallest + 1.0 <= union_ops(t.union_shape).rows;
+    t.cell_h = !row_to_spare || (t.union_shape == kUnion32x16 && per_px >= 6.0) ? 1
+               : per_px < 2.0                                                   ? 3
+                                                                                : 2;
     t.cell_w = per_px < 2.0 ? 2 : 1;
     t.tan_shift = per_px < 2.0 ? 8 : 7;
   }
@@ -369,7 +377,8 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   int n_sms = 0;
   JPET_CUDA(h, cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, h->device),
             "cudaDeviceGetAttribute");
-  choose_tiling(h->opts, hw, hh, nonempty, n_sms, h->g.n_y, h->g.n_z, widest_row(h->g), h->tiling);
+  choose_tiling(h->opts, hw, hh, nonempty, n_sms, h->g.n_y, h->g.n_z, widest_row(h->g),
+                3.0 * h->g.sigma_dl / h->g.pixel_height, h->tiling);
   h->tiling.fast_shape = std::max(h->tiling.fast_shape, fast_width_shape(h->g));
   {
     int64_t tail = static_cast<int64_t>(std::floor(0.001 * nonempty)), acc_h = 0;
