@@ -224,8 +224,8 @@ int jpet_strip_nll_grad(jpet_strip_t* h, double sigma_z, double sigma_dl, const 
  * (rejected with JPET_ERR_ARGUMENT).  Work runs on cuda_stream (a cudaStream_t, NULL = the
  * default stream) in the reference's CPU float semantics and operation order;
  * no handle is involved.  It evaluates every box pixel in that order and adds
- * with global float atomics: on a GB300, 18 ms per iteration of 1048576 events
- * at 2 mm pixels (sigma 10 / 42 mm), about 17 times the time of a handle's
+ * with global float atomics: on a GB300, 4.6 ms per iteration of 1048576 events
+ * at 2 mm pixels (sigma 10 / 42 mm), about 6 times the time of a handle's
  * default kernel, which prepares its events into buffers it allocates.  The per-event working data live in one fixed 24 MiB
  * device array of the library, which every GPU that loads the library keeps
  * until the process exits; calls share it, so calls that overlap on the GPU

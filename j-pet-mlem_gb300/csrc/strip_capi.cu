@@ -71,6 +71,7 @@ struct jpet_strip {
   DevBuf<float> rho, out, sens_point, sens_pixel;
   DevBuf<float> out_lo;              // compensation image of the compensated modes
   DevBuf<unsigned long long> out_q;  // 64-bit fixed-point image of the FIXED mode
+  DevBuf<double> out_sum;            // image sums of the exact kernel (EXACT, GPU-reference)
   DevBuf<float> raw;                 // staging for uploaded events (kept for the next upload)
   DevBuf<float4> ev_geom, sorted_geom, over_geom;
   DevBuf<short4> ev_box, sorted_box, over_box;
@@ -315,7 +316,6 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
     t.cell_w = per_px < 2.0 ? 2 : 1;
     t.tan_shift = per_px < 2.0 ? 8 : 7;
   }
-  t.group = 32;
   // one spare entry per event for its widest row; a multiple of 8 entries so
   // that every event's table starts on a 16-byte boundary
   t.row_stride = (mh + 1 + 7) & ~7;
@@ -537,7 +537,12 @@ int iterate_on(jpet_strip* h, int n, cudaStream_t s) {
   const size_t n_pix = static_cast<size_t>(h->g.n_y) * h->g.n_z;
   const float* sens = h->sens_pixel.p;
   for (int it = 0; it < n; ++it) {
-    JPET_CUDA(h, cudaMemsetAsync(h->out.p, 0, n_pix * sizeof(float), s), "clear image");
+    // every variant adds into a cleared image: the exact kernel into its double one
+    const bool exact = h->out_sum.p != nullptr;
+    if (exact)
+      JPET_CUDA(h, cudaMemsetAsync(h->out_sum.p, 0, n_pix * sizeof(double), s), "clear image");
+    else
+      JPET_CUDA(h, cudaMemsetAsync(h->out.p, 0, n_pix * sizeof(float), s), "clear image");
     JPET_CUDA(h, cudaMemsetAsync(h->counters.p, 0, sizeof(DevCounters), s), "clear counters");
     const bool aux_img = h->opts.precision != JPET_PRECISION_FP32;
     const AuxImage aux{h->out_lo.p, h->out_q.p};
@@ -570,14 +575,22 @@ int iterate_on(jpet_strip* h, int n, cudaStream_t s) {
                   "iteration kernel launch");
       }
     } else {
-      JPET_CUDA(h, launch_iterate(h->g, h->tiling, h->opts.mode, h->chunks.p, h->n_chunks,
-                                  h->sorted_geom.p, h->sorted_box.p, h->rho.p, sens, h->out.p,
-                                  h->counters.p, s),
+      JPET_CUDA(h, launch_iterate_exact(h->g, h->opts.mode, h->n_sorted, h->sorted_geom.p,
+                                        h->sorted_box.p, h->rho.p, sens, h->out_sum.p,
+                                        h->counters.p, s),
                 "iteration kernel launch");
     }
-    JPET_CUDA(h, launch_iterate_global(h->g, h->opts.mode, h->n_oversize, h->over_geom.p,
-                                       h->over_box.p, h->rho.p, sens, h->out.p, h->counters.p, s),
-              "large-box kernel launch");
+    if (exact) {
+      JPET_CUDA(h, launch_iterate_exact(h->g, h->opts.mode, h->n_oversize, h->over_geom.p,
+                                        h->over_box.p, h->rho.p, sens, h->out_sum.p,
+                                        h->counters.p, s),
+                "large-box kernel launch");
+      JPET_CUDA(h, launch_round_image(h->out_sum.p, h->out.p, n_pix, s), "image rounding launch");
+    } else {
+      JPET_CUDA(h, launch_iterate_exact(h->g, h->opts.mode, h->n_oversize, h->over_geom.p,
+                                        h->over_box.p, h->rho.p, sens, h->out.p, h->counters.p, s),
+                "large-box kernel launch");
+    }
     if (aux_img)
       JPET_CUDA(h, launch_combine_aux(precision_code(h->opts.precision), aux, h->out.p, h->out.p,
                                       n_pix, s),
@@ -739,7 +752,9 @@ int jpet_strip_create(const jpet_strip_geom* geom, const jpet_strip_opts* opts,
   const size_t n_pix = static_cast<size_t>(h->g.n_y) * h->g.n_z;
   const bool comp = o.precision == JPET_PRECISION_COMPENSATED ||
                     o.precision == JPET_PRECISION_FP64_DEN;
+  const bool exact = o.mode == JPET_MODE_GPU_REFERENCE || o.variant == JPET_VARIANT_EXACT;
   if ((comp && h->out_lo.alloc(n_pix) != cudaSuccess) ||
+      (exact && h->out_sum.alloc(n_pix) != cudaSuccess) ||
       (o.precision == JPET_PRECISION_FIXED && h->out_q.alloc(n_pix) != cudaSuccess) ||
       h->rho.alloc(n_pix) != cudaSuccess || h->out.alloc(n_pix) != cudaSuccess ||
       h->sens_point.alloc(n_pix) != cudaSuccess || h->sens_pixel.alloc(n_pix) != cudaSuccess ||
@@ -770,6 +785,7 @@ int jpet_strip_destroy(jpet_strip_t* h) {
   h->out.release();
   h->out_lo.release();
   h->out_q.release();
+  h->out_sum.release();
   h->sens_point.release();
   h->sens_pixel.release();
   h->raw.release();

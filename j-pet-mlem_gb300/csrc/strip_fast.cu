@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(256) iterate_fast_kernel(
       if (ACC == kAccFloat) {
         process_event<kCpuReference>(g, 32, ev, box, acc, nullptr, dummy_calls, contrib);
       } else {
-        GlobalAccess gacc{rho, out, g.n_z};
+        GlobalAccess<float> gacc{rho, out, g.n_z};
         process_event<kCpuReference>(g, 32, ev, box, gacc, nullptr, dummy_calls, contrib);
       }
       continue;

@@ -40,7 +40,6 @@ struct Tiling {
   int32_t n_tiles_x, n_tiles_y;
   int32_t chunk_events;    // events per chunk
   int32_t threads;         // threads per CTA
-  int32_t group;           // lanes per image row in the warp rasteriser (8/16/32)
   int32_t row_stride;      // entries per event in the row table (>= max_box_h, even)
   int32_t fast_shape;      // register-cache shape of the warp-per-event kernel (FastShape)
   int32_t rows_shape;      // register-cache shape of the row-owned kernel (RowsShape)
@@ -249,14 +248,14 @@ cudaError_t launch_nll_finish(const float* sens, const float* rho, float* grad, 
 // out holds the contributions of events taken by the reference-order paths).
 cudaError_t launch_combine_aux(int precision, AuxImage aux, const float* out, float* rho,
                                int64_t n, cudaStream_t s);
-cudaError_t launch_iterate(const DevGeom& g, const Tiling& t, int32_t semantics,
-                           const Chunk* chunks, int32_t n_chunks, const float4* ev_geom,
-                           const short4* ev_box, const float* rho, const float* sens,
-                           float* out, DevCounters* counters, cudaStream_t s);
-cudaError_t launch_iterate_global(const DevGeom& g, int32_t semantics, int32_t n_events,
-                                  const float4* ev_geom, const short4* ev_box,
-                                  const float* rho, const float* sens, float* out,
-                                  DevCounters* counters, cudaStream_t s);
+// The iteration in the reference's operation order into an image of Sum (float or
+// double), and a double image rounded to float.
+template <class Sum>
+cudaError_t launch_iterate_exact(const DevGeom& g, int32_t semantics, int32_t n_events,
+                                 const float4* ev_geom, const short4* ev_box, const float* rho,
+                                 const float* sens, Sum* out, DevCounters* counters,
+                                 cudaStream_t s);
+cudaError_t launch_round_image(const double* in, float* out, int64_t n, cudaStream_t s);
 cudaError_t launch_sensitivity(const DevGeom& g, int kind, float* out, cudaStream_t s);
 
 }  // namespace jpet

@@ -121,8 +121,8 @@ int jpet_strip_iterate_noalloc(const jpet_strip_geom* geom, const float* d_respo
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && n > 0)
-    e = launch_iterate_global(g, kCpuReference, static_cast<int32_t>(n), sc->geom, sc->box,
-                              d_rho_in, nullptr, d_rho_out, &sc->counters, s);
+    e = launch_iterate_exact(g, kCpuReference, static_cast<int32_t>(n), sc->geom, sc->box, d_rho_in,
+                             nullptr, d_rho_out, &sc->counters, s);
   if (e != cudaSuccess) {
     set_call_error(std::string("jpet_strip_iterate_noalloc: ") + cudaGetErrorString(e));
     return JPET_ERR_CUDA;

@@ -40,13 +40,14 @@ struct WindowAccess {
   }
 };
 
+template <class Sum>
 struct GlobalAccess {
   const float* rho;
-  float* out;
+  Sum* out;
   int n_z;
   __device__ __forceinline__ float rho_at(int y, int x) const { return __ldg(&rho[y * n_z + x]); }
   __device__ __forceinline__ void add(int y, int x, float v) const {
-    atomicAdd(&out[y * n_z + x], v);
+    atomicAdd(&out[y * n_z + x], static_cast<Sum>(v));
   }
 };
 

@@ -328,7 +328,7 @@ __device__ __forceinline__ void rows_chunk(
       WindowAccess acc{w_rho, w_out, ox, c.oy, pitch};
       process_event<kCpuReference>(g, 32, ev, box, acc, nullptr, dummy_calls, contrib);
     } else {
-      GlobalAccess gacc{rho, out, g.n_z};
+      GlobalAccess<float> gacc{rho, out, g.n_z};
       process_event<kCpuReference>(g, 32, ev, box, gacc, nullptr, dummy_calls, contrib);
     }
   }

@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
       // the other modes' windows hold compensated or integer sums: these events
       // add into the FP32 image directly (combined with the second image after
       // the iteration)
-      GlobalAccess gacc{rho, out, g.n_z};
+      GlobalAccess<float> gacc{rho, out, g.n_z};
       process_event<kCpuReference>(g, 32, ev_geom[ei], ev_box[ei], gacc, nullptr, dummy_calls,
                                    contrib);
     }
