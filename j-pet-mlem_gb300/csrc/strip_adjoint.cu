@@ -18,22 +18,31 @@
 // constant is rounded differently at sigma +- h, and a float rounding of, e.g.,
 // ipd shifts log K of every pixel in the same direction.  So the kernel value
 // uses the accurate exp2f (not the .approx form of the MLEM kernel), the row
-// prefactor -log2(aMa(py)/aMa(y))/2 - 2 log2(e) ipd sec^2 dy^2 is computed in
-// FP64 from FP64 constants, the per-pixel coefficient kz = -log2(e) ipz is
-// applied as a float pair (kz + kz_lo), and the event constant
+// prefactor -log2(aMa(py)/aMa(y))/2 - 2 log2(e) ipd sec^2 dy^2 is computed to ~1e-9
+// of itself and rounded to float once, the per-pixel coefficient kz = -log2(e)
+// ipz is applied as a float pair (kz + kz_lo), and the event constant
 // log(c0 / sqrt(aMa(y))) enters the loss in FP64.
 //
-// One warp per event; each row's exact in-ellipse interval is found with the
-// same search as the MLEM row tables (row_interval), so the support is exactly
-// the reference's.  The rows' constants are set up 32 at a time, one row per
-// lane, and broadcast to the warp for the row's pixels; the constants of the
-// first 128 rows are kept in registers for the second (gradient) pass.  For the
-// events of the tiled chunks the rho window and a
-// gradient window live in shared memory (as in the MLEM kernel); events whose
-// box exceeds the windows use the global image.  Per-event log-likelihood and
-// sigma-derivative terms are reduced in FP64 per CTA.
+// One warp per event.  The lanes set up a block of rows, 32 at a time and one each
+// (the exact in-ellipse interval of the MLEM row tables, so the support is exactly
+// the reference's, read from the row table where the handle has one, and the row's
+// terms), then sweep the rows with 8, 16 or 32 lanes each; the first kNllCache
+// kernel values are kept for the gradient pass, which adds them with
+// float reductions to one of a few partial images (many small additions to one
+// float image lose digits; nll_finish_kernel sums the partial images in FP64).
+//
+// This GPU's FP64 pipe is a sixty-fourth of its FP32 one, so FP64 is left where
+// one lane's instruction serves one event: a warp takes `group` events, lane j
+// prepares event j's FP64 constants before and forms its logarithm and quotients
+// after; the row prefactor and the sums over lanes are double-float (pairs of
+// FP32 values, Dekker 1971; the sum and product errors are Knuth's TwoSum and an
+// FMA).  5e5 events of 1763 pixels (2 mm, support 14 / 55): 8.0 ms with FP64 row
+// terms and per-event FP64 on one lane (FP64 pipe 70-81 % busy) and float
+// atomics on windows in shared memory, 3.65 ms now (FP64 pipe 3 %), bound by
+// instruction issue (63 % of the slots, 52 instructions a pixel for both passes).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 
@@ -45,208 +54,298 @@ namespace jpet {
 namespace {
 
 constexpr double kNllLog2e = 1.4426950408889634;
+constexpr int kNllWarps = 4;     // warps per CTA
+constexpr int kNllCache = 1536;  // kernel values kept per event
+constexpr int kNllRows = 96;     // rows of a block (an event's set-up is then kept for the
+                                 // gradient pass)
 
-struct NllWindow {
-  const float* rho;
-  float* grad;
-  int ox, oy, pitch;
-  __device__ __forceinline__ int index(int y, int x) const { return (y - oy) * pitch + (x - ox); }
+// ---- double-float arithmetic: h + l, |l| <= ulp(h) / 2 ---------------------------------
+struct Pair {
+  float h, l;
+};
+__device__ __forceinline__ Pair pair_of(double v) {
+  const float h = __double2float_rn(v);
+  return Pair{h, __double2float_rn(v - static_cast<double>(h))};
+}
+__device__ __forceinline__ Pair two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b), v = __fsub_rn(s, a);
+  return Pair{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, v)), __fsub_rn(b, v))};
+}
+__device__ __forceinline__ Pair two_prod(float a, float b) {
+  const float p = __fmul_rn(a, b);
+  return Pair{p, __fmaf_rn(a, b, -p)};
+}
+__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
+  Pair p = two_prod(a.h, b.h);
+  p.l = __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, p.l));
+  return p;
+}
+__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
+  Pair s = two_sum(a.h, b.h);
+  s.l = __fadd_rn(s.l, __fadd_rn(a.l, b.l));
+  return s;
+}
+// sum over the warp's lanes
+__device__ __forceinline__ Pair pair_warp_sum(float v) {
+  Pair s{v, 0.0f};
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const Pair other{__shfl_xor_sync(kFull, s.h, o), __shfl_xor_sync(kFull, s.l, o)};
+    s = pair_add(s, other);
+  }
+  return s;
+}
+
+// -log2(1 + x) / 2 for |x| up to about 1: log(1 + x) = 2 artanh(r), r = x / (2 + x),
+// with the first term of the series in r a double-float; relative error below
+// 5e-9 (the float part of the series is at most a twentieth of the whole).
+__device__ __forceinline__ Pair half_neg_log2_1p(Pair x) {
+  Pair d = two_sum(2.0f, x.h);
+  d.l = __fadd_rn(d.l, x.l);
+  const float inv = __frcp_rn(d.h);
+  const float q = __fmul_rn(x.h, inv);
+  const float rem = __fadd_rn(__fmaf_rn(-q, d.h, x.h), __fmaf_rn(-q, d.l, x.l));
+  Pair r{q, __fmul_rn(rem, inv)};
+  const float z = q * q;
+  float s = 1.0f / 19.0f;
+  s = fmaf(s, z, 1.0f / 17.0f);
+  s = fmaf(s, z, 1.0f / 15.0f);
+  s = fmaf(s, z, 1.0f / 13.0f);
+  s = fmaf(s, z, 1.0f / 11.0f);
+  s = fmaf(s, z, 1.0f / 9.0f);
+  s = fmaf(s, z, 1.0f / 7.0f);
+  s = fmaf(s, z, 1.0f / 5.0f);
+  s = fmaf(s, z, 1.0f / 3.0f);
+  r.l = __fmaf_rn(__fmul_rn(q, z), s, r.l);
+  // -log2(e), twice artanh and half of it
+  constexpr double c = -kNllLog2e;
+  constexpr float ch = static_cast<float>(c);
+  constexpr float cl = static_cast<float>(c - static_cast<double>(ch));
+  return pair_mul(r, Pair{ch, cl});
+}
+
+struct NllWarp {
+  float4 row[kNllRows];     // prefactor exponent, d/dipz and d/dipd terms, u at column 0
+  int4 at[kNllRows];        // pixels before the row | width << 16, image index of its first
+                            // pixel, first column (float bits), unused
+  float cache[kNllCache];   // kernel values
 };
 
-// One event on one warp: forward sums (den, d den / d sigma) and, if den > 0,
-// the gradient contributions -K / den; returns the per-event terms on lane 0.
-template <class Win>
-__device__ __forceinline__ void nll_event(const DevGeom& g, const NllConst& k, float4 ev,
-                                          short4 box, const Win& wv, double& loss, double& gz,
-                                          double& gdl, unsigned long long& skipped) {
+template <bool GRAD, bool TABLE>
+__global__ void __launch_bounds__(32 * kNllWarps) nll_kernel(
+    DevGeom g, NllConst k, int32_t n, int32_t group, const float4* __restrict__ ev_geom,
+    const short4* __restrict__ ev_box, const uint16_t* __restrict__ table, int32_t stride,
+    const float* __restrict__ rho, float* __restrict__ parts, int32_t n_parts, int64_t n_pix, double* __restrict__ acc, unsigned long long* skipped) {
+  __shared__ NllWarp shared[kNllWarps];
+  NllWarp& s = shared[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const float z = ev.x, y = ev.y, tn = ev.z, sec = ev.w;
-  float A, B, C;
-  ellipse_abc(g, tn, sec, A, B, C);
-  const float sec2 = sec * sec;
-  const float pa_c = 2.0f * sec2 * sec2;     // Pa = pa_c (py^2 + R^2)
-  const float qa_c = 4.0f * sec2 * tn * tn;  // Qa = qa_c py^2
-  const double ama_ref_d =
-      (static_cast<double>(pa_c) * (static_cast<double>(y) * y +
-                                    static_cast<double>(g.radius) * g.radius)) * k.ipz_d +
-      static_cast<double>(qa_c) * y * y * k.ipd_d;
-  // aMa(py) / aMa(y) = 1 + qq (py - y)(py + y)
-  const double qq = (pa_c * k.ipz_d + qa_c * k.ipd_d) / ama_ref_d;
-  const double kdl_sec2 = k.kdl_d * sec2;
-  const int nrows = box.w - box.y;
-  float den = 0.0f, dz = 0.0f, ddl = 0.0f, inv = 0.0f;
-  // lane l sets up row rb + l: exact interval and FP64 row term
-  struct RowConst {
-    int first, w;
-    float arg, cz, cdl, u;
-  };
-  auto setup = [&](int rb) {
-    RowConst c{0, 0, 0.0f, 0.0f, 0.0f, 0.0f};
-    const int ri = rb + lane;
-    if (ri < nrows) {
-      const int iy = box.y + ri;
-      c.w = row_interval(g, A, B, C, z, y, tn, sec, box.x, box.z, iy, c.first);
-      const float py = g.tl_y_half_h - static_cast<float>(iy) * g.pixel_height;
-      const float dy = py - y;
-      const float pa = pa_c * (py * py + g.radius * g.radius), qa = qa_c * py * py;
-      const float ama = pa * k.ipz + qa * k.ipd;
-      const double dyd = dy;
-      c.arg = static_cast<float>(-0.5 * kNllLog2e * log1p(qq * dyd * (static_cast<double>(py) + y)) +
-                                 kdl_sec2 * dyd * dyd);
-      c.cz = k.inv_ipz - 0.5f * pa / ama;
-      c.cdl = k.half_inv_ipd - 0.5f * qa / ama - 2.0f * sec2 * dy * dy;
-      c.u = g.tl_z_half_w - z - dy * tn;
-    }
-    return c;
-  };
-  // the warp sweeps the group's rows one by one with the constants broadcast
-  // from their lanes: forward sums (pass 0) or gradient contributions (pass 1)
-  auto sweep = [&](int pass, int rb, const RowConst& c) {
-    const int n_group = min(32, nrows - rb);
-    for (int r = 0; r < n_group; ++r) {
-      const int wr = __shfl_sync(kFull, c.w, r);
-      if (wr == 0) continue;
-      const int fr = __shfl_sync(kFull, c.first, r);
-      const float ra = __shfl_sync(kFull, c.arg, r);
-      const float czr = __shfl_sync(kFull, c.cz, r);
-      const float cdr = __shfl_sync(kFull, c.cdl, r);
-      const float ur = __shfl_sync(kFull, c.u, r);
-      const int iy = box.y + rb + r;
-      for (int j = lane; j < wr; j += 32) {
-        const int col = fr + j;
-        const float u = fmaf(static_cast<float>(col), g.pixel_width, ur);
-        const float kv = exp2f(fmaf(k.kz * u, u, fmaf(k.kz_lo * u, u, ra)));
-        const int wi = wv.index(iy, col);
-        if (pass == 0) {
-          const float kr = kv * wv.rho[wi];
-          den += kr;
-          dz += kr * (czr - u * u);
-          ddl += kr * cdr;
-        } else {
-          atomicAdd(&wv.grad[wi], -kv * inv);
-        }
-      }
-    }
-  };
-  // the constants of up to kCachedGroups x 32 rows stay in registers between
-  // the two passes; taller boxes set their rows up again in the second pass
-  constexpr int kCachedGroups = 4;
-  RowConst cache[kCachedGroups];
-  for (int pass = 0; pass < 2; ++pass) {
-    if (pass == 1) {
-      dz *= k.dipz_dsz;
-      ddl *= k.dipd_dsdl;
-      double dd = den, dzz = dz, ddd = ddl;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        dd += __shfl_xor_sync(kFull, dd, o);
-        dzz += __shfl_xor_sync(kFull, dzz, o);
-        ddd += __shfl_xor_sync(kFull, ddd, o);
-      }
-      if (!(dd > 0.0)) {
-        if (lane == 0) ++skipped;
-        return;
-      }
-      if (lane == 0) {
-        // log of the absolute denominator: K = K_ref K', K_ref = c0 / sqrt(aMa(y))
-        loss -= log(dd) + k.log_c0 - 0.5 * log(ama_ref_d);
-        gz -= dzz / dd;
-        gdl -= ddd / dd;
-      }
-      inv = static_cast<float>(1.0 / dd);
-    }
-#pragma unroll 1
-    for (int rb = 0; rb < nrows; rb += 32) {
-      const int gi = rb >> 5;
-      RowConst c;
-      if (gi >= kCachedGroups || pass == 0) {
-        c = setup(rb);
-        if (gi < kCachedGroups) cache[gi] = c;
-      } else {
-        c = cache[gi];
-      }
-      sweep(pass, rb, c);
-    }
-  }
-}
-
-__device__ __forceinline__ void nll_block_reduce(double loss, double gz, double gdl,
-                                                 unsigned long long sk, double* s_acc,
-                                                 double* acc, unsigned long long* skipped) {
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&s_acc[0], loss);
-    atomicAdd(&s_acc[1], gz);
-    atomicAdd(&s_acc[2], gdl);
-    if (sk) atomicAdd(skipped, sk);
-  }
-  __syncthreads();
-  if (threadIdx.x < 3) atomicAdd(&acc[threadIdx.x], s_acc[threadIdx.x]);
-}
-
-__global__ void __launch_bounds__(256) nll_grad_tiles_kernel(
-    DevGeom g, NllConst k, Tiling t, const Chunk* __restrict__ chunks,
-    const float4* __restrict__ ev_geom, const short4* __restrict__ ev_box,
-    const float* __restrict__ rho, float* __restrict__ grad, double* __restrict__ acc,
-    unsigned long long* skipped) {
-  extern __shared__ __align__(16) float smem[];
-  const int pitch = t.win_w;
-  const int win = t.win_w * t.win_h;
-  float* w_rho = smem;
-  float* w_grad = smem + win;
-  __shared__ double s_acc[3];
-  const Chunk c = chunks[blockIdx.x];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-  if (threadIdx.x < 3) s_acc[threadIdx.x] = 0.0;
-  for (int r = warp; r < t.win_h; r += n_warps) {
-    const int gy = c.oy + r;
-    for (int col = lane; col < pitch; col += 32) {
-      const int gx = c.ox + col;
-      w_rho[r * pitch + col] = (gy < g.n_y && gx < g.n_z) ? rho[gy * g.n_z + gx] : 0.0f;
-      w_grad[r * pitch + col] = 0.0f;
-    }
-  }
-  __syncthreads();
-  NllWindow wv{w_rho, w_grad, c.ox, c.oy, pitch};
-  double loss = 0.0, gz = 0.0, gdl = 0.0;
-  unsigned long long sk = 0;
-  for (int e = warp; e < c.count; e += n_warps)
-    nll_event(g, k, ev_geom[c.start + e], ev_box[c.start + e], wv, loss, gz, gdl, sk);
-  nll_block_reduce(loss, gz, gdl, sk, s_acc, acc, skipped);
-  for (int r = warp; r < t.win_h; r += n_warps) {
-    const int gy = c.oy + r;
-    for (int col = lane; col < pitch; col += 32) {
-      const int gx = c.ox + col;
-      const float v = w_grad[r * pitch + col];
-      if (v != 0.0f && gy < g.n_y && gx < g.n_z) atomicAdd(&grad[gy * g.n_z + gx], v);
-    }
-  }
-}
-
-__global__ void __launch_bounds__(256) nll_grad_global_kernel(
-    DevGeom g, NllConst k, int32_t n, const float4* __restrict__ ev_geom,
-    const short4* __restrict__ ev_box, const float* __restrict__ rho, float* __restrict__ grad,
-    double* __restrict__ acc, unsigned long long* skipped) {
-  __shared__ double s_acc[3];
-  if (threadIdx.x < 3) s_acc[threadIdx.x] = 0.0;
-  __syncthreads();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int n_warps = (gridDim.x * blockDim.x) >> 5;
-  NllWindow wv{rho, grad, 0, 0, g.n_z};
+  float* grad = GRAD ? parts + static_cast<int64_t>(blockIdx.x % n_parts) * n_pix : nullptr;
   double loss = 0.0, gz = 0.0, gdl = 0.0;
   unsigned long long sk = 0;
-  for (int e = warp; e < n; e += n_warps) nll_event(g, k, ev_geom[e], ev_box[e], wv, loss, gz, gdl, sk);
-  nll_block_reduce(loss, gz, gdl, sk, s_acc, acc, skipped);
+  for (int64_t e0 = static_cast<int64_t>(warp) * group; e0 < n;
+       e0 += static_cast<int64_t>(n_warps) * group) {
+    const int cnt = static_cast<int>(e0 + group <= n ? group : n - e0);
+    // lane j: event e0 + j
+    float4 ev = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    short4 bx = make_short4(0, 0, 0, 0);
+    Pair qq{0.0f, 0.0f}, kd{0.0f, 0.0f};
+    double log_ref = 0.0;  // log(c0 / sqrt(aMa(y)))
+    if (lane < cnt) {
+      ev = ev_geom[e0 + lane];
+      bx = ev_box[e0 + lane];
+      const float y = ev.y, sec2 = ev.w * ev.w;
+      const float pa_c = 2.0f * sec2 * sec2, qa_c = 4.0f * sec2 * ev.z * ev.z;
+      const double ama =
+          (static_cast<double>(pa_c) * (static_cast<double>(y) * y +
+                                        static_cast<double>(g.radius) * g.radius)) * k.ipz_d +
+          static_cast<double>(qa_c) * y * y * k.ipd_d;
+      // aMa(py) / aMa(y) = 1 + qq (py - y)(py + y)
+      qq = pair_of((pa_c * k.ipz_d + qa_c * k.ipd_d) / ama);
+      kd = pair_of(k.kdl_d * sec2);
+      log_ref = k.log_c0 - 0.5 * log(ama);
+    }
+    Pair den_j{0.0f, 0.0f}, dz_j{0.0f, 0.0f}, ddl_j{0.0f, 0.0f};
+    for (int j = 0; j < cnt; ++j) {
+      const float z = __shfl_sync(kFull, ev.x, j), y = __shfl_sync(kFull, ev.y, j);
+      const float tn = __shfl_sync(kFull, ev.z, j), sec = __shfl_sync(kFull, ev.w, j);
+      const int b0 = __shfl_sync(kFull, static_cast<int>(bx.x) | (static_cast<int>(bx.y) << 16), j);
+      const int b1 = __shfl_sync(kFull, static_cast<int>(bx.z) | (static_cast<int>(bx.w) << 16), j);
+      const int bx0 = b0 & 0xffff, by0 = b0 >> 16, bx1 = b1 & 0xffff, by1 = b1 >> 16;
+      const Pair q{__shfl_sync(kFull, qq.h, j), __shfl_sync(kFull, qq.l, j)};
+      const Pair kdl{__shfl_sync(kFull, kd.h, j), __shfl_sync(kFull, kd.l, j)};
+      float A, B, C;
+      ellipse_abc(g, tn, sec, A, B, C);
+      const float sec2 = sec * sec;
+      const float pa_c = 2.0f * sec2 * sec2;     // Pa = pa_c (py^2 + R^2)
+      const float qa_c = 4.0f * sec2 * tn * tn;  // Qa = qa_c py^2
+      const int nrows = by1 - by0;
+      // rows per block
+      const int step = nrows <= kNllRows ? kNllRows : 32;
+      int n_rows = 0, total = 0, widest = 0;  // of the block last set up: rows with pixels
+      auto setup = [&](int rb) {
+        n_rows = total = widest = 0;
+        __syncwarp();
+        for (int r0 = rb; r0 < min(rb + step, nrows); r0 += 32) {
+          int first = 0, w = 0;
+          const int iy = by0 + r0 + lane;
+          if (r0 + lane < nrows) {
+            if (TABLE) {
+              const uint32_t e = table[(e0 + j) * stride + r0 + lane];
+              first = bx0 + static_cast<int>(e & 255u);
+              w = static_cast<int>(e >> 8);
+            } else {
+              w = row_interval(g, A, B, C, z, y, tn, sec, bx0, bx1, iy, first);
+            }
+          }
+          int off = w;  // inclusive sum of the widths
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFull, off, o);
+            if (lane >= o) off += v;
+          }
+          const int sum = __shfl_sync(kFull, off, 31);
+          off += total - w;
+          total += sum;
+          widest = max(widest, static_cast<int>(__reduce_max_sync(kFull, static_cast<unsigned>(w))));
+          const unsigned rows = __ballot_sync(kFull, w > 0);
+          if (w > 0) {
+            const int r = n_rows + __popc(rows & ((1u << lane) - 1u));
+            const float py = g.tl_y_half_h - static_cast<float>(iy) * g.pixel_height;
+            const float dy = py - y;
+            const float pa = pa_c * (py * py + g.radius * g.radius), qa = qa_c * py * py;
+            const float ama = pa * k.ipz + qa * k.ipd;
+            // x = qq dy (py + y)
+            const Pair ys = two_sum(py, y);
+            Pair x = two_prod(dy, ys.h);
+            x.l = __fmaf_rn(dy, ys.l, x.l);
+            x = pair_mul(x, q);
+            Pair a = half_neg_log2_1p(x);
+            if (!(fabsf(x.h) <= 0.9f))  // beyond the series
+              a = pair_of(-0.5 * kNllLog2e *
+                          log1p(static_cast<double>(x.h) + static_cast<double>(x.l)));
+            a = pair_add(a, pair_mul(two_prod(dy, dy), kdl));
+            s.row[r] = make_float4(__fadd_rn(a.h, a.l), k.inv_ipz - 0.5f * pa / ama,
+                                   k.half_inv_ipd - 0.5f * qa / ama - 2.0f * sec2 * dy * dy,
+                                   g.tl_z_half_w - z - dy * tn);
+            s.at[r] = make_int4(min(off, kNllCache) | (w << 16), iy * g.n_z + first,
+                                __float_as_int(static_cast<float>(first)), 0);
+          }
+          n_rows += __popc(rows);
+        }
+        __syncwarp();
+      };
+      // f(row, its record, pixel of the row, that as a float, whether there is such a
+      // pixel) over a block's pixels: as many lanes per row as fit the widest, four
+      // rows in flight, lanes past a row's end along without a branch
+      auto walk = [&](auto&& f) {
+        const int sh = widest <= 8 ? 3 : widest <= 16 ? 4 : 5;
+        const int l = lane & ((1 << sh) - 1);
+        const float fl = static_cast<float>(l);
+#pragma unroll 4
+        for (int r0 = 0; r0 < n_rows; r0 += 32 >> sh) {
+          const int r = min(r0 + (lane >> sh), n_rows - 1);
+          const int4 at = s.at[r];
+          f(r, at, l, fl, l < (at.x >> 16) && r == r0 + (lane >> sh));
+        }
+        if (widest > 32) {
+          for (int r = 0; r < n_rows; ++r) {
+            const int4 at = s.at[r];
+            for (int i = lane + 32; i < (at.x >> 16); i += 32)
+              f(r, at, i, static_cast<float>(i), true);
+          }
+        }
+      };
+      auto value = [&](const float4 r, float col, float& u) {
+        u = fmaf(col, g.pixel_width, r.w);
+        return exp2f(fmaf(k.kz * u, u, fmaf(k.kz_lo * u, u, r.x)));
+      };
+      float den = 0.0f, dz = 0.0f, ddl = 0.0f;
+      int before = 0;  // pixels of the blocks before
+      for (int rb = 0; rb < nrows; rb += step) {
+        setup(rb);
+        walk([&](int r, const int4 at, int i, float fi, bool in) {
+          const float4 row = s.row[r];
+          const float rh = in ? __ldg(&rho[at.y + i]) : 0.0f;
+          float u;
+          const float kv = value(row, __int_as_float(at.z) + fi, u);
+          const float kr = in ? kv * rh : 0.0f;
+          den += kr;
+          dz += kr * (row.y - u * u);
+          ddl += kr * row.z;
+          const int c = before + (at.x & 0xffff) + i;
+          if (GRAD && in && c < kNllCache) s.cache[c] = kv;
+        });
+        before = min(before + total, kNllCache);
+      }
+      const Pair d = pair_warp_sum(den);
+      const Pair a = pair_warp_sum(dz * k.dipz_dsz), b = pair_warp_sum(ddl * k.dipd_dsdl);
+      if (lane == j) {
+        den_j = d;
+        dz_j = a;
+        ddl_j = b;
+      }
+      if (!GRAD || !(d.h > 0.0f)) continue;
+      const float i0 = __frcp_rn(d.h);
+      const float inv = fmaf(fmaf(-d.h, i0, 1.0f) - d.l * i0, i0, i0);
+      before = 0;
+      for (int rb = 0; rb < nrows; rb += step) {
+        if (nrows > step) setup(rb);
+        walk([&](int r, const int4 at, int i, float fi, bool in) {
+          const int c = before + (at.x & 0xffff) + i;
+          float u;
+          float kv = s.cache[min(c, kNllCache - 1)];
+          if (in && c >= kNllCache) kv = value(s.row[r], __int_as_float(at.z) + fi, u);
+          if (in) atomicAdd(&grad[at.y + i], -kv * inv);
+        });
+        before = min(before + total, kNllCache);
+      }
+      __syncwarp();  // the next event's set-up overwrites the rows
+    }
+    if (lane < cnt) {
+      const double dd = static_cast<double>(den_j.h) + static_cast<double>(den_j.l);
+      if (dd > 0.0) {
+        // log of the absolute denominator: K = K_ref K', K_ref = c0 / sqrt(aMa(y))
+        loss -= log(dd) + log_ref;
+        const double inv = 1.0 / dd;
+        gz -= (static_cast<double>(dz_j.h) + static_cast<double>(dz_j.l)) * inv;
+        gdl -= (static_cast<double>(ddl_j.h) + static_cast<double>(ddl_j.l)) * inv;
+      } else {
+        ++sk;
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    loss += __shfl_xor_sync(kFull, loss, o);
+    gz += __shfl_xor_sync(kFull, gz, o);
+    gdl += __shfl_xor_sync(kFull, gdl, o);
+  }
+  sk = warp_sum_u64(sk);
+  if (lane == 0) {
+    atomicAdd(&acc[0], loss);
+    atomicAdd(&acc[1], gz);
+    atomicAdd(&acc[2], gdl);
+    if (sk) atomicAdd(skipped, sk);
+  }
 }
 
-// grad += s; acc[0] += sum s * rho
+// grad = s + the partial images; acc[0] += sum s * rho
 __global__ void nll_finish_kernel(const float* __restrict__ s, const float* __restrict__ rho,
+                                  const float* __restrict__ parts, int32_t n_parts,
                                   float* __restrict__ grad, double* acc, int64_t n) {
   __shared__ double part[8];
   double v = 0.0;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    v += static_cast<double>(s[i]) * rho[i];
-    if (grad) grad[i] += s[i];
+    const float si = s[i];
+    v += static_cast<double>(si) * rho[i];
+    if (grad) {
+      double t = si;
+      for (int32_t p = 0; p < n_parts; ++p) t += parts[p * n + i];
+      grad[i] = __double2float_rn(t);
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
@@ -280,33 +379,31 @@ NllConst make_nll_const(double sigma_z, double sigma_dl) {
   return k;
 }
 
-cudaError_t launch_nll_grad(const DevGeom& g, const NllConst& k, const Tiling& t,
-                            const Chunk* chunks, int32_t n_chunks, const float4* ev_geom,
-                            const short4* ev_box, int32_t n_over, const float4* over_geom,
-                            const short4* over_box, const float* rho, float* grad, double* acc,
-                            unsigned long long* skipped, cudaStream_t s) {
-  if (n_chunks > 0) {
-    const size_t smem = 2ull * t.win_w * t.win_h * sizeof(float);
-    cudaError_t err = cudaFuncSetAttribute(nll_grad_tiles_kernel,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(smem));
-    if (err != cudaSuccess) return err;
-    nll_grad_tiles_kernel<<<n_chunks, 256, smem, s>>>(g, k, t, chunks, ev_geom, ev_box, rho, grad,
-                                                      acc, skipped);
-    if ((err = cudaGetLastError()) != cudaSuccess) return err;
-  }
-  if (n_over > 0) {
-    int blocks = (n_over + 7) / 8;
-    if (blocks > 4096) blocks = 4096;
-    nll_grad_global_kernel<<<blocks, 256, 0, s>>>(g, k, n_over, over_geom, over_box, rho, grad,
-                                                   acc, skipped);
-  }
+// Partial gradient images: eight while they are small beside the device's memory.
+int nll_grad_parts(int64_t n_pix) { return n_pix <= (int64_t(1) << 22) ? 8 : 1; }
+
+cudaError_t launch_nll(const DevGeom& g, const NllConst& k, int32_t n, const float4* ev_geom,
+                       const short4* ev_box, const uint16_t* table, int32_t stride,
+                       const float* rho, float* parts, double* acc, unsigned long long* skipped,
+                       cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  // events per warp: up to 32, so that the FP64 of a lane serves an event, but
+  // enough warps to fill the SMs (152 x 28)
+  int group = 32;
+  while (group > 2 && n / group < 2 * 152 * 28) group /= 2;
+  const int64_t n_pix = static_cast<int64_t>(g.n_y) * g.n_z;
+  const int warps = (n + group - 1) / group;
+  const int blocks = std::min((warps + kNllWarps - 1) / kNllWarps, 152 * 7 * 4);
+  auto* kern = parts ? (table ? nll_kernel<true, true> : nll_kernel<true, false>)
+                     : (table ? nll_kernel<false, true> : nll_kernel<false, false>);
+  kern<<<blocks, 32 * kNllWarps, 0, s>>>(g, k, n, group, ev_geom, ev_box, table, stride, rho, parts,
+                                         nll_grad_parts(n_pix), n_pix, acc, skipped);
   return cudaGetLastError();
 }
 
-cudaError_t launch_nll_finish(const float* sens, const float* rho, float* grad, double* acc,
-                              int64_t n, cudaStream_t s) {
-  nll_finish_kernel<<<152 * 4, 256, 0, s>>>(sens, rho, grad, acc, n);
+cudaError_t launch_nll_finish(const float* sens, const float* rho, const float* parts, float* grad,
+                              double* acc, int64_t n, cudaStream_t s) {
+  nll_finish_kernel<<<152 * 4, 256, 0, s>>>(sens, rho, parts, nll_grad_parts(n), grad, acc, n);
   return cudaGetLastError();
 }
 

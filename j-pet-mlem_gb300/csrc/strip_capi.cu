@@ -95,7 +95,7 @@ struct jpet_strip {
   unsigned long long table_kernel_calls = 0;
   DevBuf<unsigned long long> box_pixels;
   DevBuf<double> nll_acc;            // loss, d/dsigma_z, d/dsigma_dl
-  DevBuf<float> nll_grad_tmp;        // gradient image when the caller passes none
+  DevBuf<float> nll_parts;           // partial gradient images
   DevBuf<DevCounters> counters;
 
   int64_t n_events = 0;
@@ -815,7 +815,7 @@ int jpet_strip_destroy(jpet_strip_t* h) {
   h->event_rows.release();
   h->box_pixels.release();
   h->nll_acc.release();
-  h->nll_grad_tmp.release();
+  h->nll_parts.release();
   h->counters.release();
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   delete h;
@@ -956,22 +956,24 @@ int jpet_strip_nll_grad(jpet_strip_t* h, double sigma_z, double sigma_dl, const 
   cudaStream_t s = h->stream;
   const size_t n_pix = static_cast<size_t>(h->g.n_y) * h->g.n_z;
   JPET_CUDA(h, h->nll_acc.alloc(4), "cudaMalloc(likelihood)");
-  float* grad = d_grad_rho;
-  if (!grad) {
-    JPET_CUDA(h, h->nll_grad_tmp.alloc(n_pix), "cudaMalloc(gradient)");
-    grad = h->nll_grad_tmp.p;
-  }
+  const size_t n_parts = d_grad_rho ? nll_grad_parts(static_cast<int64_t>(n_pix)) * n_pix : 0;
+  if (d_grad_rho) JPET_CUDA(h, h->nll_parts.alloc(n_parts), "cudaMalloc(gradient)");
+  float* parts = d_grad_rho ? h->nll_parts.p : nullptr;
   const float* rho = d_rho ? d_rho : h->rho.p;
   const float* sens = d_sens ? d_sens : h->sens_point.p;
   JPET_CUDA(h, cudaMemsetAsync(h->nll_acc.p, 0, 4 * sizeof(double), s), "memset");
-  JPET_CUDA(h, cudaMemsetAsync(grad, 0, n_pix * sizeof(float), s), "memset");
+  if (parts) JPET_CUDA(h, cudaMemsetAsync(parts, 0, n_parts * sizeof(float), s), "memset");
   const NllConst k = make_nll_const(sigma_z, sigma_dl);
-  JPET_CUDA(h, launch_nll_grad(h->g, k, h->tiling, h->chunks.p, h->n_chunks, h->sorted_geom.p,
-                               h->sorted_box.p, h->n_oversize, h->over_geom.p, h->over_box.p, rho,
-                               grad, h->nll_acc.p,
-                               reinterpret_cast<unsigned long long*>(h->nll_acc.p + 3), s),
+  auto* skipped = reinterpret_cast<unsigned long long*>(h->nll_acc.p + 3);
+  JPET_CUDA(h, launch_nll(h->g, k, h->n_sorted, h->sorted_geom.p, h->sorted_box.p,
+                          h->use_fast ? h->row_table.p : nullptr, h->tiling.row_stride, rho, parts,
+                          h->nll_acc.p, skipped, s),
             "likelihood kernel launch");
-  JPET_CUDA(h, launch_nll_finish(sens, rho, grad, h->nll_acc.p, static_cast<int64_t>(n_pix), s),
+  JPET_CUDA(h, launch_nll(h->g, k, h->n_oversize, h->over_geom.p, h->over_box.p, nullptr, 0, rho,
+                          parts, h->nll_acc.p, skipped, s),
+            "likelihood kernel launch");
+  JPET_CUDA(h, launch_nll_finish(sens, rho, parts, d_grad_rho, h->nll_acc.p,
+                                 static_cast<int64_t>(n_pix), s),
             "likelihood finish launch");
   double host[4];
   JPET_CUDA(h, cudaMemcpyAsync(host, h->nll_acc.p, sizeof(host), cudaMemcpyDeviceToHost, s),

@@ -114,8 +114,8 @@ __global__ void scatter_events_kernel(int64_t n, const float4* __restrict__ ev_g
 // events too large for any window, jpet_strip_iterate_noalloc)
 // ---------------------------------------------------------------------------------
 //
-// One warp per event.  The lanes set up 32 box rows at a time, one each: the
-// row's exact in-ellipse interval and the terms of the kernel that are the same
+// One warp per event.  The lanes set up a block of box rows, one each: the row's
+// exact in-ellipse interval and the terms of the kernel that are the same
 // along the row, every operation rounded as in gauss_exact / analytic_exact, so
 // that hoisting changes no bit.  The block's pixels are then walked flattened, 32
 // at a time: a bit per pixel marks the rows' first pixels, and the set bits up to
@@ -135,14 +135,17 @@ __global__ void scatter_events_kernel(int64_t n, const float4* __restrict__ ev_g
 // square roots of the reference's order.
 constexpr int kExactWarps = 4;       // warps per CTA
 constexpr int kExactCache = 1024;    // values kept per event
-constexpr int kExactWidth = 256;     // box columns; wider boxes take process_event
+constexpr int kExactRows = 64;       // rows of a block (an event's set-up is then kept for the
+                                     // back-projection)
+constexpr int kExactPixels = 8192;   // pixels of a block: boxes wider than this / 32 take
+                                     // process_event
 
 struct ExactWarp {
-  float4 ra[32];            // dy tan | element before exp or a_ic_a | r terms of b_ic_b, b_ic_a
-  float4 rb[32];            // GPU-reference: ap, aq, op ipz, oq ipz
-  float rc[32];             // GPU-reference: r term of o_ic_b
-  int2 at[32];              // column minus pixel number, image row offset
-  uint32_t starts[kExactWidth];  // bit per pixel: first of its row
+  float4 ra[kExactRows];    // dy tan | element before exp or a_ic_a | r terms of b_ic_b, b_ic_a
+  float4 rb[kExactRows];    // GPU-reference: ap, aq, op ipz, oq ipz
+  float rc[kExactRows];     // GPU-reference: r term of o_ic_b
+  int2 at[kExactRows];      // column minus pixel number, image row offset
+  uint32_t starts[kExactPixels / 32];  // bit per pixel: first of its row
   float cache[kExactCache];
 };
 
@@ -179,7 +182,8 @@ __global__ void __launch_bounds__(32 * kExactWarps) iterate_exact_kernel(
   for (int e = warp; e < n_events; e += n_warps) {
     const float4 ev = ev_geom[e];
     const short4 box = ev_box[e];
-    if (box.z - box.x > kExactWidth) {
+    const int width = box.z - box.x, nrows = box.w - box.y;
+    if (width > kExactPixels / 32) {
       GlobalAccess<Sum> acc{rho, out, g.n_z};
       unsigned long long c = 0;
       process_event<SEM>(g, 32, ev, box, acc, sens, c, contrib);
@@ -189,48 +193,55 @@ __global__ void __launch_bounds__(32 * kExactWarps) iterate_exact_kernel(
     const float z = ev.x, y = ev.y, t = ev.z, sec = ev.w;
     float A, B, C;
     ellipse_abc(g, t, sec, A, B, C);
-    const int nrows = box.w - box.y;
+    const int step = nrows <= kExactRows && width * nrows <= kExactPixels ? kExactRows : 32;
     int total = 0;  // pixels of the block of rows last set up
     auto setup = [&](int rb) {
-      int first = 0, w = 0;
-      const int iy = box.y + rb + lane;
-      if (rb + lane < nrows)
-        w = row_interval(g, A, B, C, z, y, t, sec, box.x, box.z, iy, first);
-      int off = w;  // inclusive sum of the widths
+      total = 0;
+      int n_rows = 0;  // rows with pixels so far
+      __syncwarp();
+      const int words = (min(step, nrows - rb) * width + 31) >> 5;  // at least the pixels'
+      for (int i = lane; i < words; i += 32) s.starts[i] = 0u;
+      __syncwarp();
+      for (int r0 = rb; r0 < min(rb + step, nrows); r0 += 32) {
+        int first = 0, w = 0;
+        const int iy = box.y + r0 + lane;
+        if (r0 + lane < nrows)
+          w = row_interval(g, A, B, C, z, y, t, sec, box.x, box.z, iy, first);
+        int off = w;  // inclusive sum of the widths
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(kFull, off, o);
-        if (lane >= o) off += v;
-      }
-      total = __shfl_sync(kFull, off, 31);
-      off -= w;
-      const unsigned rows = __ballot_sync(kFull, w > 0);
-      __syncwarp();
-      for (int i = lane; i < (total + 31) >> 5; i += 32) s.starts[i] = 0u;
-      __syncwarp();
-      if (w > 0) {
-        const int r = __popc(rows & ((1u << lane) - 1u));
-        atomicOr(&s.starts[off >> 5], 1u << (off & 31));
-        const float dy = __fsub_rn(pixel_center_y(g, iy), y);
-        const float sec_sq = __fmul_rn(sec, sec);
-        const float yp = __fadd_rn(dy, y);
-        const float ap = __fmul_rn(-__fsub_rn(yp, g.radius), sec_sq);
-        const float aq = __fmul_rn(-__fadd_rn(yp, g.radius), sec_sq);
-        const float ar = __fmul_rn(__fmul_rn(__fmul_rn(-2.0f, yp), sec), t);
-        const float br = __fmul_rn(__fmul_rn(-2.0f, dy), sec);
-        const float a_ic_a = mic(g, ap, aq, ar, ap, aq, ar);
-        const float bd = __fmul_rn(br, g.ipd);
-        s.ra[r] = make_float4(__fmul_rn(dy, t),
-                              SEM == kCpuReference ? __fdiv_rn(g.c0, __fsqrt_rn(a_ic_a)) : a_ic_a,
-                              __fmul_rn(bd, br), __fmul_rn(bd, ar));
-        if (SEM == kGpuReference) {
-          const float op = __fmul_rn(ap, t), oq = __fmul_rn(aq, t);
-          const float orr = __fmul_rn(__fmul_rn(-yp, sec),
-                                      __fadd_rn(1.0f, __fmul_rn(__fmul_rn(2.0f, t), t)));
-          s.rb[r] = make_float4(ap, aq, __fmul_rn(op, g.ipz), __fmul_rn(oq, g.ipz));
-          s.rc[r] = __fmul_rn(__fmul_rn(orr, g.ipd), br);
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(kFull, off, o);
+          if (lane >= o) off += v;
         }
-        s.at[r] = make_int2(first - off, iy * g.n_z);
+        const int sum = __shfl_sync(kFull, off, 31);
+        off += total - w;
+        total += sum;
+        const unsigned rows = __ballot_sync(kFull, w > 0);
+        if (w > 0) {
+          const int r = n_rows + __popc(rows & ((1u << lane) - 1u));
+          atomicOr(&s.starts[off >> 5], 1u << (off & 31));
+          const float dy = __fsub_rn(pixel_center_y(g, iy), y);
+          const float sec_sq = __fmul_rn(sec, sec);
+          const float yp = __fadd_rn(dy, y);
+          const float ap = __fmul_rn(-__fsub_rn(yp, g.radius), sec_sq);
+          const float aq = __fmul_rn(-__fadd_rn(yp, g.radius), sec_sq);
+          const float ar = __fmul_rn(__fmul_rn(__fmul_rn(-2.0f, yp), sec), t);
+          const float br = __fmul_rn(__fmul_rn(-2.0f, dy), sec);
+          const float a_ic_a = mic(g, ap, aq, ar, ap, aq, ar);
+          const float bd = __fmul_rn(br, g.ipd);
+          s.ra[r] = make_float4(__fmul_rn(dy, t),
+                                SEM == kCpuReference ? __fdiv_rn(g.c0, __fsqrt_rn(a_ic_a)) : a_ic_a,
+                                __fmul_rn(bd, br), __fmul_rn(bd, ar));
+          if (SEM == kGpuReference) {
+            const float op = __fmul_rn(ap, t), oq = __fmul_rn(aq, t);
+            const float orr = __fmul_rn(__fmul_rn(-yp, sec),
+                                        __fadd_rn(1.0f, __fmul_rn(__fmul_rn(2.0f, t), t)));
+            s.rb[r] = make_float4(ap, aq, __fmul_rn(op, g.ipz), __fmul_rn(oq, g.ipz));
+            s.rc[r] = __fmul_rn(__fmul_rn(orr, g.ipd), br);
+          }
+          s.at[r] = make_int2(first - off, iy * g.n_z);
+        }
+        n_rows += __popc(rows);
       }
       __syncwarp();
     };
@@ -250,7 +261,7 @@ __global__ void __launch_bounds__(32 * kExactWarps) iterate_exact_kernel(
     };
     float den = 0.0f;
     int done = 0;
-    for (int rb = 0; rb < nrows; rb += 32) {
+    for (int rb = 0; rb < nrows; rb += step) {
       setup(rb);
       walk(done, [&](int i, int pix, int r, int col) {
         const float k = exact_value<SEM>(g, s, r, __fsub_rn(pixel_center_z(g, col), z));
@@ -266,8 +277,8 @@ __global__ void __launch_bounds__(32 * kExactWarps) iterate_exact_kernel(
     if (lane == 0) ++contrib;
     const float inv = __fdiv_rn(1.0f, den);
     done = 0;
-    for (int rb = 0; rb < nrows; rb += 32) {
-      if (nrows > 32) setup(rb);
+    for (int rb = 0; rb < nrows; rb += step) {
+      if (nrows > step) setup(rb);
       walk(done, [&](int i, int pix, int r, int col) {
         float kr;
         if (i < kExactCache)
