@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/jpet_strip.h"
@@ -85,9 +86,11 @@ struct jpet_strip {
   DevBuf<int32_t> sort_idx;       // set-up sort: event indices (input, output)
   DevBuf<unsigned char> sort_tmp; // set-up sort: radix-sort scratch
   DevBuf<uint32_t> batches;       // batch-union kernel: batch words per chunk
-  DevBuf<unsigned char> ev_const; // batch-union kernel: per-event constants
   DevBuf<uint16_t> union_rows;    // batch-union kernel: union row words per batch
-  DevBuf<uint16_t> event_rows;    // batch-union kernel: event row words per event
+  DevBuf<float4> records;         // batch-union kernel: event row records
+  // batch-union kernel: the chunks whose records the workspace holds at a time
+  // (first, count); with one part the records are written once
+  std::vector<std::pair<int32_t, int32_t>> parts;
   FastConst fc{};
   bool use_fast = false;
   bool use_union = false;
@@ -339,6 +342,54 @@ int precision_code(int precision) {
                                                  : kPrecisionFloat;
 }
 
+// Row records of the batch-union kernel for the chunks of part k.
+cudaError_t write_records(jpet_strip* h, size_t k, cudaStream_t s) {
+  return launch_union_records(h->g, h->fc, h->tiling, h->chunks.p + h->parts[k].first,
+                              h->parts[k].second, h->sorted_geom.p, h->sorted_box.p,
+                              h->row_table.p, h->batches.p, h->union_rows.p, h->records.p, s);
+}
+
+// Workspace of the row records (16 bytes per event and row of the batch shape:
+// 1 KB per event with 64 rows), the parts of the chunk list that it holds at a
+// time and each chunk's place in it.  Up to half of the free memory is taken
+// (looked up above 1 GB only); with less than all events' records they are
+// written again, part by part, in every iteration.
+cudaError_t alloc_records(jpet_strip* h, std::vector<Chunk>& chunks, int64_t n_events) {
+  const size_t rows = union_row_words(h->tiling), each = rows * sizeof(float4);
+  const size_t least = static_cast<size_t>(h->tiling.chunk_events);
+  size_t cap = static_cast<size_t>(std::max<int64_t>(n_events, 1));
+  h->parts.clear();
+  if (chunks.empty()) return cudaSuccess;
+  if (cap * rows > h->records.n) {
+    h->records.release();
+    if (cap * each > (1ull << 30)) {
+      size_t free_bytes = 0, total = 0;
+      const cudaError_t e = cudaMemGetInfo(&free_bytes, &total);
+      if (e != cudaSuccess) return e;
+      cap = std::min(cap, free_bytes / 2 / each);
+    }
+    for (;; cap /= 2) {
+      cap = std::max(cap, least);
+      const cudaError_t e = h->records.alloc(cap * rows);
+      if (e == cudaSuccess) break;
+      if (e != cudaErrorMemoryAllocation || cap == least) return e;
+      cudaGetLastError();
+    }
+  }
+  size_t used = 0;
+  for (size_t k = 0; k < chunks.size(); ++k) {
+    const size_t count = static_cast<size_t>(chunks[k].count);
+    if (k == 0 || used + count > cap) {
+      h->parts.emplace_back(static_cast<int32_t>(k), 0);
+      used = 0;
+    }
+    chunks[k].rec = static_cast<int32_t>(used);
+    used += count;
+    ++h->parts.back().second;
+  }
+  return cudaSuccess;
+}
+
 int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const float* d_dl,
                    int64_t n, int32_t stride = 1) {
   cudaStream_t s = h->stream;
@@ -346,6 +397,7 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   ++h->generation;
   h->n_events = n;
   h->n_sorted = h->n_oversize = h->n_chunks = h->n_tiles_nonempty = 0;
+  h->parts.clear();
   h->total_box_pixels = 0;
   if (n > (int64_t)INT32_MAX - 1)
     return h->fail(JPET_ERR_ARGUMENT, "at most %d events per handle", INT32_MAX - 1);
@@ -430,9 +482,6 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   h->n_oversize = n_over;
   h->n_chunks = static_cast<int32_t>(full.size());
   JPET_CUDA(h, h->chunks.alloc(std::max<size_t>(full.size(), 1)), "cudaMalloc(chunks)");
-  if (!full.empty())
-    JPET_CUDA(h, cudaMemcpyAsync(h->chunks.p, full.data(), full.size() * sizeof(Chunk),
-                                 cudaMemcpyHostToDevice, s), "copy chunks");
   JPET_CUDA(h, cudaMemcpyAsync(h->tile_offset.p, offset.data(), n_tiles * sizeof(int32_t),
                                cudaMemcpyHostToDevice, s), "copy tile offsets");
   JPET_CUDA(h, h->sorted_geom.alloc(std::max(acc, 1)), "cudaMalloc(sorted events)");
@@ -462,17 +511,18 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
               "row_table launch");
     if (h->use_union) {
       JPET_CUDA(h, h->batches.alloc(static_cast<size_t>(acc)), "cudaMalloc(batches)");
-      JPET_CUDA(h, h->ev_const.alloc(static_cast<size_t>(acc) * union_event_bytes()),
-                "cudaMalloc(event constants)");
       JPET_CUDA(h, h->union_rows.alloc(static_cast<size_t>(acc) * union_row_words(t)),
                 "cudaMalloc(union rows)");
-      JPET_CUDA(h, h->event_rows.alloc(static_cast<size_t>(acc) * union_row_words(t)),
-                "cudaMalloc(event rows)");
-      JPET_CUDA(h, launch_union_setup(h->g, h->fc, t, h->chunks.p, h->n_chunks, acc,
-                                      h->sorted_geom.p, h->sorted_box.p, h->row_table.p,
-                                      h->ev_const.p, h->batches.p, h->union_rows.p,
-                                      h->event_rows.p, s),
+      // the last allocation of the event set: it takes what it can get
+      JPET_CUDA(h, alloc_records(h, full, acc), "cudaMalloc(row records)");
+    }
+    JPET_CUDA(h, cudaMemcpyAsync(h->chunks.p, full.data(), full.size() * sizeof(Chunk),
+                                 cudaMemcpyHostToDevice, s), "copy chunks");
+    if (h->use_union) {
+      JPET_CUDA(h, launch_union_batches(t, h->chunks.p, h->n_chunks, h->sorted_box.p,
+                                        h->row_table.p, h->batches.p, h->union_rows.p, s),
                 "batch formation launch");
+      if (h->parts.size() == 1) JPET_CUDA(h, write_records(h, 0, s), "row record launch");
       JPET_CUDA(h, union_prepare_kernel(t, precision_code(h->opts.precision)),
                 "batch-union kernel attributes");
     } else if (h->opts.variant == JPET_VARIANT_FAST || h->opts.variant == JPET_VARIANT_ROWS) {
@@ -555,12 +605,15 @@ int iterate_on(jpet_strip* h, int n, cudaStream_t s) {
       const int prec = precision_code(h->opts.precision);
       const uint32_t seed = 0x9E3779B9u * static_cast<uint32_t>(h->iterations_done + 1);
       if (h->use_union) {
-        JPET_CUDA(h, launch_iterate_union(h->g, h->fc, h->tiling, h->chunks.p, h->n_chunks,
-                                          h->sorted_geom.p, h->sorted_box.p, h->ev_const.p,
-                                          h->event_rows.p, h->union_rows.p, h->batches.p,
-                                          h->rho.p, h->out.p, aux, h->counters.p, prec, seed,
-                                          s),
-                  "iteration kernel launch");
+        for (size_t k = 0; k < h->parts.size(); ++k) {
+          if (h->parts.size() > 1) JPET_CUDA(h, write_records(h, k, s), "row record launch");
+          JPET_CUDA(h, launch_iterate_union(h->g, h->fc, h->tiling,
+                                            h->chunks.p + h->parts[k].first, h->parts[k].second,
+                                            h->sorted_geom.p, h->sorted_box.p, h->records.p,
+                                            h->union_rows.p, h->batches.p, h->rho.p, h->out.p,
+                                            aux, h->counters.p, prec, seed, s),
+                    "iteration kernel launch");
+        }
       } else if (h->opts.variant == JPET_VARIANT_WARP) {
         JPET_CUDA(h, launch_iterate_fast(h->g, h->fc, h->tiling, h->chunks.p, h->n_chunks,
                                          h->sorted_geom.p, h->sorted_box.p, h->row_table.p,
@@ -626,7 +679,8 @@ uint64_t handle_generation(const jpet_strip* h) { return h->generation; }
 const float* handle_image(const jpet_strip* h) { return h->rho.p; }
 // kernels of one iteration
 int handle_launches(const jpet_strip* h) {
-  return (h->n_chunks > 0 ? 1 : 0) + (h->n_oversize > 0 ? 1 : 0);
+  const int parts = static_cast<int>(h->parts.size());  // with several, their records too
+  return (parts > 1 ? 2 * parts : h->n_chunks > 0 ? 1 : 0) + (h->n_oversize > 0 ? 1 : 0);
 }
 
 // Issues n iterations on the (capturing) stream and leaves the handle as it was:
@@ -810,9 +864,8 @@ int jpet_strip_destroy(jpet_strip_t* h) {
   h->sort_idx.release();
   h->sort_tmp.release();
   h->batches.release();
-  h->ev_const.release();
   h->union_rows.release();
-  h->event_rows.release();
+  h->records.release();
   h->box_pixels.release();
   h->nll_acc.release();
   h->nll_parts.release();

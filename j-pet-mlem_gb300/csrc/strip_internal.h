@@ -30,6 +30,7 @@ struct Chunk {
   int32_t ox, oy; // window origin (pixel column, row)
   int32_t n_batches;  // batch-union kernel: batches of the chunk (set-up)
   int32_t n_exact;    // batch-union kernel: events rasterised in the reference's order
+  int32_t rec;        // batch-union kernel: first event's place among the records
 };
 
 // Window and tiling parameters chosen at set_events time.
@@ -180,8 +181,8 @@ cudaError_t sort_events(const Tiling& t, int64_t n, const float4* ev_geom, const
                         int64_t n_tile_events, int64_t n_over, float4* sorted_geom,
                         short4* sorted_box, float4* over_geom, short4* over_box,
                         cudaStream_t s);
-// Batch-union kernel (strip_union.cuh; set-up in strip_union.cu): per-event
-// constants and batches of similar events per chunk (set-up), and the iteration
+// Batch-union kernel (strip_union.cuh; set-up in strip_union.cu): batches of
+// similar events per chunk and their row records (set-up), and the iteration
 // over them in every accumulation mode (precision: a FastPrecision code; aux: the
 // second image of the compensated and fixed-point modes; seed: the fixed-point
 // dither's per-iteration seed).
@@ -191,10 +192,9 @@ struct UnionOps {
   cudaError_t (*prepare)(int precision);
   cudaError_t (*launch)(const DevGeom& g, const FastConst& fc, const Tiling& t,
                         const Chunk* chunks, int32_t n_chunks, const float4* ev_geom,
-                        const short4* ev_box, const void* ev_const, const uint16_t* erows,
-                        const uint16_t* urows, const uint32_t* batches, const float* rho,
-                        float* out, AuxImage aux, DevCounters* counters, int precision,
-                        uint32_t seed, cudaStream_t s);
+                        const short4* ev_box, const float4* records, const uint16_t* urows,
+                        const uint32_t* batches, const float* rho, float* out, AuxImage aux,
+                        DevCounters* counters, int precision, uint32_t seed, cudaStream_t s);
 };
 const UnionOps& union_ops_64x32();
 const UnionOps& union_ops_64x32n4();
@@ -203,24 +203,27 @@ const UnionOps& union_ops_32x32();
 const UnionOps& union_ops_96x40();
 const UnionOps& union_ops_64x16();
 const UnionOps& union_ops(int shape);
-size_t union_event_bytes();
 size_t union_smem_bytes(const Tiling& t, int precision);
 cudaError_t union_prepare_kernel(const Tiling& t, int precision);
-// union_row_words(): 16-bit words per event of the union-row and event-row
-// arrays (urows: per batch, indexed by the batch word's position; erows: per
-// event), written by launch_union_setup from the row table.
+// union_row_words(): rows of the shape's batches, so 16-bit words per batch of
+// the union rows (urows, indexed by the batch word's position) and 16-byte
+// records per event.  launch_union_batches forms the batches of the chunks from
+// the row table; launch_union_records writes the records of n_chunks chunks, an
+// event's from (Chunk.rec + its place in the chunk) x rows.
 size_t union_row_words(const Tiling& t);
-cudaError_t launch_union_setup(const DevGeom& g, const FastConst& fc, const Tiling& t,
-                               Chunk* chunks, int32_t n_chunks, int32_t n_events,
-                               const float4* ev_geom, const short4* ev_box, const uint16_t* rows,
-                               void* ev_const, uint32_t* batches, uint16_t* urows,
-                               uint16_t* erows, cudaStream_t s);
+cudaError_t launch_union_batches(const Tiling& t, Chunk* chunks, int32_t n_chunks,
+                                 const short4* ev_box, const uint16_t* rows, uint32_t* batches,
+                                 uint16_t* urows, cudaStream_t s);
+cudaError_t launch_union_records(const DevGeom& g, const FastConst& fc, const Tiling& t,
+                                 const Chunk* chunks, int32_t n_chunks, const float4* ev_geom,
+                                 const short4* ev_box, const uint16_t* rows,
+                                 const uint32_t* batches, const uint16_t* urows, float4* records,
+                                 cudaStream_t s);
 cudaError_t launch_iterate_union(const DevGeom& g, const FastConst& fc, const Tiling& t,
                                  const Chunk* chunks, int32_t n_chunks, const float4* ev_geom,
-                                 const short4* ev_box, const void* ev_const,
-                                 const uint16_t* erows, const uint16_t* urows,
-                                 const uint32_t* batches, const float* rho, float* out,
-                                 AuxImage aux, DevCounters* counters, int precision,
+                                 const short4* ev_box, const float4* records,
+                                 const uint16_t* urows, const uint32_t* batches, const float* rho,
+                                 float* out, AuxImage aux, DevCounters* counters, int precision,
                                  uint32_t seed, cudaStream_t s);
 cudaError_t launch_iterate_fast(const DevGeom& g, const FastConst& fc, const Tiling& t,
                                 const Chunk* chunks, int32_t n_chunks, const float4* ev_geom,

@@ -8,24 +8,31 @@
 // union_batches_kernel groups each chunk's events greedily into batches of up
 // to E consecutive events whose union -- per window row, from the smallest first
 // column (rounded down to even) to the largest last column -- spans at most the
-// rows and columns of the shape (UShape; chosen from the events' boxes), and writes, per batch, each union row's start column and width and, per event
-// and union row, its in-ellipse interval relative to that start.  An event
-// that does not fit that rectangle on its own is rasterised in the reference's
-// order instead (the exact path); union_events_kernel stores each event's
-// constants (y, tan, exponent coefficients, window-relative box).
+// rows and columns of the shape (UShape; chosen from the events' boxes), and
+// writes each union row's start column and width.  An event that does not fit
+// that rectangle on its own is rasterised in the reference's order instead (the
+// exact path).  union_records_kernel then writes a 16-byte record per event and
+// union row: the exponent's coefficients and the mask of the event's columns.
 //
 // The iteration kernel runs one CTA of NW warps per chunk, with the rho and
-// back-projection windows of the tile in shared memory.  For a batch, union row r belongs to the 4 lanes (gid) of one warp,
-// lane gl owning the pixel pairs 2 gl + 8 s (s < SW) of the row from its even
-// start column: the SAME pixels for every event of the batch.  So rho is read
-// once per batch, each event's K rho stays in registers, and the
-// back-projection adds sum_e K_e rho inv_e to each owned pixel pair with one
-// shared-memory read-modify-write per batch (not per event); no pixel has two
-// writers in a batch and no atomics are issued.  The per-(event, row)
-// exponent coefficients and column masks of batch b + 1 are computed by all
-// threads in the same straight-line block as batch b's forward sums
-// (double-buffered), so a batch costs one CTA barrier (the one that publishes
-// the denominators).
+// back-projection windows of the tile in shared memory.  For a batch, union row
+// r belongs to the 4 lanes (gid) of one warp, lane gl owning the pixel pairs
+// 2 gl + 8 s (s < SW) of the row from its even start column: the SAME pixels for
+// every event of the batch.  So rho is read once per batch, each event's K rho
+// stays in registers, and the back-projection adds sum_e K_e rho inv_e to each
+// owned pixel pair with one shared-memory read-modify-write per batch (not per
+// event); no pixel has two writers in a batch and no atomics are issued.  A
+// batch's records arrive by asynchronous copies, issued when the batch before
+// the last is through with its buffer, so a batch costs one CTA barrier (the one
+// that publishes the denominators, the next records and the free buffer).
+//
+// Bound by instruction issue.  The records used to be computed on chip for
+// every batch, about 65 of its 490 instructions per warp; read from memory they
+// cost 16 bytes per event and row of DRAM traffic, which the kernel otherwise
+// leaves idle (2e7 events at 2 mm: at most 20 GB per iteration, 2 TB/s).  Iterations,
+// computed on chip -> read: 2e7 events at 2 mm 12.39 -> 10.43 ms, 6e6 at 1 mm
+// 3.99 -> 3.37 ms, 1e6 at 5 mm 0.293 -> 0.244 ms, 1e6 at 2 mm with sigma 14 / 60
+// 1.49 -> 1.28 ms, 2e6 at 2 mm compensated 2.38 -> 2.06 ms.
 //
 // Accumulation modes (template argument ACC, DEN64): FP32 windows flushed with
 // float atomics; compensated windows (each batch's addition followed by
@@ -44,15 +51,13 @@
 // (rho'' = rho 2^(c jc^2)) and a pixel costs one FFMA2 per pixel pair, one ex2
 // per pixel and one FMUL2; otherwise (coarse pixels, where 2^(c jc^2) would
 // underflow while 2^(p' + q' jc) overflows) the full exponent is evaluated,
-// one FADD2 more per pair.  The coefficients p', q' are regenerated on chip for
-// every batch from the event's constants and the row (no per-row coefficient
-// table in memory).
+// one FADD2 more per pair.
 //
 // Chain form (where the row Gaussian spans several pixels, e.g. 2 mm or 1 mm
 // pixels at sigma_z = 5 pixels: |c| = 0.058): along a row
 // K' = 2^(p' + q' jc) is geometric, so a lane evaluates two ex2 per event and
 // row (its first pixel pair) and steps to its next pair, 8 columns on, with one
-// FMUL2 by R8 = 2^(8 q') (computed once per event and row at set-up).  Every
+// FMUL2 by R8 = 2^(8 q') (part of the record up to 32 columns).  Every
 // K' a lane forms is a product of at most SW rounded factors, within ~1e-6
 // of the direct value, and stays a normal float (u_exponent_form).
 // The masked K' stay in registers; the forward sum takes K' rho'' in one FFMA2
@@ -92,21 +97,10 @@ struct UShape {
   static constexpr int kThreads = 32 * NW;
   static constexpr int kMinCtas = MIN_CTAS;
   static constexpr int kPartials = (NW + 3) & ~3;  // warp partials of a denominator, padded
-  using Mask = typename std::conditional<(SW <= 4), uint32_t, uint64_t>::type;
 };
 
 constexpr int kUMaxChunk = 2048;     // events per chunk (batch words keep 11 bits of offset)
 constexpr int kUMaxChunkFixed = 512; // fixed point: a window pixel's integer sum stays < 2^31
-
-// Per-event constants (union_events_kernel): K / K_ref exponent terms as in
-// row_coeff_kernel, and the box relative to the tile's window origin
-// (first row | rows << 8 | first column << 16).
-struct UEvConst {
-  float y, tn, ky, lref;
-  float P, Q, ub;
-  uint32_t box;
-};
-static_assert(sizeof(UEvConst) == 32, "two 16-byte pieces");
 
 // Batch word: first event (offset in the chunk) | events << 11 | union rows << 15
 // | union's first window row << 22 (below 256: boxes of up to 1024 rows are
@@ -117,64 +111,36 @@ __host__ __device__ inline uint32_t ubatch_word(int first, int cnt, int rows, in
 }
 __device__ __forceinline__ int ub_first(uint32_t w) { return static_cast<int>(w & 2047u); }
 __device__ __forceinline__ int ub_cnt(uint32_t w) { return static_cast<int>((w >> 11) & 15u); }
+__device__ __forceinline__ int ub_rows(uint32_t w) { return static_cast<int>((w >> 15) & 127u); }
 __device__ __forceinline__ int ub_u0(uint32_t w) { return static_cast<int>(w >> 22); }
 
 // Union row word (per batch and union row): start column in the window | width << 9.
 __host__ __device__ inline uint16_t urow_word(int u, int wu) {
   return static_cast<uint16_t>(u | (wu << 9));
 }
-// Event row word (per event and union row of its batch): first in-ellipse
-// column relative to the union row's start | width << 8 (0: no pixel).
 
-// Padded per-event strides of the shared-memory batch arrays: the set-up
-// threads of one union row write different events at once, and with unpadded
-// strides (multiples of 128 bytes) those writes hit the same banks.
-template <class C>
-struct UStage {
-  UEvConst ev[C::E];
-  uint16_t rows[C::E][C::kRows + 8];  // event row words of the batch's union rows
-  uint16_t urows[C::kRows];           // union row words
-};
-
+// Record of an event in a union row of its batch: p, q, and for up to 32 columns
+// R8 and the column mask, else the mask's two halves.  The mask holds the 2 SW
+// columns of a lane together, in the order in which the lane takes them (column
+// 8 s + 2 gl + h is bit 2 s + h of lane gl's 8 bits, or 16 with two halves), so
+// that a lane's tests are of a register's low bits.
+__device__ __forceinline__ uint32_t u_lane_mask(uint32_t m) {
+  // transpose of 4 x 4 cells of two bits
+  uint32_t t = (m ^ (m >> 6)) & 0x00CC00CCu;
+  m ^= t ^ (t << 6);
+  t = (m ^ (m >> 12)) & 0x0000F0F0u;
+  return m ^ t ^ (t << 12);
+}
 template <class C, class DT>
 struct USmem {
-  UStage<C> stage[2];
-  float4 pq[2][C::E][C::kRows + 1];  // {p, p, q, q}, chain form {p, q, R8, R8}
-  typename C::Mask mask[2][C::E][C::kRows + 4];  // columns of the union row inside the event's interval
-  uint32_t urow[2][C::kRows];        // union start column | union width << 16
+  float4 rec[2][C::E][C::kRows];  // records of two batches
+  uint16_t urow[2][C::kRows];     // their union row words
   __align__(16) DT den_part[2][C::E][C::kPartials];  // float, or double (FP64 denominators)
   float gfac[2 * C::kCols];          // 2^(c jc^2), jc = index - kCols (split exponent)
   float cjc[2 * C::kCols];           // c jc^2 (full exponent)
-  uint32_t bw[4];  // the chunk's batch words and exact-path list (+ one read past the last
-                   // batch): chunk_events + 4 words, the last of the allocation
+  uint32_t bw[4];  // the chunk's batch words and exact-path list: chunk_events + 4 words,
+                   // the last of the allocation
 };
-
-template <class C>
-__device__ __forceinline__ void u_issue_stage(UStage<C>& st, const UEvConst* __restrict__ evc,
-                                              const uint16_t* __restrict__ erows,
-                                              const uint16_t* __restrict__ urows, int bi,
-                                              int first, int cnt) {
-  constexpr int E = C::E, kQ = C::kRows / 8;  // 16-byte pieces of one event's row words
-  static_assert(2 * E + kQ <= 32 && 32 + E * kQ <= C::kThreads, "one piece per thread");
-  const int tid = threadIdx.x;
-  if (tid < 2 * E) {
-    const int j = tid >> 1, h = tid & 1;
-    const bool v = j < cnt;
-    const int e = first + (v ? j : 0);
-    cp_async16(reinterpret_cast<float4*>(&st.ev[j]) + h,
-               reinterpret_cast<const float4*>(evc + e) + h, v);
-  } else if (tid < 2 * E + kQ) {
-    const int q = tid - 2 * E;
-    cp_async16(&st.urows[8 * q], urows + static_cast<size_t>(bi) * C::kRows + 8 * q, true);
-  } else if (tid >= 32 && tid < 32 + E * kQ) {
-    const int k = tid - 32;
-    const int j = k / kQ, q = k % kQ;
-    const bool v = j < cnt;
-    const size_t src = static_cast<size_t>(first + (v ? j : 0)) * C::kRows + 8 * q;
-    cp_async16(&st.rows[j][8 * q], erows + src, v);
-  }
-  cp_async_commit();
-}
 
 // Exponent forms of the iteration kernel (template argument XM).
 constexpr int kXFull = 0;   // p + q jc + c jc^2 per pixel
@@ -186,58 +152,40 @@ constexpr int kXChain = 2;  // split, and K' stepped along the row by R8
 __device__ __forceinline__ int u_centre(int wu) { return (wu >> 1) & ~1; }
 
 // Union rows and per-(event, row) records of one batch: 4 / RS threads per
-// union row (consecutive lanes), each handling RS E / 4 events.
-template <class C, int XM, class DT>
-__device__ __forceinline__ void u_setup(const DevGeom& g, const FastConst& fc, USmem<C, DT>& S,
-                                        int buf, uint32_t bw, int ox, int oy) {
-  constexpr int kTPR = 4 / C::RS;       // threads per union row
-  constexpr int kEPT = C::E / kTPR;     // events per thread
-  static_assert(kTPR * kEPT == C::E, "whole events per set-up thread");
-  const UStage<C>& st = S.stage[buf];
-  const int u0 = ub_u0(bw);
-  const int r = threadIdx.x / kTPR, sub = threadIdx.x % kTPR;
-  // union row (start column, width) and the events' intervals relative to it,
-  // as the batch former wrote them (rows past the union, and events past the
-  // batch's count, read as 0: no pixel)
-  const uint32_t ur = st.urows[r];
-  const int u = static_cast<int>(ur & 511u), wu = static_cast<int>(ur >> 9);
-  if (sub == 0) S.urow[buf][r] = static_cast<uint32_t>(u) | (static_cast<uint32_t>(wu) << 16);
-  const float py = g.tl_y_half_h - static_cast<float>(oy + u0 + r) * g.pixel_height;
-  const float colm = static_cast<float>(ox + u + u_centre(wu));
-  const float kz2pw = 2.0f * fc.kz * g.pixel_width;
+
+// A batch's records (zero, so no pixel, for events past its count and rows past
+// its union) and union rows.  rec: the batch's first event's records.
+template <class C, class DT>
+__device__ __forceinline__ void u_issue_records(USmem<C, DT>& S, int buf, const float4* rec,
+                                                const uint16_t* urows, int cnt, int rows) {
+  constexpr int kPieces = C::E * C::kRows;
+  static_assert(kPieces % C::kThreads == 0, "whole pieces per thread");
+  float4* dst = &S.rec[buf][0][0];
 #pragma unroll
-  for (int k = 0; k < kEPT; ++k) {
-    const int j = kEPT * sub + k;
-    const UEvConst& e = st.ev[j];
-    const float dy = py - e.y;
-    const float lf = e.lref - 0.5f * lg2_approx(fmaf(e.Q, py * py, e.P));
-    const float ua = fmaf(colm, g.pixel_width, e.ub - dy * e.tn);
-    const float p = fmaf(fc.kz * ua, ua, fmaf(e.ky * dy, dy, lf));
-    const float q = kz2pw * ua;
-    const uint32_t ew = st.rows[j][r];
-    const int w = static_cast<int>(ew >> 8);
-    const int lr = static_cast<int>(ew & 255u);  // 0 <= lr, lr + w <= wu <= kCols
-    if (XM == kXChain) {
-      const float r8 = ex2_approx(8.0f * q);
-      S.pq[buf][j][r] = make_float4(p, q, r8, r8);
-    } else {
-      S.pq[buf][j][r] = make_float4(p, p, q, q);
-    }
-    if constexpr (C::SW <= 4) {
-      // w low bits set (0 <= w <= 32): the clamped funnel shift of ~0 by 32 - w
-      const uint32_t bits = __funnelshift_rc(0xFFFFFFFFu, 0u, static_cast<unsigned>(32 - w));
-      S.mask[buf][j][r] = bits << lr;
-    } else {
-      S.mask[buf][j][r] = ((1ull << w) - 1ull) << lr;  // w <= kCols < 64
-    }
+  for (int i = 0; i < kPieces / C::kThreads; ++i) {
+    const int k = i * C::kThreads + threadIdx.x;
+    const bool v = k < cnt * C::kRows && k % C::kRows < rows;
+    cp_async16(dst + k, rec + (v ? k : 0), v);
   }
+  if (threadIdx.x < C::kRows / 8)
+    cp_async16(&S.urow[buf][8 * threadIdx.x], urows + 8 * threadIdx.x, true);
+  cp_async_commit();
 }
 
-// Column j (a compile-time constant) of a mask; 64-bit masks test one half.
-__device__ __forceinline__ bool u_column(uint32_t m, int j) { return (m & (1u << j)) != 0u; }
-__device__ __forceinline__ bool u_column(uint64_t m, int j) {
-  const uint32_t h = j < 32 ? static_cast<uint32_t>(m) : static_cast<uint32_t>(m >> 32);
-  return (h & (1u << (j & 31))) != 0u;
+// A lane's part of a record.
+struct URecord {
+  float p, q, r8;
+  uint32_t m;  // bit 2 s + h: column 8 s + 2 gl + h inside the event's interval
+};
+template <class C, int XM, class DT>
+__device__ __forceinline__ URecord u_record(const USmem<C, DT>& S, int buf, int j, int r_u,
+                                            int gl) {
+  const float4 a = S.rec[buf][j][r_u];
+  if constexpr (C::SW <= 4)
+    return URecord{a.x, a.y, a.z, __float_as_uint(a.w) >> (8 * gl)};
+  else
+    return URecord{a.x, a.y, XM == kXChain ? ex2_approx(8.0f * a.y) : 0.0f,
+                   __float_as_uint(gl & 2 ? a.w : a.z) >> (16 * (gl & 1))};
 }
 
 // Forward sums of one row step with SWN active sweeps: rho'' of the owned
@@ -262,17 +210,16 @@ __device__ __forceinline__ void u_forward(float2 (&kr)[C::E][C::RS][C::SW], DT (
   }
 #pragma unroll
   for (int j = 0; j < C::E; ++j) {
-    const float4 a = S.pq[buf][j][r_u];
-    const typename C::Mask m = S.mask[buf][j][r_u] >> (2 * gl);
-    const float2 p2 = make_float2(a.x, a.y), q2 = make_float2(a.z, a.w);
+    const URecord a = u_record<C, SPLIT ? kXSplit : kXFull>(S, buf, j, r_u, gl);
+    const float2 p2 = make_float2(a.p, a.p), q2 = make_float2(a.q, a.q);
     float2 dd = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int s = 0; s < SWN; ++s) {
       const float2 e = SPLIT ? __ffma2_rn(q2, jc2[s], p2)
                              : __ffma2_rn(q2, jc2[s], __fadd2_rn(p2, cq[s]));
       float2 v = __fmul2_rn(make_float2(ex2_approx(e.x), ex2_approx(e.y)), rr[s]);
-      v.x = u_column(m, 8 * s) ? v.x : 0.0f;
-      v.y = u_column(m, 8 * s + 1) ? v.y : 0.0f;
+      v.x = (a.m & (1u << (2 * s))) ? v.x : 0.0f;
+      v.y = (a.m & (2u << (2 * s))) ? v.y : 0.0f;
       kr[j][RSI][s] = v;
       dd = __fadd2_rn(dd, v);
     }
@@ -298,18 +245,17 @@ __device__ __forceinline__ void u_forward_chain(float2 (&kr)[C::E][C::RS][C::SW]
   }
 #pragma unroll
   for (int j = 0; j < C::E; ++j) {
-    const float4 a = S.pq[buf][j][r_u];
-    const typename C::Mask m = S.mask[buf][j][r_u] >> (2 * gl);
-    const float e0 = fmaf(a.y, jf, a.x);
-    float2 k = make_float2(ex2_approx(e0), ex2_approx(e0 + a.y));
-    const float2 r8 = make_float2(a.z, a.w);
+    const URecord a = u_record<C, kXChain>(S, buf, j, r_u, gl);
+    const float e0 = fmaf(a.q, jf, a.p);
+    float2 k = make_float2(ex2_approx(e0), ex2_approx(e0 + a.q));
+    const float2 r8 = make_float2(a.r8, a.r8);
     float2 dd;
 #pragma unroll
     for (int s = 0; s < SWN; ++s) {
       if (s > 0) k = __fmul2_rn(k, r8);
       float2 v;
-      v.x = u_column(m, 8 * s) ? k.x : 0.0f;
-      v.y = u_column(m, 8 * s + 1) ? k.y : 0.0f;
+      v.x = (a.m & (1u << (2 * s))) ? k.x : 0.0f;
+      v.y = (a.m & (2u << (2 * s))) ? k.y : 0.0f;
       kr[j][RSI][s] = v;
       dd = (s == 0) ? __fmul2_rn(v, rr[0]) : __ffma2_rn(v, rr[s], dd);
     }
@@ -482,8 +428,8 @@ template <class C, int XM, int ACC, bool DEN64>
 __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel(
     DevGeom g, FastConst fc, Tiling t, const Chunk* __restrict__ chunks,
     const float4* __restrict__ ev_geom, const short4* __restrict__ ev_box,
-    const UEvConst* __restrict__ evc, const uint16_t* __restrict__ erows,
-    const uint16_t* __restrict__ urows, const uint32_t* __restrict__ batches,
+    const float4* __restrict__ records, const uint16_t* __restrict__ urows,
+    const uint32_t* __restrict__ batches,
     const float* __restrict__ rho, float* __restrict__ out, AuxImage aux, uint32_t seed,
     DevCounters* counters) {
   using DT = typename std::conditional<DEN64, double, float>::type;
@@ -505,8 +451,10 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
   const int nb = c.n_batches;
   const uint32_t* bws = batches + c.start;
   auto issue = [&](int b, int buf, uint32_t w) {
-    u_issue_stage<C>(S.stage[buf], evc, erows, urows, c.start + b, c.start + ub_first(w),
-                     ub_cnt(w));
+    u_issue_records<C, DT>(S, buf,
+                           records + static_cast<size_t>(c.rec + ub_first(w)) * C::kRows,
+                           urows + static_cast<size_t>(c.start + b) * C::kRows, ub_cnt(w),
+                           ub_rows(w));
   };
 
   if (nb > 0) issue(0, 0, bws[0]);
@@ -535,14 +483,11 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
   unsigned long long contrib = 0;
   cp_async_wait_all();
   __syncthreads();
-  if (nb > 0) u_setup<C, XM, DT>(g, fc, S, 0, S.bw[0], ox, oy);
-  __syncthreads();
 
   for (int b = 0; b < nb; ++b) {
     const int buf = b & 1;
     const uint32_t bw = S.bw[b];
     const int cnt = ub_cnt(bw), u0 = ub_u0(bw);
-    if (b + 2 < nb) issue(b + 2, buf, S.bw[b + 2]);
     // ---- forward: this warp's union rows of every event of the batch
     float2 kr[E][RS][SW];
     DT dsum[E];
@@ -554,42 +499,39 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
       const int r_u = kRowsPerStep * rs + 8 * warp + gid;
       const uint32_t ur = S.urow[buf][r_u];
       const int wrow = min(u0 + r_u, t.win_h - 1);
-      base[rs] = wrow * pitch + static_cast<int>(ur & 0xFFFFu) + 2 * gl;
-      wu[rs] = static_cast<int>(ur >> 16);
+      base[rs] = wrow * pitch + static_cast<int>(ur & 511u) + 2 * gl;
+      wu[rs] = static_cast<int>(ur >> 9);
       jc0[rs] = 2 * gl - u_centre(wu[rs]);
       nsw[rs] = (__reduce_max_sync(kFull, static_cast<unsigned>(wu[rs])) + 7) >> 3;
     }
-    // ---- forward, and the set-up of the next batch (its staged data was
-    // published by the last barrier)
+    // (RS == 1) forward sums and their transposed warp sum in one straight-line
+    // block per sweep count, so that the scheduler interleaves the sum's shuffles
+    // with the evaluation
     DT tot;
-    // (RS == 1) forward sums, their transposed warp sum and the set-up in one
-    // straight-line block per sweep count, so that the scheduler interleaves the
-    // set-up's loads, ex2/lg2 and the sum's shuffles with the evaluation.  The
-    // set-up runs even after a chunk's last batch (it then fills the unused
-    // buffer from stale staged data).
     if constexpr (RS == 1) {
       u_sweeps<SW>(nsw[0], [&](auto n) {
-        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, w_rho, S, buf, base[0], 8 * warp + gid, jc0[0],
-                                                  gl);
+        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, w_rho, S, buf, base[0],
+                                                      8 * warp + gid, jc0[0], gl);
         tot = rows_transpose_sum<E>(dsum);
-        u_setup<C, XM, DT>(g, fc, S, buf ^ 1, S.bw[b + 1], ox, oy);
       });
     } else {
       u_sweeps<SW>(nsw[0], [&](auto n) {
-        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, w_rho, S, buf, base[0], 8 * warp + gid, jc0[0],
-                                                  gl);
+        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, w_rho, S, buf, base[0],
+                                                      8 * warp + gid, jc0[0], gl);
       });
       u_sweeps<SW>(nsw[RS - 1], [&](auto n) {
         u_forward_x<C, decltype(n)::value, RS - 1, XM, DT>(kr, dsum, w_rho, S, buf, base[RS - 1],
-                                            kRowsPerStep + 8 * warp + gid, jc0[RS - 1],
-                                                       gl);
+                                                           kRowsPerStep + 8 * warp + gid,
+                                                           jc0[RS - 1], gl);
       });
-      if (b + 1 < nb) u_setup<C, XM, DT>(g, fc, S, buf ^ 1, S.bw[b + 1], ox, oy);
       tot = rows_transpose_sum<E>(dsum);
     }
     if (rows_lane_writes<E>(lane)) S.den_part[buf][rows_lane_event<E>(lane)][warp] = tot;
-    if (b + 2 < nb) cp_async_wait_all();
+    // the barrier also publishes the next batch's records (this thread's copies,
+    // issued one batch ago, are waited for first), and frees this batch's
+    cp_async_wait_all();
     __syncthreads();
+    if (b + 2 < nb) issue(b + 2, buf, S.bw[b + 2]);
     // ---- denominators: lane j (mod E) adds the warps' partials of event j
     float inv_l;
     {
@@ -726,10 +668,10 @@ struct UnionHost {
   }
   static cudaError_t launch(const DevGeom& g, const FastConst& fc, const Tiling& t,
                             const Chunk* chunks, int32_t n_chunks, const float4* ev_geom,
-                            const short4* ev_box, const void* ev_const, const uint16_t* erows,
-                            const uint16_t* urows, const uint32_t* batches, const float* rho,
-                            float* out, AuxImage aux, DevCounters* counters, int precision,
-                            uint32_t seed, cudaStream_t s) {
+                            const short4* ev_box, const float4* records, const uint16_t* urows,
+                            const uint32_t* batches, const float* rho, float* out, AuxImage aux,
+                            DevCounters* counters, int precision, uint32_t seed,
+                            cudaStream_t s) {
     const int xm = u_exponent_form<C>(g, fc);
     const size_t bytes = smem(t, precision);
     auto go = [&](auto acc, auto den64) {
@@ -738,8 +680,7 @@ struct UnionHost {
       auto* k = xm == kXChain   ? iterate_union_kernel<C, kXChain, ACC, DEN64>
                 : xm == kXSplit ? iterate_union_kernel<C, kXSplit, ACC, DEN64>
                                 : iterate_union_kernel<C, kXFull, ACC, DEN64>;
-      k<<<n_chunks, C::kThreads, bytes, s>>>(g, fc, t, chunks, ev_geom, ev_box,
-                                             static_cast<const UEvConst*>(ev_const), erows, urows,
+      k<<<n_chunks, C::kThreads, bytes, s>>>(g, fc, t, chunks, ev_geom, ev_box, records, urows,
                                              batches, rho, out, aux, seed, counters);
       return cudaGetLastError();
     };
