@@ -33,6 +33,10 @@
 // computed on chip -> read: 2e7 events at 2 mm 12.39 -> 10.43 ms, 6e6 at 1 mm
 // 3.99 -> 3.37 ms, 1e6 at 5 mm 0.293 -> 0.244 ms, 1e6 at 2 mm with sigma 14 / 60
 // 1.49 -> 1.28 ms, 2e6 at 2 mm compensated 2.38 -> 2.06 ms.
+// With the records read, the shared-memory pipe is 63 % busy; rho'' kept in
+// registers from the forward sums to the back-projection instead of read and
+// multiplied again there (the compiler has room for it: 123 registers): 2e7 at
+// 2 mm 10.43 -> 10.0 ms, 6e6 at 1 mm 3.37 -> 3.21 ms.
 //
 // Accumulation modes (template argument ACC, DEN64): FP32 windows flushed with
 // float atomics; compensated windows (each batch's addition followed by
@@ -232,10 +236,9 @@ __device__ __forceinline__ void u_forward(float2 (&kr)[C::E][C::RS][C::SW], DT (
 // K' stay in kr and the sum takes K' rho'' with one FFMA2 per pair.
 template <class C, int SWN, int RSI, class DT>
 __device__ __forceinline__ void u_forward_chain(float2 (&kr)[C::E][C::RS][C::SW],
-                                                DT (&dsum)[C::E], const float* w_rho,
-                                                const USmem<C, DT>& S, int buf, int base, int r_u,
-                                                int jc0, int gl) {
-  float2 rr[C::SW];
+                                                DT (&dsum)[C::E], float2 (&rr)[C::SW],
+                                                const float* w_rho, const USmem<C, DT>& S,
+                                                int buf, int base, int r_u, int jc0, int gl) {
   const float jf = static_cast<float>(jc0);
 #pragma unroll
   for (int s = 0; s < SWN; ++s) {
@@ -308,12 +311,13 @@ __device__ __forceinline__ void u_accumulate(float* w_out, float* w_comp, int id
 }
 
 // Back-projection of one row step in the chain form: rho'' sum_e K'_e inv_e
-// per owned pixel pair (rho'' read again), one read-modify-write of the pair.
+// per owned pixel pair (rho'' kept since the forward sums), one
+// read-modify-write of the pair.
 template <class C, int SWN, int RSI, int ACC>
-__device__ __forceinline__ void u_back_chain(const float2 (&kr)[C::E][C::RS][C::SW], float inv_l,
-                                             const float* w_rho, const float* gfac,
+__device__ __forceinline__ void u_back_chain(const float2 (&kr)[C::E][C::RS][C::SW],
+                                             const float2 (&rr)[C::SW], float inv_l,
                                              float* w_out, float* w_comp, int base, int wu,
-                                             int jc0, int gl, float dither) {
+                                             int gl, float dither) {
   // events outer, so that one event's 1/den is live at a time (lane j holds
   // event j's); the per-pair sums take the events in the same order as before
   float2 acc[C::SW];
@@ -330,15 +334,13 @@ __device__ __forceinline__ void u_back_chain(const float2 (&kr)[C::E][C::RS][C::
     // loads stay inside the windows (a row's last pair ends before the next
     // row's pitch plus the 64-float padding); the store is predicated on the
     // union row's width, the only pixels this row group owns
-    const float2 rv = *reinterpret_cast<const float2*>(w_rho + base + 8 * s);
-    const float2 gv = *reinterpret_cast<const float2*>(gfac + C::kCols + jc0 + 8 * s);
     const bool own = 2 * gl + 8 * s < wu;
     if (ACC == kAccFloat) {
       float2* op = reinterpret_cast<float2*>(w_out + base + 8 * s);
-      const float2 nv = __ffma2_rn(acc[s], __fmul2_rn(rv, gv), *op);
+      const float2 nv = __ffma2_rn(acc[s], rr[s], *op);
       if (own) *op = nv;
     } else {
-      u_accumulate<ACC>(w_out, w_comp, base + 8 * s, __fmul2_rn(acc[s], __fmul2_rn(rv, gv)),
+      u_accumulate<ACC>(w_out, w_comp, base + 8 * s, __fmul2_rn(acc[s], rr[s]),
                         own, dither);
     }
   }
@@ -368,11 +370,12 @@ __device__ __forceinline__ void u_back(const float2 (&kr)[C::E][C::RS][C::SW],
 
 template <class C, int SWN, int RSI, int XM, class DT>
 __device__ __forceinline__ void u_forward_x(float2 (&kr)[C::E][C::RS][C::SW], DT (&dsum)[C::E],
-                                            const float* w_rho, const USmem<C, DT>& S, int buf,
-                                            int base, int r_u, int jc0, int gl) {
+                                            float2 (&rr)[C::RS][C::SW], const float* w_rho,
+                                            const USmem<C, DT>& S, int buf, int base, int r_u,
+                                            int jc0, int gl) {
   if constexpr (SWN > 0) {
     if constexpr (XM == kXChain)
-      u_forward_chain<C, SWN, RSI, DT>(kr, dsum, w_rho, S, buf, base, r_u, jc0, gl);
+      u_forward_chain<C, SWN, RSI, DT>(kr, dsum, rr[RSI], w_rho, S, buf, base, r_u, jc0, gl);
     else
       u_forward<C, SWN, RSI, XM == kXSplit, DT>(kr, dsum, w_rho, S, buf, base, r_u, jc0, gl);
   }
@@ -393,13 +396,12 @@ __device__ __forceinline__ void u_sweeps(int nsw, F&& f) {
 }
 
 template <class C, int SWN, int RSI, int XM, int ACC>
-__device__ __forceinline__ void u_back_x(const float2 (&kr)[C::E][C::RS][C::SW], float inv_l,
-                                         const float* w_rho, const float* gfac, float* w_out,
-                                         float* w_comp, int base, int wu, int jc0, int gl,
+__device__ __forceinline__ void u_back_x(const float2 (&kr)[C::E][C::RS][C::SW],
+                                         const float2 (&rr)[C::RS][C::SW], float inv_l,
+                                         float* w_out, float* w_comp, int base, int wu, int gl,
                                          float dither) {
   if constexpr (SWN > 0 && XM == kXChain) {
-    u_back_chain<C, SWN, RSI, ACC>(kr, inv_l, w_rho, gfac, w_out, w_comp, base, wu, jc0, gl,
-                                   dither);
+    u_back_chain<C, SWN, RSI, ACC>(kr, rr[RSI], inv_l, w_out, w_comp, base, wu, gl, dither);
   } else if constexpr (SWN > 0) {
     float2 inv2[C::E];
 #pragma unroll
@@ -489,7 +491,7 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
     const uint32_t bw = S.bw[b];
     const int cnt = ub_cnt(bw), u0 = ub_u0(bw);
     // ---- forward: this warp's union rows of every event of the batch
-    float2 kr[E][RS][SW];
+    float2 kr[E][RS][SW], rr[RS][SW];  // K' (chain) or K rho''; rho'' (chain)
     DT dsum[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) dsum[j] = DT(0);
@@ -510,17 +512,17 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
     DT tot;
     if constexpr (RS == 1) {
       u_sweeps<SW>(nsw[0], [&](auto n) {
-        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, w_rho, S, buf, base[0],
+        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, rr, w_rho, S, buf, base[0],
                                                       8 * warp + gid, jc0[0], gl);
         tot = rows_transpose_sum<E>(dsum);
       });
     } else {
       u_sweeps<SW>(nsw[0], [&](auto n) {
-        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, w_rho, S, buf, base[0],
+        u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, rr, w_rho, S, buf, base[0],
                                                       8 * warp + gid, jc0[0], gl);
       });
       u_sweeps<SW>(nsw[RS - 1], [&](auto n) {
-        u_forward_x<C, decltype(n)::value, RS - 1, XM, DT>(kr, dsum, w_rho, S, buf, base[RS - 1],
+        u_forward_x<C, decltype(n)::value, RS - 1, XM, DT>(kr, dsum, rr, w_rho, S, buf, base[RS - 1],
                                                            kRowsPerStep + 8 * warp + gid,
                                                            jc0[RS - 1], gl);
       });
@@ -568,12 +570,12 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
       // one call per row step; RSI has to be a constant
       u_sweeps<SW>(nsw[rs], [&](auto n) {
         if (rs == 0)
-          u_back_x<C, decltype(n)::value, 0, XM, ACC>(kr, inv_l, w_rho, S.gfac, w_out, w_comp, base[0], wu[0],
-                                       jc0[0], gl, dither);
+          u_back_x<C, decltype(n)::value, 0, XM, ACC>(kr, rr, inv_l, w_out, w_comp, base[0],
+                                                       wu[0], gl, dither);
         else
-          u_back_x<C, decltype(n)::value, RS - 1, XM, ACC>(kr, inv_l, w_rho, S.gfac, w_out, w_comp,
-                                            base[RS - 1], wu[RS - 1], jc0[RS - 1], gl,
-                                            dither);
+          u_back_x<C, decltype(n)::value, RS - 1, XM, ACC>(kr, rr, inv_l, w_out, w_comp,
+                                                            base[RS - 1], wu[RS - 1], gl,
+                                                            dither);
       });
     }
   }
