@@ -76,7 +76,7 @@ struct jpet_strip {
   DevBuf<float> raw;                 // staging for uploaded events (kept for the next upload)
   DevBuf<float4> ev_geom, sorted_geom, over_geom;
   DevBuf<short4> ev_box, sorted_box, over_box;
-  DevBuf<int32_t> ev_key, tile_count, tile_offset, tile_cursor, hist, small;
+  DevBuf<int32_t> tile_count, hist, small;
   DevBuf<Chunk> chunks;
   DevBuf<uint16_t> row_table;
   DevBuf<float2> row_pq;     // per-row exponent coefficients of the row-owned kernel
@@ -407,7 +407,6 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   if (n > 0) {
     JPET_CUDA(h, h->ev_geom.alloc(n), "cudaMalloc(events)");
     JPET_CUDA(h, h->ev_box.alloc(n), "cudaMalloc(events)");
-    JPET_CUDA(h, h->ev_key.alloc(n), "cudaMalloc(events)");
   }
   JPET_CUDA(h, cudaMemsetAsync(h->hist.p, 0, 2 * kHistBins * sizeof(int32_t), s), "memset");
   JPET_CUDA(h, cudaMemsetAsync(h->box_pixels.p, 0, sizeof(unsigned long long), s), "memset");
@@ -446,26 +445,21 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   const Tiling& t = h->tiling;
   const int32_t n_tiles = t.n_tiles_x * t.n_tiles_y;
   JPET_CUDA(h, h->tile_count.alloc(n_tiles), "cudaMalloc(tiles)");
-  JPET_CUDA(h, h->tile_offset.alloc(n_tiles), "cudaMalloc(tiles)");
-  JPET_CUDA(h, h->tile_cursor.alloc(n_tiles), "cudaMalloc(tiles)");
   JPET_CUDA(h, cudaMemsetAsync(h->tile_count.p, 0, n_tiles * sizeof(int32_t), s), "memset");
-  JPET_CUDA(h, cudaMemsetAsync(h->tile_cursor.p, 0, n_tiles * sizeof(int32_t), s), "memset");
-  JPET_CUDA(h, launch_key_events(t, n, h->ev_box.p, h->ev_key.p, h->tile_count.p, h->small.p, s),
-            "key_events launch");
+  JPET_CUDA(h, launch_count_tiles(t, n, h->ev_box.p, h->tile_count.p, h->small.p, s),
+            "count_tiles launch");
   std::vector<int32_t> count(n_tiles);
   int32_t n_over = 0;
   JPET_CUDA(h, cudaMemcpyAsync(count.data(), h->tile_count.p, n_tiles * sizeof(int32_t),
                                cudaMemcpyDeviceToHost, s), "copy tile counts");
   JPET_CUDA(h, cudaMemcpyAsync(&n_over, h->small.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s),
             "copy counter");
-  JPET_CUDA(h, cudaStreamSynchronize(s), "key_events");
-  // exclusive scan over tiles and chunk list (full chunks first, then the
+  JPET_CUDA(h, cudaStreamSynchronize(s), "count_tiles");
+  // chunk list over the tiles' ranges of the sorted events (full chunks first, then the
   // partial tail chunks by decreasing size, so the longest work starts first)
-  std::vector<int32_t> offset(n_tiles);
   std::vector<Chunk> full, partial;
   int32_t acc = 0;
   for (int32_t k = 0; k < n_tiles; ++k) {
-    offset[k] = acc;
     const int32_t c = count[k];
     if (c > 0) ++h->n_tiles_nonempty;
     const int32_t ox = (k % t.n_tiles_x) * t.tile_w, oy = (k / t.n_tiles_x) * t.tile_h;
@@ -482,8 +476,6 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   h->n_oversize = n_over;
   h->n_chunks = static_cast<int32_t>(full.size());
   JPET_CUDA(h, h->chunks.alloc(std::max<size_t>(full.size(), 1)), "cudaMalloc(chunks)");
-  JPET_CUDA(h, cudaMemcpyAsync(h->tile_offset.p, offset.data(), n_tiles * sizeof(int32_t),
-                               cudaMemcpyHostToDevice, s), "copy tile offsets");
   JPET_CUDA(h, h->sorted_geom.alloc(std::max(acc, 1)), "cudaMalloc(sorted events)");
   JPET_CUDA(h, h->sorted_box.alloc(std::max(acc, 1)), "cudaMalloc(sorted events)");
   JPET_CUDA(h, h->over_geom.alloc(std::max(n_over, 1)), "cudaMalloc(large events)");
@@ -546,7 +538,6 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   // unsorted copies and sort buffers are no longer needed
   h->ev_geom.release();
   h->ev_box.release();
-  h->ev_key.release();
   h->sort_keys.release();
   h->sort_idx.release();
   h->sort_tmp.release();
@@ -849,10 +840,7 @@ int jpet_strip_destroy(jpet_strip_t* h) {
   h->ev_box.release();
   h->sorted_box.release();
   h->over_box.release();
-  h->ev_key.release();
   h->tile_count.release();
-  h->tile_offset.release();
-  h->tile_cursor.release();
   h->hist.release();
   h->small.release();
   h->chunks.release();

@@ -116,13 +116,8 @@ cudaError_t launch_prep_events(const DevGeom& g, const float* z_u, const float* 
                                const float* dl, int32_t stride, int64_t n, float4* ev_geom,
                                short4* ev_box, int32_t* hist_w, int32_t* hist_h,
                                unsigned long long* box_pixels, cudaStream_t s);
-cudaError_t launch_key_events(const Tiling& t, int64_t n, const short4* ev_box, int32_t* ev_key,
-                              int32_t* tile_count, int32_t* n_oversize, cudaStream_t s);
-cudaError_t launch_scatter_events(int64_t n, const float4* ev_geom, const short4* ev_box,
-                                  const int32_t* ev_key, const int32_t* tile_offset,
-                                  int32_t* tile_cursor, float4* sorted_geom, short4* sorted_box,
-                                  int32_t* over_cursor, float4* over_geom, short4* over_box,
-                                  cudaStream_t s);
+cudaError_t launch_count_tiles(const Tiling& t, int64_t n, const short4* ev_box,
+                               int32_t* tile_count, int32_t* n_oversize, cudaStream_t s);
 cudaError_t launch_fill(float* p, float v, int64_t n, cudaStream_t s);
 // Exact in-ellipse column interval of every box row of every sorted event
 // (GaussianKernel::in_ellipse evaluated in the reference's rounding),
