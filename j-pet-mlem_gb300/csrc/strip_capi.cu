@@ -37,8 +37,9 @@ template <typename T>
 struct DevBuf {
   T* p = nullptr;
   size_t n = 0;
+  bool own = true;  // else a part of a block (carve)
   cudaError_t alloc(size_t count) {
-    if (count <= n && p) return cudaSuccess;
+    if (count <= n && p && own) return cudaSuccess;
     release();
     if (count == 0) return cudaSuccess;
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), count * sizeof(T));
@@ -51,11 +52,40 @@ struct DevBuf {
     return cudaSuccess;
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p && own) cudaFree(p);
     p = nullptr;
     n = 0;
+    own = true;
   }
 };
+
+// Several buffers as parts of one block, so that an event set costs a few
+// cudaMalloc / cudaFree calls and not twenty (65 to 250 us a pair): layout names
+// the buffers and their sizes, once to add them up and once to place them.
+struct Carver {
+  unsigned char* base;
+  size_t used;
+  template <class T>
+  void operator()(DevBuf<T>& b, size_t count) {
+    b.release();
+    if (base) {
+      b.p = reinterpret_cast<T*>(base + used);
+      b.n = count;
+      b.own = false;
+    }
+    used += (count * sizeof(T) + 255) & ~static_cast<size_t>(255);
+  }
+};
+template <class F>
+cudaError_t carve(DevBuf<unsigned char>& block, F layout) {
+  Carver size{nullptr, 0};
+  layout(size);
+  const cudaError_t e = block.alloc(size.used);
+  if (e != cudaSuccess) return e;
+  Carver place{block.p, 0};
+  layout(place);
+  return cudaSuccess;
+}
 
 }  // namespace
 
@@ -77,6 +107,7 @@ struct jpet_strip {
   DevBuf<float4> ev_geom, sorted_geom, over_geom;
   DevBuf<short4> ev_box, sorted_box, over_box;
   DevBuf<int32_t> tile_count, hist, small;
+  DevBuf<unsigned char> scratch, set_block;  // of the set-up; of the prepared events
   DevBuf<Chunk> chunks;
   DevBuf<uint16_t> row_table;
   DevBuf<float2> row_pq;     // per-row exponent coefficients of the row-owned kernel
@@ -401,16 +432,22 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   h->total_box_pixels = 0;
   if (n > (int64_t)INT32_MAX - 1)
     return h->fail(JPET_ERR_ARGUMENT, "at most %d events per handle", INT32_MAX - 1);
-  JPET_CUDA(h, h->hist.alloc(2 * kHistBins), "cudaMalloc(histogram)");
-  JPET_CUDA(h, h->box_pixels.alloc(1), "cudaMalloc(counter)");
-  JPET_CUDA(h, h->small.alloc(4), "cudaMalloc(counter)");
-  if (n > 0) {
-    JPET_CUDA(h, h->ev_geom.alloc(n), "cudaMalloc(events)");
-    JPET_CUDA(h, h->ev_box.alloc(n), "cudaMalloc(events)");
-  }
-  JPET_CUDA(h, cudaMemsetAsync(h->hist.p, 0, 2 * kHistBins * sizeof(int32_t), s), "memset");
-  JPET_CUDA(h, cudaMemsetAsync(h->box_pixels.p, 0, sizeof(unsigned long long), s), "memset");
-  JPET_CUDA(h, cudaMemsetAsync(h->small.p, 0, 4 * sizeof(int32_t), s), "memset");
+  const size_t sort_bytes = n > 0 ? sort_temp_bytes(n) : 0;
+  JPET_CUDA(h, carve(h->scratch, [&](Carver& c) {
+              c(h->hist, 2 * kHistBins);
+              c(h->box_pixels, 1);
+              c(h->small, 4);
+              c(h->ev_geom, n);
+              c(h->ev_box, n);
+              c(h->sort_keys, 2 * static_cast<size_t>(n));
+              c(h->sort_idx, 2 * static_cast<size_t>(n));
+              c(h->sort_tmp, sort_bytes);
+            }),
+            "cudaMalloc(event set-up)");
+  // the counters and histograms, placed first
+  JPET_CUDA(h, cudaMemsetAsync(h->scratch.p, 0,
+                               reinterpret_cast<unsigned char*>(h->ev_geom.p) - h->scratch.p, s),
+            "memset");
   JPET_CUDA(h, launch_prep_events(h->g, d_zu, d_zd, d_dl, stride, n, h->ev_geom.p, h->ev_box.p,
                                   h->hist.p, h->hist.p + kHistBins, h->box_pixels.p, s),
             "prep_events launch");
@@ -475,39 +512,39 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   h->n_sorted = acc;
   h->n_oversize = n_over;
   h->n_chunks = static_cast<int32_t>(full.size());
-  JPET_CUDA(h, h->chunks.alloc(std::max<size_t>(full.size(), 1)), "cudaMalloc(chunks)");
-  JPET_CUDA(h, h->sorted_geom.alloc(std::max(acc, 1)), "cudaMalloc(sorted events)");
-  JPET_CUDA(h, h->sorted_box.alloc(std::max(acc, 1)), "cudaMalloc(sorted events)");
-  JPET_CUDA(h, h->over_geom.alloc(std::max(n_over, 1)), "cudaMalloc(large events)");
-  JPET_CUDA(h, h->over_box.alloc(std::max(n_over, 1)), "cudaMalloc(large events)");
+  h->use_fast = h->opts.mode == JPET_MODE_CPU_REFERENCE && h->opts.variant != JPET_VARIANT_EXACT;
+  h->use_union = h->use_fast && h->opts.variant == JPET_VARIANT_FAST;
+  const size_t n_acc = static_cast<size_t>(acc), table = n_acc * t.row_stride;
+  const bool rows_k = h->use_fast && h->opts.variant == JPET_VARIANT_ROWS;
+  JPET_CUDA(h, carve(h->set_block, [&](Carver& c) {
+              c(h->chunks, full.size());
+              c(h->sorted_geom, n_acc);
+              c(h->sorted_box, n_acc);
+              c(h->over_geom, n_over);
+              c(h->over_box, n_over);
+              c(h->row_table, h->use_fast ? table : 0);
+              c(h->batches, h->use_union ? n_acc : 0);
+              c(h->union_rows, h->use_union ? n_acc * union_row_words(t) : 0);
+              c(h->row_pq, rows_k ? table : 0);
+              c(h->row_pk, rows_k ? table : 0);
+              c(h->ev_pk, rows_k ? n_acc : 0);
+            }),
+            "cudaMalloc(events)");
+  // the last allocation of the event set: it takes what it can get
+  if (h->use_union) JPET_CUDA(h, alloc_records(h, full, acc), "cudaMalloc(row records)");
   if (n > 0) {
     // tile, then box corner inside the tile, then tan (strip_sort.cu)
-    const size_t tmp = sort_temp_bytes(n);
-    JPET_CUDA(h, h->sort_keys.alloc(2 * static_cast<size_t>(n)), "cudaMalloc(sort keys)");
-    JPET_CUDA(h, h->sort_idx.alloc(2 * static_cast<size_t>(n)), "cudaMalloc(sort indices)");
-    JPET_CUDA(h, h->sort_tmp.alloc(std::max<size_t>(tmp, 1)), "cudaMalloc(sort scratch)");
     JPET_CUDA(h, sort_events(t, n, h->ev_geom.p, h->ev_box.p, h->sort_keys.p, h->sort_idx.p,
-                             h->sort_tmp.p, tmp, acc, n_over, h->sorted_geom.p, h->sorted_box.p,
+                             h->sort_tmp.p, sort_bytes, acc, n_over, h->sorted_geom.p, h->sorted_box.p,
                              h->over_geom.p, h->over_box.p, s),
               "event sort");
   }
-  h->use_fast = h->opts.mode == JPET_MODE_CPU_REFERENCE && h->opts.variant != JPET_VARIANT_EXACT;
-  h->use_union = h->use_fast && h->opts.variant == JPET_VARIANT_FAST;
   h->table_kernel_calls = 0;
   if (h->use_fast && acc > 0) {
-    JPET_CUDA(h, h->row_table.alloc(static_cast<size_t>(acc) * t.row_stride),
-              "cudaMalloc(row table)");
     JPET_CUDA(h, cudaMemsetAsync(h->box_pixels.p, 0, sizeof(unsigned long long), s), "memset");
     JPET_CUDA(h, launch_row_tables(h->g, t, acc, h->sorted_geom.p, h->sorted_box.p,
                                    h->row_table.p, h->box_pixels.p, s),
               "row_table launch");
-    if (h->use_union) {
-      JPET_CUDA(h, h->batches.alloc(static_cast<size_t>(acc)), "cudaMalloc(batches)");
-      JPET_CUDA(h, h->union_rows.alloc(static_cast<size_t>(acc) * union_row_words(t)),
-                "cudaMalloc(union rows)");
-      // the last allocation of the event set: it takes what it can get
-      JPET_CUDA(h, alloc_records(h, full, acc), "cudaMalloc(row records)");
-    }
     JPET_CUDA(h, cudaMemcpyAsync(h->chunks.p, full.data(), full.size() * sizeof(Chunk),
                                  cudaMemcpyHostToDevice, s), "copy chunks");
     if (h->use_union) {
@@ -517,12 +554,7 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
       if (h->parts.size() == 1) JPET_CUDA(h, write_records(h, 0, s), "row record launch");
       JPET_CUDA(h, union_prepare_kernel(t, precision_code(h->opts.precision)),
                 "batch-union kernel attributes");
-    } else if (h->opts.variant == JPET_VARIANT_FAST || h->opts.variant == JPET_VARIANT_ROWS) {
-      JPET_CUDA(h, h->row_pq.alloc(static_cast<size_t>(acc) * t.row_stride),
-                "cudaMalloc(row coefficients)");
-      JPET_CUDA(h, h->row_pk.alloc(static_cast<size_t>(acc) * t.row_stride),
-                "cudaMalloc(row words)");
-      JPET_CUDA(h, h->ev_pk.alloc(static_cast<size_t>(acc)), "cudaMalloc(event words)");
+    } else if (rows_k) {
       JPET_CUDA(h, launch_row_coefficients(h->g, h->fc, t, acc, h->sorted_geom.p,
                                            h->sorted_box.p, h->row_table.p, h->row_pq.p,
                                            h->row_pk.p, h->ev_pk.p, s),
@@ -535,12 +567,7 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
               "copy counter");
   }
   JPET_CUDA(h, cudaStreamSynchronize(s), "prepare events");
-  // unsorted copies and sort buffers are no longer needed
-  h->ev_geom.release();
-  h->ev_box.release();
-  h->sort_keys.release();
-  h->sort_idx.release();
-  h->sort_tmp.release();
+  h->scratch.release();
   h->events_ready = true;
   h->counters_valid = false;
   return JPET_OK;
@@ -834,27 +861,10 @@ int jpet_strip_destroy(jpet_strip_t* h) {
   h->sens_point.release();
   h->sens_pixel.release();
   h->raw.release();
-  h->ev_geom.release();
-  h->sorted_geom.release();
-  h->over_geom.release();
-  h->ev_box.release();
-  h->sorted_box.release();
-  h->over_box.release();
   h->tile_count.release();
-  h->hist.release();
-  h->small.release();
-  h->chunks.release();
-  h->row_table.release();
-  h->row_pq.release();
-  h->row_pk.release();
-  h->ev_pk.release();
-  h->sort_keys.release();
-  h->sort_idx.release();
-  h->sort_tmp.release();
-  h->batches.release();
-  h->union_rows.release();
+  h->scratch.release();
+  h->set_block.release();
   h->records.release();
-  h->box_pixels.release();
   h->nll_acc.release();
   h->nll_parts.release();
   h->counters.release();
