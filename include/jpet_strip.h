@@ -71,7 +71,8 @@ typedef struct jpet_strip_geom {
                                         each atomic found), with the tile compensations, go
                                         into an FP32 compensation image added at the end */
 #define JPET_PRECISION_FP64_DEN 2    /* as COMPENSATED, plus per-event denominators reduced
-                                        in FP64 (the only FP64 arithmetic of the modes) */
+                                        in double-floats, about 45 bits (FAST), or FP64 (the
+                                        other variants) */
 #define JPET_PRECISION_FIXED 3       /* deterministic image: each pixel's contribution of a
                                         batch of events (FAST) or of one event (ROWS) rounded
                                         once to 2^-22 of an event (unbiased dither), summed as

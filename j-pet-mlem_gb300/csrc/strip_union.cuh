@@ -31,8 +31,8 @@
 // cost 16 bytes per event and row of DRAM traffic, which the kernel otherwise
 // leaves idle (2e7 events at 2 mm: at most 20 GB per iteration, 2 TB/s).  Iterations,
 // computed on chip -> read: 2e7 events at 2 mm 12.39 -> 10.43 ms, 6e6 at 1 mm
-// 3.99 -> 3.37 ms, 1e6 at 5 mm 0.293 -> 0.244 ms, 1e6 at 2 mm with sigma 14 / 60
-// 1.49 -> 1.28 ms, 2e6 at 2 mm compensated 2.38 -> 2.06 ms.
+// 3.99 -> 3.37 ms, 1e6 at 5 mm 0.293 -> 0.244 ms, 1e6 at 2 mm with sigma 14 / 55
+// 1.49 -> 1.28 ms, 2e6 at 2 mm compensated 1.59 -> 1.37 ms.
 // With the records read, the shared-memory pipe is 63 % busy; rho'' kept in
 // registers from the forward sums to the back-projection instead of read and
 // multiplied again there (the compiler has room for it: 123 registers): 2e7 at
@@ -41,8 +41,9 @@
 // Accumulation modes (template argument ACC, DEN64): FP32 windows flushed with
 // float atomics; compensated windows (each batch's addition followed by
 // Knuth's TwoSum into a compensation window, flushed into the FP32 image and
-// its FP32 compensation image); FP64 denominators on top of that (lane
-// partials over <= 8 pixels in FP32, the sums across lanes and warps in FP64);
+// its FP32 compensation image); denominators in double-floats on top of that
+// (lane partials over <= 8 pixels in FP32, the sums across lanes and warps as
+// USum);
 // fixed-point integer windows (a batch's value rounded once to 2^-22 of an
 // event with a per-batch dither, flushed into the 64-bit integer image).
 //
@@ -135,11 +136,74 @@ __device__ __forceinline__ uint32_t u_lane_mask(uint32_t m) {
   t = (m ^ (m >> 12)) & 0x0000F0F0u;
   return m ^ t ^ (t << 12);
 }
+// Denominator sums of the FP64_DEN mode: double-floats (value h + l, |l| of the
+// order of h's last bit; the partials are positive, so a sum of a few hundred
+// keeps about 45 bits, of which the reciprocal takes 24).  In FP64 the 17 additions
+// of a warp's batch were the bound, at 1/64 of the FP32 rate: 2e6 events at 2 mm
+// 3.49 -> 1.50 ms per iteration, 1e6 at 5 mm 0.97 -> 0.33 ms, 1e6 at 2 mm with
+// sigma 14 / 55 3.75 -> 1.60 ms; against an FP64 image the error is the same
+// (8.6e-7 to 1.5e-5 after 1 to 10 iterations, the single-precision evaluation's).
+struct __align__(8) USum {
+  float h, l;
+  __device__ __forceinline__ explicit USum(float v) : h(v), l(0.0f) {}
+  USum() = default;
+};
+__device__ __forceinline__ USum u_two_sum(float a, float b) {
+  USum r;
+  r.h = __fadd_rn(a, b);
+  const float v = __fsub_rn(r.h, a);
+  r.l = __fadd_rn(__fsub_rn(a, __fsub_rn(r.h, v)), __fsub_rn(b, v));
+  return r;
+}
+__device__ __forceinline__ USum operator+(USum a, USum b) {
+  USum r = u_two_sum(a.h, b.h);
+  r.l = __fadd_rn(r.l, __fadd_rn(a.l, b.l));
+  return r;
+}
+__device__ __forceinline__ USum u_from_lane(USum v, int off) {
+  USum r;
+  r.h = __shfl_xor_sync(kFull, v.h, off);
+  r.l = __shfl_xor_sync(kFull, v.l, off);
+  return r;
+}
+// an overflow leaves h infinite and l not a number
+__device__ __forceinline__ float u_value(USum v) {
+  const float f = __fadd_rn(v.h, v.l);
+  return f == f ? f : v.h;
+}
+// Warp sums of E values per lane, transposed as rows_transpose_sum does it.
+// PLAIN: the lanes' values have no low part yet.
+template <int E, bool PLAIN>
+__device__ __forceinline__ USum u_warp_sum(USum (&v)[E]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int n = E, off = 16; off > 0; off >>= 1) {
+    if (n == 1) {
+      v[0] = v[0] + u_from_lane(v[0], off);
+      continue;
+    }
+    const bool hi = (lane & off) != 0;
+    n /= 2;
+#pragma unroll
+    for (int k = 0; k < E / 2; ++k) {
+      if (k >= n) break;
+      const USum send = hi ? v[k] : v[k + n], keep = hi ? v[k + n] : v[k];
+      v[k] = PLAIN && off == 16 ? u_two_sum(keep.h, __shfl_xor_sync(kFull, send.h, off))
+                                : keep + u_from_lane(send, off);
+    }
+  }
+  return v[0];
+}
+template <int E, bool PLAIN>
+__device__ __forceinline__ float u_warp_sum(float (&v)[E]) {
+  return rows_transpose_sum<E>(v);
+}
+
 template <class C, class DT>
 struct USmem {
   float4 rec[2][C::E][C::kRows];  // records of two batches
   uint16_t urow[2][C::kRows];     // their union row words
-  __align__(16) DT den_part[2][C::E][C::kPartials];  // float, or double (FP64 denominators)
+  __align__(16) DT den_part[2][C::E][C::kPartials];  // warp sums of the denominators
   float gfac[2 * C::kCols];          // 2^(c jc^2), jc = index - kCols (split exponent)
   float cjc[2 * C::kCols];           // c jc^2 (full exponent)
   uint32_t bw[4];  // the chunk's batch words and exact-path list: chunk_events + 4 words,
@@ -227,7 +291,8 @@ __device__ __forceinline__ void u_forward(float2 (&kr)[C::E][C::RS][C::SW], DT (
       kr[j][RSI][s] = v;
       dd = __fadd2_rn(dd, v);
     }
-    dsum[j] += static_cast<DT>(dd.x + dd.y);
+    const DT pr(dd.x + dd.y);
+    dsum[j] = (RSI == 0) ? pr : dsum[j] + pr;
   }
 }
 
@@ -262,9 +327,9 @@ __device__ __forceinline__ void u_forward_chain(float2 (&kr)[C::E][C::RS][C::SW]
       kr[j][RSI][s] = v;
       dd = (s == 0) ? __fmul2_rn(v, rr[0]) : __ffma2_rn(v, rr[s], dd);
     }
-    // a lane's partial over its <= 8 pixels of the row in FP32; FP64 (DEN64)
+    // a lane's partial over its <= 8 pixels of the row in FP32; a USum (DEN64)
     // from the sums across lanes and warps on
-    const DT pr = static_cast<DT>(dd.x + dd.y);
+    const DT pr(dd.x + dd.y);
     dsum[j] = (RSI == 0) ? pr : dsum[j] + pr;
   }
 }
@@ -417,7 +482,7 @@ __device__ __forceinline__ void u_back_x(const float2 (&kr)[C::E][C::RS][C::SW],
 // compensation window of the compensated modes), then the batch records.
 template <class C, int ACC, bool DEN64>
 size_t u_smem(const Tiling& t) {
-  using DT = typename std::conditional<DEN64, double, float>::type;
+  using DT = typename std::conditional<DEN64, USum, float>::type;
   return (ACC == kAccCompensated ? 3ull : 2ull) * fast_window_floats(t) * sizeof(float) +
          sizeof(USmem<C, DT>) + static_cast<size_t>(t.chunk_events) * sizeof(uint32_t);
 }
@@ -425,7 +490,7 @@ size_t u_smem(const Tiling& t) {
 // ACC: kAccFloat (the FP32 iteration), kAccCompensated (tile windows with
 // TwoSum compensation, flushed into the FP32 image and its FP32 compensation
 // image), kAccFixed (integer tile windows flushed into the 64-bit fixed-point
-// image); DEN64: per-event denominators reduced in FP64.
+// image); DEN64: per-event denominators reduced in double-floats.
 template <class C, int XM, int ACC, bool DEN64>
 __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel(
     DevGeom g, FastConst fc, Tiling t, const Chunk* __restrict__ chunks,
@@ -434,7 +499,7 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
     const uint32_t* __restrict__ batches,
     const float* __restrict__ rho, float* __restrict__ out, AuxImage aux, uint32_t seed,
     DevCounters* counters) {
-  using DT = typename std::conditional<DEN64, double, float>::type;
+  using DT = typename std::conditional<DEN64, USum, float>::type;
   constexpr int NW = C::NW, E = C::E, RS = C::RS, SW = C::SW;
   constexpr int kRowsPerStep = NW * 8;  // union rows per step of all warps
   constexpr int kWindows = ACC == kAccCompensated ? 3 : 2;
@@ -494,7 +559,7 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
     float2 kr[E][RS][SW], rr[RS][SW];  // K' (chain) or K rho''; rho'' (chain)
     DT dsum[E];
 #pragma unroll
-    for (int j = 0; j < E; ++j) dsum[j] = DT(0);
+    for (int j = 0; j < E; ++j) dsum[j] = DT(0.0f);
     int base[RS], wu[RS], nsw[RS], jc0[RS];
 #pragma unroll
     for (int rs = 0; rs < RS; ++rs) {
@@ -514,7 +579,7 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
       u_sweeps<SW>(nsw[0], [&](auto n) {
         u_forward_x<C, decltype(n)::value, 0, XM, DT>(kr, dsum, rr, w_rho, S, buf, base[0],
                                                       8 * warp + gid, jc0[0], gl);
-        tot = rows_transpose_sum<E>(dsum);
+        tot = u_warp_sum<E, RS == 1>(dsum);
       });
     } else {
       u_sweeps<SW>(nsw[0], [&](auto n) {
@@ -526,7 +591,7 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
                                                            kRowsPerStep + 8 * warp + gid,
                                                            jc0[RS - 1], gl);
       });
-      tot = rows_transpose_sum<E>(dsum);
+      tot = u_warp_sum<E, RS == 1>(dsum);
     }
     if (rows_lane_writes<E>(lane)) S.den_part[buf][rows_lane_event<E>(lane)][warp] = tot;
     // the barrier also publishes the next batch's records (this thread's copies,
@@ -538,11 +603,18 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
     float inv_l;
     {
       const int jl = lane & (E - 1);
-      DT den;
+      float den;
       if constexpr (DEN64) {
-        den = S.den_part[buf][jl][0];
+        // 32 / E lanes share an event's partials
+        USum d(0.0f);
 #pragma unroll
-        for (int w = 1; w < NW; ++w) den += S.den_part[buf][jl][w];
+        for (int i = 0; i < NW; i += 32 / E) {
+          const int w = i + lane / E;
+          if (w < NW) d = i == 0 ? S.den_part[buf][jl][w] : d + S.den_part[buf][jl][w];
+        }
+#pragma unroll
+        for (int off = E; off < 32; off *= 2) d = d + u_from_lane(d, off);
+        den = u_value(d);
       } else {
         const float4* dp = reinterpret_cast<const float4*>(S.den_part[buf][jl]);
         const float4 d0 = dp[0];
@@ -553,8 +625,8 @@ __global__ void __launch_bounds__(C::kThreads, C::kMinCtas) iterate_union_kernel
           den += (d1.x + d1.y) + (d1.z + d1.w);
         }
       }
-      const bool ok = den > DT(0);  // inv_denominator = 0 otherwise (reconstruction.h:290)
-      inv_l = ok ? rcp_approx(static_cast<float>(den)) : 0.0f;
+      const bool ok = den > 0.0f;  // inv_denominator = 0 otherwise (reconstruction.h:290)
+      inv_l = ok ? rcp_approx(den) : 0.0f;
       const unsigned okm = __ballot_sync(kFull, ok && lane < cnt);
       if (threadIdx.x == 0) contrib += __popc(okm);
     }
