@@ -26,7 +26,7 @@
 // One warp per event.  The lanes set up a block of rows, 32 at a time and one each
 // (the exact in-ellipse interval of the MLEM row tables, so the support is exactly
 // the reference's, read from the row table where the handle has one, and the row's
-// terms), then sweep the rows with 8, 16 or 32 lanes each; the first kNllCache
+// terms), then sweep the rows with 4 to 32 lanes each, two pixels a lane; the first kNllCache
 // kernel values are kept for the gradient pass, which adds them with
 // float reductions to one of a few partial images (many small additions to one
 // float image lose digits; nll_finish_kernel sums the partial images in FP64).
@@ -38,8 +38,10 @@
 // FP32 values, Dekker 1971; the sum and product errors are Knuth's TwoSum and an
 // FMA).  5e5 events of 1763 pixels (2 mm, support 14 / 55): 8.0 ms with FP64 row
 // terms and per-event FP64 on one lane (FP64 pipe 70-81 % busy) and float
-// atomics on windows in shared memory, 3.65 ms now (FP64 pipe 3 %), bound by
-// instruction issue (63 % of the slots, 52 instructions a pixel for both passes).
+// atomics on windows in shared memory, 3.65 ms with all that (FP64 pipe 3 %), bound
+// by instruction issue (63 % of the slots, 52 instructions a pixel for both
+// passes); 2.92 ms with two pixels a lane in packed arithmetic (rows unrolled by
+// 2; by 1, 3 and 4: 3.31, 3.04 and 3.00).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -86,8 +88,8 @@ __device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
   return s;
 }
 // sum over the warp's lanes
-__device__ __forceinline__ Pair pair_warp_sum(float v) {
-  Pair s{v, 0.0f};
+__device__ __forceinline__ Pair pair_warp_sum(float2 v) {
+  Pair s = two_sum(v.x, v.y);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const Pair other{__shfl_xor_sync(kFull, s.h, o), __shfl_xor_sync(kFull, s.l, o)};
@@ -236,51 +238,67 @@ __global__ void __launch_bounds__(32 * kNllWarps) nll_kernel(
         }
         __syncwarp();
       };
-      // f(row, its record, pixel of the row, that as a float, whether there is such a
-      // pixel) over a block's pixels: as many lanes per row as fit the widest, four
-      // rows in flight, lanes past a row's end along without a branch
+      // f(row, its record, pixel of the row, that and the lane's other pixel as
+      // floats, how far on that is, whether there are such pixels) over a block's
+      // pixels: two pixels per lane, as many lanes per row as then fit the widest,
+      // two rows in flight, lanes past a row's end along without a branch.  A
+      // lane's pixels are a row's lanes apart, so that neighbouring lanes read
+      // and add to neighbouring pixels.
       auto walk = [&](auto&& f) {
-        const int sh = widest <= 8 ? 3 : widest <= 16 ? 4 : 5;
-        const int l = lane & ((1 << sh) - 1);
-        const float fl = static_cast<float>(l);
-#pragma unroll 4
+        const int sh = widest <= 8 ? 2 : widest <= 16 ? 3 : widest <= 32 ? 4 : 5;
+        const int l = lane & ((1 << sh) - 1), on = 1 << sh;
+        const float2 fl = make_float2(static_cast<float>(l), static_cast<float>(l + on));
+#pragma unroll 2
         for (int r0 = 0; r0 < n_rows; r0 += 32 >> sh) {
           const int r = min(r0 + (lane >> sh), n_rows - 1);
           const int4 at = s.at[r];
-          f(r, at, l, fl, l < (at.x >> 16) && r == r0 + (lane >> sh));
+          const int w = r == r0 + (lane >> sh) ? at.x >> 16 : 0;
+          f(r, at, l, fl, on, l < w, l + on < w);
         }
-        if (widest > 32) {
+        if (widest > 64) {
           for (int r = 0; r < n_rows; ++r) {
             const int4 at = s.at[r];
-            for (int i = lane + 32; i < (at.x >> 16); i += 32)
-              f(r, at, i, static_cast<float>(i), true);
+            const int w = at.x >> 16;
+            for (int i = lane + 64; i < w; i += 64)
+              f(r, at, i, make_float2(static_cast<float>(i), static_cast<float>(i + 32)), 32,
+                true, i + 32 < w);
           }
         }
       };
-      auto value = [&](const float4 r, float col, float& u) {
-        u = fmaf(col, g.pixel_width, r.w);
-        return exp2f(fmaf(k.kz * u, u, fmaf(k.kz_lo * u, u, r.x)));
+      auto value = [&](const float4 r, float2 col, float2& u) {
+        u = __ffma2_rn(col, make_float2(g.pixel_width, g.pixel_width), make_float2(r.w, r.w));
+        const float2 lo = __ffma2_rn(__fmul2_rn(make_float2(k.kz_lo, k.kz_lo), u), u,
+                                     make_float2(r.x, r.x));
+        const float2 e = __ffma2_rn(__fmul2_rn(make_float2(k.kz, k.kz), u), u, lo);
+        return make_float2(exp2f(e.x), exp2f(e.y));
       };
-      float den = 0.0f, dz = 0.0f, ddl = 0.0f;
+      float2 den = make_float2(0.0f, 0.0f), dz = den, ddl = den;
       int before = 0;  // pixels of the blocks before
       for (int rb = 0; rb < nrows; rb += step) {
         setup(rb);
-        walk([&](int r, const int4 at, int i, float fi, bool in) {
+        walk([&](int r, const int4 at, int i, float2 fi, int on, bool in0, bool in1) {
           const float4 row = s.row[r];
-          const float rh = in ? __ldg(&rho[at.y + i]) : 0.0f;
-          float u;
-          const float kv = value(row, __int_as_float(at.z) + fi, u);
-          const float kr = in ? kv * rh : 0.0f;
-          den += kr;
-          dz += kr * (row.y - u * u);
-          ddl += kr * row.z;
+          const float* rp = &rho[at.y + i];
+          const float2 rh = make_float2(in0 ? __ldg(rp) : 0.0f, in1 ? __ldg(rp + on) : 0.0f);
+          const float first = __int_as_float(at.z);
+          float2 u;
+          const float2 kv = value(row, __fadd2_rn(make_float2(first, first), fi), u);
+          float2 kr = __fmul2_rn(kv, rh);
+          kr.x = in0 ? kr.x : 0.0f;
+          kr.y = in1 ? kr.y : 0.0f;
+          den = __fadd2_rn(den, kr);
+          dz = __ffma2_rn(kr, __ffma2_rn(make_float2(-u.x, -u.y), u, make_float2(row.y, row.y)),
+                          dz);
+          ddl = __ffma2_rn(kr, make_float2(row.z, row.z), ddl);
           const int c = before + (at.x & 0xffff) + i;
-          if (GRAD && in && c < kNllCache) s.cache[c] = kv;
+          if (GRAD && in0 && c < kNllCache) s.cache[c] = kv.x;
+          if (GRAD && in1 && c + on < kNllCache) s.cache[c + on] = kv.y;
         });
         before = min(before + total, kNllCache);
       }
       const Pair d = pair_warp_sum(den);
-      const Pair a = pair_warp_sum(dz * k.dipz_dsz), b = pair_warp_sum(ddl * k.dipd_dsdl);
+      const Pair a = pair_warp_sum(make_float2(dz.x * k.dipz_dsz, dz.y * k.dipz_dsz)),
+                 b = pair_warp_sum(make_float2(ddl.x * k.dipd_dsdl, ddl.y * k.dipd_dsdl));
       if (lane == j) {
         den_j = d;
         dz_j = a;
@@ -288,16 +306,23 @@ __global__ void __launch_bounds__(32 * kNllWarps) nll_kernel(
       }
       if (!GRAD || !(d.h > 0.0f)) continue;
       const float i0 = __frcp_rn(d.h);
-      const float inv = fmaf(fmaf(-d.h, i0, 1.0f) - d.l * i0, i0, i0);
+      const float minus_inv = -fmaf(fmaf(-d.h, i0, 1.0f) - d.l * i0, i0, i0);
       before = 0;
       for (int rb = 0; rb < nrows; rb += step) {
         if (nrows > step) setup(rb);
-        walk([&](int r, const int4 at, int i, float fi, bool in) {
+        walk([&](int r, const int4 at, int i, float2 fi, int on, bool in0, bool in1) {
           const int c = before + (at.x & 0xffff) + i;
-          float u;
-          float kv = s.cache[min(c, kNllCache - 1)];
-          if (in && c >= kNllCache) kv = value(s.row[r], __int_as_float(at.z) + fi, u);
-          if (in) atomicAdd(&grad[at.y + i], -kv * inv);
+          float2 kv = make_float2(s.cache[min(c, kNllCache - 1)],
+                                  s.cache[min(c + on, kNllCache - 1)]);
+          if (in0 && c + on >= kNllCache) {  // not kept (either pixel, or none in the row)
+            const float first = __int_as_float(at.z);
+            float2 u;
+            const float2 v = value(s.row[r], __fadd2_rn(make_float2(first, first), fi), u);
+            if (c >= kNllCache) kv.x = v.x;
+            kv.y = v.y;
+          }
+          if (in0) atomicAdd(&grad[at.y + i], kv.x * minus_inv);
+          if (in1) atomicAdd(&grad[at.y + i + on], kv.y * minus_inv);
         });
         before = min(before + total, kNllCache);
       }
