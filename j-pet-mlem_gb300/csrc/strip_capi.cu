@@ -254,9 +254,9 @@ UnionLimits union_limits(const jpet_strip_opts& o, int rows, int widest) {
   // a batch's rows are wider than its events' by a column of alignment and, at
   // the ends of the box, by the spread of slopes in half a sort bucket
   const bool narrow = widest + 1 + rows / 8 <= 16;
-  if (rows <= 30 && narrow) return UnionLimits{kUnion32x16, 3328, 5, 1024};
+  if (rows <= 30 && narrow) return UnionLimits{kUnion32x16, 3328, 4, 1024};
   if (rows <= 30 && widest <= 28) return UnionLimits{kUnion32x32, 3328, 4, 1024};
-  if (rows <= 64 && narrow) return UnionLimits{kUnion64x16, 4096, 3, 1024};
+  if (rows <= 64 && narrow) return UnionLimits{kUnion64x16, 4096, 2, 1024};
   if (rows <= 64 && widest <= 28) return m;
   return UnionLimits{kUnion96x40, 10752, 1, 1024};
 }

@@ -54,10 +54,10 @@ struct Tiling {
 enum UnionShape : int32_t {
   kUnion64x32 = 0,    // 8 warps, 8 events
   kUnion64x32n4 = 1,  // 4 warps, 4 events
-  kUnion32x16 = 2,    // 4 warps, 8 events
+  kUnion32x16 = 2,    // 4 warps, 16 events
   kUnion32x32 = 3,    // 4 warps, 8 events
   kUnion96x40 = 4,    // 12 warps, 8 events
-  kUnion64x16 = 5,    // 8 warps, 8 events
+  kUnion64x16 = 5,    // 8 warps, 16 events
 };
 
 // Register-cache shapes of the fast iteration kernel: 4 lanes per image row,

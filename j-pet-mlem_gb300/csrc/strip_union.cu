@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256) union_records_kernel(
     const float4* __restrict__ ev_geom, const short4* __restrict__ ev_box,
     const uint16_t* __restrict__ rows, const uint32_t* __restrict__ batches,
     const uint16_t* __restrict__ urows, float4* __restrict__ records) {
-  constexpr int kMaxEvents = 8;
+  constexpr int kMaxEvents = 16;
   __shared__ __align__(16) URecordEvent events[8][kMaxEvents];
   const Chunk c = chunks[blockIdx.x];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

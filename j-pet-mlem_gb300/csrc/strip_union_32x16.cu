@@ -5,7 +5,7 @@
 namespace jpet {
 
 const UnionOps& union_ops_32x16() {
-  static const UnionOps ops = UnionHost<UShape<4, 8, 2, 1, 5>>::ops();
+  static const UnionOps ops = UnionHost<UShape<4, 16, 2, 1, 4>>::ops();
   return ops;
 }
 

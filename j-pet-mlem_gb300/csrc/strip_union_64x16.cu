@@ -5,7 +5,7 @@
 namespace jpet {
 
 const UnionOps& union_ops_64x16() {
-  static const UnionOps ops = UnionHost<UShape<8, 8, 2, 1, 3>>::ops();
+  static const UnionOps ops = UnionHost<UShape<8, 16, 2, 1, 2>>::ops();
   return ops;
 }
 
