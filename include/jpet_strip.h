@@ -81,10 +81,12 @@ typedef struct jpet_strip_geom {
 
 /* iteration kernel */
 #define JPET_VARIANT_FAST 0  /* default, every precision: batch-union kernel -- batches of
-                                <= 8 similar events share one lane-to-pixel map, rho is read
-                                and the back-projection written once per batch, exp2-form
-                                kernel with packed f32x2, per-row coefficients regenerated
-                                on chip */
+                                <= 8 or 16 similar events share one lane-to-pixel map, rho is
+                                read and the back-projection written once per batch,
+                                exp2-form kernel with packed f32x2; per-row records of 16
+                                bytes written at set-up (0.5 to 1.5 KB per event, above
+                                1 GB at most half of the free memory: what does not fit is
+                                written again part by part in every iteration) */
 #define JPET_VARIANT_EXACT 1 /* every pixel evaluated in the reference's operation order */
 #define JPET_VARIANT_WARP 2  /* one warp per event, shared-memory atomics */
 #define JPET_VARIANT_ROWS 3  /* row-owned kernel: image rows owned by warps, one event at a
@@ -107,9 +109,9 @@ typedef struct jpet_strip_opts {
   int32_t precision;    /* JPET_PRECISION_* */
   int32_t tile_w;       /* image tile width in pixels, 0 = chosen by the tuner */
   int32_t tile_h;       /* image tile height in pixels, 0 = chosen by the tuner */
-  int32_t block_threads;/* threads per CTA of the iteration kernel, 0 = default (256 for
-                           the FAST kernel: 8 events per batch; 128 for the ROWS kernel;
-                           both take 128 or 256; 256 otherwise) */
+  int32_t block_threads;/* threads per CTA of the iteration kernel, 0 = default (FAST: 128
+                           to 384 by the events' boxes; 128 for the ROWS kernel; both
+                           take 128 or 256; 256 otherwise) */
   int32_t variant;      /* JPET_VARIANT_*; the GPU-reference mode always runs EXACT */
   int32_t raster_shape; /* JPET_RASTER_*; events outside the shape take the exact path */
   int32_t reserved[8];  /* must be zero */

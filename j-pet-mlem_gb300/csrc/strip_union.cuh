@@ -100,7 +100,7 @@ struct UShape {
   // batches of 16 events: two halves, the second only where the batch has it.
   // A batch's fixed costs (rows, sums over lanes and warps, barrier) are halved
   // where events are dense; 16 columns leave the registers for it.  1e6 events at
-  // 5 mm 0.243 -> 0.222 ms per iteration; 1e4 events the same.  Batches of 4
+  // 5 mm 0.243 -> 0.222 ms per iteration; 2e4 events the same.  Batches of 4
   // instead, with 3 CTAs of 8 warps per SM: 22 % slower at 2 mm, 17 % at 5 mm.
   static constexpr int H = E > 8 ? E / 8 : 1, kHalf = E / H;
   static constexpr int kRows = 8 * NW * RS;
