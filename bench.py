@@ -101,7 +101,7 @@ def config_of(wl, n_events, world):
     return {"workload": wl.name, "events": n_events, "grid": f"{wl.n_z}x{wl.n_y}",
             "pixel_mm": wl.pixel, "sigma_z": wl.sigma_z, "sigma_dl": wl.sigma_dl,
             "phantom": wl.phantom, "seed": wl.seed,
-            "l2": "inputs larger than L2 (prepared events and row tables, ~160 B each)",
+            "l2": "inputs larger than L2 (prepared events and row records, ~1 KB each)",
             "parallelism": f"replicas{world}"}
 
 
@@ -805,8 +805,8 @@ def adjoint_summary(local, n_events=5_000_000, ex2_peak=None, calibrate=True):
         # each evaluation needs one exp of K and its sigma derivatives
         out["roofline"] = {"bound": "sfu", "achieved": evals / dt / 1e9, "peak": ex2_peak / 1e9,
                            "unit": "Gex2/s", "frac": evals / dt / ex2_peak,
-                           "note": "FP64 row terms and sigma derivatives per evaluation; the "
-                                   "kernel is bound by FP64 and FP32 issue, not the SFU"}
+                           "note": "double-float row terms and sums; the kernel is bound by "
+                                   "instruction issue, not the SFU"}
     if calibrate:
         t0 = time.perf_counter()
         sigma, hist = calibrate_sigma(geom, ev, img, (14.0, 55.0), device=local)
