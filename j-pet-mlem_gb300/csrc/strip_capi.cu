@@ -607,18 +607,17 @@ int iterate_on(jpet_strip* h, int n, cudaStream_t s) {
   for (int it = 0; it < n; ++it) {
     // every variant adds into a cleared image: the exact kernel into its double one
     const bool exact = h->out_sum.p != nullptr;
+    ClearList clear;
     if (exact)
-      JPET_CUDA(h, cudaMemsetAsync(h->out_sum.p, 0, n_pix * sizeof(double), s), "clear image");
+      clear.add(h->out_sum.p, n_pix * sizeof(double));
     else
-      JPET_CUDA(h, cudaMemsetAsync(h->out.p, 0, n_pix * sizeof(float), s), "clear image");
-    JPET_CUDA(h, cudaMemsetAsync(h->counters.p, 0, sizeof(DevCounters), s), "clear counters");
+      clear.add(h->out.p, n_pix * sizeof(float));
+    clear.add(h->counters.p, sizeof(DevCounters));
     const bool aux_img = h->opts.precision != JPET_PRECISION_FP32;
     const AuxImage aux{h->out_lo.p, h->out_q.p};
-    if (h->out_lo.p)
-      JPET_CUDA(h, cudaMemsetAsync(h->out_lo.p, 0, n_pix * sizeof(float), s), "clear image");
-    if (h->out_q.p)
-      JPET_CUDA(h, cudaMemsetAsync(h->out_q.p, 0, n_pix * sizeof(unsigned long long), s),
-                "clear image");
+    if (h->out_lo.p) clear.add(h->out_lo.p, n_pix * sizeof(float));
+    if (h->out_q.p) clear.add(h->out_q.p, n_pix * sizeof(unsigned long long));
+    JPET_CUDA(h, launch_clear(clear, s), "clear image launch");
     if (h->use_fast) {
       const int prec = precision_code(h->opts.precision);
       const uint32_t seed = 0x9E3779B9u * static_cast<uint32_t>(h->iterations_done + 1);

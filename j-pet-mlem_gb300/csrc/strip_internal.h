@@ -118,6 +118,18 @@ cudaError_t launch_prep_events(const DevGeom& g, const float* z_u, const float* 
                                unsigned long long* box_pixels, cudaStream_t s);
 cudaError_t launch_count_tiles(const Tiling& t, int64_t n, const short4* ev_box,
                                int32_t* tile_count, int32_t* n_oversize, cudaStream_t s);
+// Buffers of whole 4-byte words, 16-byte aligned, set to zero in one launch.
+struct ClearList {
+  static constexpr int kMax = 4;
+  uint32_t* p[kMax];
+  int64_t words[kMax];
+  int n = 0;
+  void add(void* buffer, size_t bytes) {
+    p[n] = static_cast<uint32_t*>(buffer);
+    words[n++] = static_cast<int64_t>(bytes / sizeof(uint32_t));
+  }
+};
+cudaError_t launch_clear(const ClearList& list, cudaStream_t s);
 cudaError_t launch_fill(float* p, float v, int64_t n, cudaStream_t s);
 // Exact in-ellipse column interval of every box row of every sorted event
 // (GaussianKernel::in_ellipse evaluated in the reference's rounding),
