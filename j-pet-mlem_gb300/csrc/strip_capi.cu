@@ -314,18 +314,21 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
   t.n_tiles_x = (n_z + tw - 1) / tw;
   t.n_tiles_y = (n_y + th - 1) / th;
   // events per chunk of the batch-union kernel: the largest power of two (64 to
-  // 2048) that still leaves at least 16 chunks per resident CTA, or 4 below 512.
-  // Larger chunks mean fewer chunk prologues and window flushes (2e7 events at
-  // 2 mm: 13.50, 13.06, 12.88 ms per iteration with 512, 1024, 2048), but
-  // fewer chunks leave SMs idle at the end of the launch.  The fixed-point mode
-  // (whose integer window sums must stay below 2^31) takes at most 512, the
-  // other kernels 512.
+  // 2048) that still leaves at least 4 chunks per resident CTA, or 2 below 1024.
+  // Larger chunks mean fewer chunk prologues and window flushes, fewer chunks
+  // leave SMs idle at the end of the launch.  Us per iteration with 16 and 4, 8
+  // and 4 or 4 and 2 chunks: 2e6 events at 2 mm 1128, 1128, 1090; 3e6 1654, 1591,
+  // 1577; 2e5 190, 190, 177; 1e6 at 5 mm 225, 225, 206.  With 2 and 2: 1e6 at 3 mm
+  // 527 instead of 507; with 1 below 1024: 2e5 at 3 mm 160 instead of 136.  Chunks
+  // of 32 events: 2e4 at 5 mm 31 instead of 25.  The fixed-point mode (whose
+  // integer window sums must stay below 2^31) takes at most 512, the other
+  // kernels 512.
   t.chunk_events = 512;
   if (union_k) {
     const int64_t resident = static_cast<int64_t>(u.ctas_per_sm) * std::max(n_sms, 1);
     t.chunk_events = o.precision == JPET_PRECISION_FIXED ? 512 : u.max_chunk;
     while (t.chunk_events > 64 &&
-           n_nonempty / t.chunk_events < (t.chunk_events > 512 ? 16 : 4) * resident)
+           n_nonempty / t.chunk_events < (t.chunk_events > 512 ? 4 : 2) * resident)
       t.chunk_events /= 2;
   }
   t.threads = o.block_threads > 0 ? o.block_threads : (rows4 ? 128 : 256);
