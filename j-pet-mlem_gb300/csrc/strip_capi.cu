@@ -697,7 +697,7 @@ const DevGeom& handle_geom(const jpet_strip* h) { return h->g; }
 const Tiling& handle_tiling(const jpet_strip* h) { return h->tiling; }
 uint64_t handle_generation(const jpet_strip* h) { return h->generation; }
 const float* handle_image(const jpet_strip* h) { return h->rho.p; }
-// kernels of one iteration
+// kernels of one iteration over the events (the clear before them not counted)
 int handle_launches(const jpet_strip* h) {
   const int parts = static_cast<int>(h->parts.size());  // with several, their records too
   return (parts > 1 ? 2 * parts : h->n_chunks > 0 ? 1 : 0) + (h->n_oversize > 0 ? 1 : 0);
