@@ -86,6 +86,7 @@ struct jpet_strip_batch {
   std::vector<RawEvents> raw;
   std::vector<jpet_strip_batch_plan> plan;
   bool fast = true;  // batch-union kernel (else row-owned)
+  int block_threads = 0;  // CTA size asked for (plan[] reports the sizes that run)
   std::vector<Captured> graphs;
   int launches = 0;  // kernels per iteration of the last graph
   std::map<TuneKey, std::tuple<int, int, int>> tune_cache;  // shape, CTA threads, tile
@@ -181,6 +182,7 @@ int jpet_strip_batch_create(int32_t n, const jpet_strip_geom* geoms, const jpet_
   }
   auto* b = new jpet_strip_batch();
   b->fast = o.variant == JPET_VARIANT_FAST;
+  b->block_threads = o.block_threads;
   b->device = o.device;
   cudaError_t e = cudaSetDevice(o.device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
@@ -295,7 +297,7 @@ int jpet_strip_batch_tune(jpet_strip_batch_t* b, int64_t max_tune_events) {
                       static_cast<int>(std::lround(gv.sigma_dl)), octave};
     const int64_t nt = std::min<int64_t>(r.n, max_tune_events);
     auto hit = b->tune_cache.find(key);
-    int best_shape = 0, best_threads = b->fast ? b->plan[i].block_threads : 128, best_tile = 0;
+    int best_shape = 0, best_threads = b->fast ? b->block_threads : 128, best_tile = 0;
     double best_ms = 1e30;
     int n_cand = 0;
     if (hit != b->tune_cache.end()) {
