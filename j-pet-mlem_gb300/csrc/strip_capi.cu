@@ -261,12 +261,20 @@ UnionLimits union_limits(const jpet_strip_opts& o, int rows, int widest) {
   return UnionLimits{kUnion96x40, 10752, 1, 1024};
 }
 
+// JPET_PRECISION_* -> the fast kernels' accumulation mode
+int precision_code(int precision) {
+  return precision == JPET_PRECISION_COMPENSATED ? kPrecisionCompensated
+         : precision == JPET_PRECISION_FP64_DEN  ? kPrecisionCompensatedDen64
+         : precision == JPET_PRECISION_FIXED     ? kPrecisionFixed
+                                                 : kPrecisionFloat;
+}
+
 // Window sizing: the largest box dimension that covers all but a tiny tail of
 // the events (the tail takes the global-memory path), then the largest square
 // tile whose window (tile + box) fits the shared-memory budget.
 void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
-                   const std::vector<int32_t>& hh, int64_t n_nonempty, int n_sms, int n_y,
-                   int n_z, int widest, double tallest, Tiling& t) {
+                   const std::vector<int32_t>& hh, int64_t n_nonempty, int n_sms,
+                   size_t most_smem, int n_y, int n_z, int widest, double tallest, Tiling& t) {
   // window pixels per array (rho, out): 12288 (~100 KiB per CTA, 2 CTAs per SM)
   // for 256-thread CTAs; 6144 (~55 KiB, 4 CTAs per SM) for the row-owned
   // kernel's 128-thread CTAs; the batch-union kernel's from its batch shape
@@ -305,12 +313,29 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
   while ((mw + tw) * (mh + th) > budget_px && (tw > 1 || th > 1)) {
     if (tw >= th && tw > 1) tw = std::max(1, tw / 2); else th = std::max(1, th / 2);
   }
-  t.tile_w = tw;
-  t.tile_h = th;
-  t.max_box_w = mw;
-  t.max_box_h = mh;
-  t.win_w = tw + mw;
-  t.win_h = th + mh;
+  auto place = [&]() {
+    t.tile_w = tw;
+    t.tile_h = th;
+    t.max_box_w = mw;
+    t.max_box_h = mh;
+    t.win_w = tw + mw;
+    t.win_h = th + mh;
+  };
+  place();
+  // The pixel budget counts a window's own columns.  A window of few columns takes
+  // up to 2.7 times as much in shared memory (fast_pitch), three times over in the
+  // compensated modes, so tall and narrow ones are cut until a CTA holds them.
+  if (union_k) {
+    t.chunk_events = u.max_chunk;
+    const int prec = precision_code(o.precision);
+    while (union_smem_bytes(t, prec) > most_smem) {
+      if (th > 8)
+        th = th / 2;
+      else
+        mh = mh * 7 / 8;
+      place();
+    }
+  }
   t.n_tiles_x = (n_z + tw - 1) / tw;
   t.n_tiles_y = (n_y + th - 1) / th;
   // events per chunk of the batch-union kernel: the largest power of two (64 to
@@ -366,14 +391,6 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
 int fast_width_shape(const DevGeom& g) {
   const int w = widest_row(g);
   return w <= 16 ? kShapeS : (w <= 24 ? kShapeM : kShapeL);
-}
-
-// JPET_PRECISION_* -> the fast kernels' accumulation mode
-int precision_code(int precision) {
-  return precision == JPET_PRECISION_COMPENSATED ? kPrecisionCompensated
-         : precision == JPET_PRECISION_FP64_DEN  ? kPrecisionCompensatedDen64
-         : precision == JPET_PRECISION_FIXED     ? kPrecisionFixed
-                                                 : kPrecisionFloat;
 }
 
 // Row records of the batch-union kernel for the chunks of part k.
@@ -465,11 +482,14 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   std::vector<int32_t> hh(hist.begin() + kHistBins, hist.end());
   int64_t nonempty = 0;
   for (int b = 1; b < kHistBins; ++b) nonempty += hw[b];
-  int n_sms = 0;
+  int n_sms = 0, most_smem = 0;
   JPET_CUDA(h, cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, h->device),
             "cudaDeviceGetAttribute");
-  choose_tiling(h->opts, hw, hh, nonempty, n_sms, h->g.n_y, h->g.n_z, widest_row(h->g),
-                3.0 * h->g.sigma_dl / h->g.pixel_height, h->tiling);
+  JPET_CUDA(h, cudaDeviceGetAttribute(&most_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin,
+                                      h->device),
+            "cudaDeviceGetAttribute");
+  choose_tiling(h->opts, hw, hh, nonempty, n_sms, static_cast<size_t>(most_smem), h->g.n_y,
+                h->g.n_z, widest_row(h->g), 3.0 * h->g.sigma_dl / h->g.pixel_height, h->tiling);
   h->tiling.fast_shape = std::max(h->tiling.fast_shape, fast_width_shape(h->g));
   {
     int64_t tail = static_cast<int64_t>(std::floor(0.001 * nonempty)), acc_h = 0;
