@@ -324,12 +324,15 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
   place();
   // The pixel budget counts a window's own columns.  A window of few columns takes
   // up to 2.7 times as much in shared memory (fast_pitch), three times over in the
-  // compensated modes, so tall and narrow ones are cut until a CTA holds them.
+  // compensated modes, so tall and narrow ones are cut until a CTA holds them; and
+  // a union row's word has 9 bits for its first column.
   if (union_k) {
     t.chunk_events = u.max_chunk;
     const int prec = precision_code(o.precision);
-    while (union_smem_bytes(t, prec) > most_smem) {
-      if (th > 8)
+    while (t.win_w > 511 || union_smem_bytes(t, prec) > most_smem) {
+      if (t.win_w > 511)
+        tw = std::max(1, tw / 2);
+      else if (th > 8)
         th = th / 2;
       else
         mh = mh * 7 / 8;

@@ -1,6 +1,6 @@
 """Windows of the batch-union kernel that are narrow and tall (their rows are padded
-in shared memory): every event set that the other kernels take, it takes, in every
-accumulation mode.
+in shared memory), or wider than a union row's word can address: every event set
+that the other kernels take, it takes, in every accumulation mode.
 
 Tolerance 1e-5 relative L2 against the kernel that evaluates every pixel in the
 reference's order, as in the other iteration tests; the fixed-point mode rounds
@@ -17,6 +17,7 @@ pytestmark = pytest.mark.gpu
 GRIDS = {
     "16 columns, boxes of 450 rows": (1000, 16, 0.3, 0.3, 3.0, 45.0, {}),
     "5 columns, boxes of 450 rows": (1000, 5, 0.3, 0.3, 3.0, 45.0, {}),
+    "tiles of 800 columns": (91, 800, 1.0, 10.0, 8.0, 20.0, dict(tile_w=2000, tile_h=1)),
 }
 PRECISIONS = [capi.PRECISION_FP32, capi.PRECISION_COMPENSATED, capi.PRECISION_FP64_DEN,
               capi.PRECISION_FIXED]
