@@ -234,6 +234,11 @@ int widest_row(const DevGeom& g) {
   return 2 * static_cast<int>(half) + 3;
 }
 
+// Pixels that the longest in-ellipse row spans: it holds at most one more.
+double row_span(const DevGeom& g) {
+  return 2.0 * 3.0 * g.sigma_z / std::sqrt(2.0) / g.pixel_width;
+}
+
 // The batch-union kernel's batch shape for events of the given box rows (99.9 %
 // of them) and widest in-ellipse row, and what a CTA of that shape can hold: the
 // pixels of its windows (the largest that still let ctas_per_sm CTAs share an
@@ -244,21 +249,29 @@ int widest_row(const DevGeom& g) {
 // events of 82 rows x 31 columns (2 mm, sigma 14 / 55), of which the 64x32
 // shape's windows and batches take one in ten, 23.0 ms there, 1.52 ms in 96x40
 // (1.64 with batches of 4 events and two CTAs per SM).
+//
+// Events whose rows no batch takes (40 columns from an even start) are rasterised
+// one by one, and its one CTA of 12 warps per SM does that slowest: 4e5 events of
+// 90 rows in the 96x40 shape / in the 64x32 one, whose windows leave them to the
+// large-box kernel, at a span of 38.2 pixels 2.2 / 9.4 ms, 39.0 4.2 / 9.5,
+// 39.2 14.0 / 9.5, 42.4 24.0 / 10.0.
+constexpr int kUnionRows = 96;          // the tallest shape's
+constexpr double kUnionSpan = 39.1;
 struct UnionLimits {
   int shape, window_px, ctas_per_sm, max_chunk;
 };
-UnionLimits union_limits(const jpet_strip_opts& o, int rows, int widest) {
-  const UnionLimits m{kUnion64x32, 6144, 2, 2048};
+constexpr UnionLimits kUnionDefault{kUnion64x32, 6144, 2, 2048};
+UnionLimits union_limits(const jpet_strip_opts& o, int rows, int widest, double span) {
   if (o.block_threads == 128) return UnionLimits{kUnion64x32n4, 6144, 4, 2048};
-  if (o.block_threads == 256) return m;
+  if (o.block_threads == 256) return kUnionDefault;
   // a batch's rows are wider than its events' by a column of alignment and, at
   // the ends of the box, by the spread of slopes in half a sort bucket
   const bool narrow = widest + 1 + rows / 8 <= 16;
   if (rows <= 30 && narrow) return UnionLimits{kUnion32x16, 3328, 4, 1024};
   if (rows <= 30 && widest <= 28) return UnionLimits{kUnion32x32, 3328, 4, 1024};
   if (rows <= 64 && narrow) return UnionLimits{kUnion64x16, 4096, 2, 1024};
-  if (rows <= 64 && widest <= 28) return m;
-  return UnionLimits{kUnion96x40, 10752, 1, 1024};
+  if (rows <= 64 && widest <= 28) return kUnionDefault;
+  return span <= kUnionSpan ? UnionLimits{kUnion96x40, 10752, 1, 1024} : kUnionDefault;
 }
 
 // JPET_PRECISION_* -> the fast kernels' accumulation mode
@@ -274,7 +287,8 @@ int precision_code(int precision) {
 // tile whose window (tile + box) fits the shared-memory budget.
 void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
                    const std::vector<int32_t>& hh, int64_t n_nonempty, int n_sms,
-                   size_t most_smem, int n_y, int n_z, int widest, double tallest, Tiling& t) {
+                   size_t most_smem, int n_y, int n_z, int widest, double span, double tallest,
+                   Tiling& t) {
   // window pixels per array (rho, out): 12288 (~100 KiB per CTA, 2 CTAs per SM)
   // for 256-thread CTAs; 6144 (~55 KiB, 4 CTAs per SM) for the row-owned
   // kernel's 128-thread CTAs; the batch-union kernel's from its batch shape
@@ -291,16 +305,33 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
     }
     return 1;
   };
-  // batch shape of the batch-union kernel
-  const UnionLimits u = union_limits(o, pct(hh, 0.999), widest);
-  t.union_shape = u.shape;
-  const int budget_px = union_k ? u.window_px : (rows4 ? 6144 : 12288);
+  // the box limits shrunk until at least an 8x8 tile fits the budget
+  auto shrink = [](int& w, int& h, int budget) {
+    while ((w + 8) * (h + 8) > budget) {
+      if (w >= h) w = w * 7 / 8; else h = h * 7 / 8;
+    }
+  };
   int mw = std::min(255, std::max(1, pct(hw, 0.99999)));
   int mh = std::min(1024, std::max(1, pct(hh, 0.99999)));
-  // shrink the box limits until at least an 8x8 tile fits
-  while ((mw + 8) * (mh + 8) > budget_px) {
-    if (mw >= mh) mw = mw * 7 / 8; else mh = mh * 7 / 8;
+  // batch shape of the batch-union kernel
+  const int rows999 = pct(hh, 0.999);
+  UnionLimits u = union_limits(o, rows999, widest, span);
+  if (u.shape == kUnion96x40 && rows999 > kUnionRows) {
+    // Boxes taller than any batch: one by one in the 64x32 shape's windows where
+    // those hold them, else in the large-box kernel, with batches of the others
+    // in the 96x40 shape.  4e5 events of up to 105 rows (2 mm, sigma 8 / 70, 62 %
+    // of them taller): 14.9 ms with the tall ones in the 96x40 shape's windows,
+    // 2.3 with them in the large-box kernel, 4.4 in the 64x32 shape.
+    int w = mw, h = mh;
+    shrink(w, h, kUnionDefault.window_px);
+    if (h > kUnionRows)
+      u = kUnionDefault;
+    else
+      mh = std::min(mh, kUnionRows);
   }
+  t.union_shape = u.shape;
+  const int budget_px = union_k ? u.window_px : (rows4 ? 6144 : 12288);
+  shrink(mw, mh, budget_px);
   int tw = o.tile_w > 0 ? o.tile_w : 0, th = o.tile_h > 0 ? o.tile_h : 0;
   if (tw == 0 || th == 0) {
     int side = 8;
@@ -386,7 +417,6 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
   t.row_stride = (mh + 1 + 7) & ~7;
   // register-cache shape of the fast kernel from the rows of 99.9% of the boxes
   // (fast_width_shape adds the widest in-ellipse row)
-  const int rows999 = pct(hh, 0.999);
   t.fast_shape = rows999 <= 32 ? kShapeS : (rows999 <= 64 ? kShapeM : kShapeL);
   t.rows_shape = kRowsShape4x1x3;
 }
@@ -492,7 +522,8 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
                                       h->device),
             "cudaDeviceGetAttribute");
   choose_tiling(h->opts, hw, hh, nonempty, n_sms, static_cast<size_t>(most_smem), h->g.n_y,
-                h->g.n_z, widest_row(h->g), 3.0 * h->g.sigma_dl / h->g.pixel_height, h->tiling);
+                h->g.n_z, widest_row(h->g), row_span(h->g), 3.0 * h->g.sigma_dl / h->g.pixel_height,
+                h->tiling);
   h->tiling.fast_shape = std::max(h->tiling.fast_shape, fast_width_shape(h->g));
   {
     int64_t tail = static_cast<int64_t>(std::floor(0.001 * nonempty)), acc_h = 0;
