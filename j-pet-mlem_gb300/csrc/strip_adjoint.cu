@@ -43,8 +43,10 @@
 // passes); 2.92 ms with two pixels a lane in packed arithmetic (rows unrolled by
 // 2; by 1, 3 and 4: 3.31, 3.04 and 3.00).
 #include <cuda_runtime.h>
+#include <math_constants.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstdint>
 
@@ -85,6 +87,13 @@ __device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
 __device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
   Pair s = two_sum(a.h, b.h);
   s.l = __fadd_rn(s.l, __fadd_rn(a.l, b.l));
+  return s;
+}
+// sum over the warp's lanes, in FP64
+__device__ __noinline__ double warp_sum_f64(float2 v) {
+  double s = static_cast<double>(v.x) + v.y;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
   return s;
 }
 // sum over the warp's lanes
@@ -299,16 +308,35 @@ __global__ void __launch_bounds__(32 * kNllWarps) nll_kernel(
         before = min(before + total, kNllCache);
       }
       const Pair d = pair_warp_sum(den);
-      const Pair a = pair_warp_sum(make_float2(dz.x * k.dipz_dsz, dz.y * k.dipz_dsz)),
-                 b = pair_warp_sum(make_float2(ddl.x * k.dipd_dsdl, ddl.y * k.dipd_dsdl));
-      if (lane == j) {
-        den_j = d;
-        dz_j = a;
-        ddl_j = b;
+      dz = make_float2(dz.x * k.dipz_dsz, dz.y * k.dipz_dsz);
+      ddl = make_float2(ddl.x * k.dipd_dsdl, ddl.y * k.dipd_dsdl);
+      const Pair a = pair_warp_sum(dz), b = pair_warp_sum(ddl);
+      float minus_inv;
+      // (the sum of the three is not finite if one of them is not)
+      if (fabsf(d.h) + fabsf(a.h) + fabsf(b.h) <= FLT_MAX && !(d.h > 0.0f && d.h < FLT_MIN)) {
+        if (lane == j) {
+          den_j = d;
+          dz_j = a;
+          ddl_j = b;
+        }
+        if (!GRAD || !(d.h > 0.0f)) continue;
+        const float i0 = __frcp_rn(d.h);
+        minus_inv = -fmaf(fmaf(-d.h, i0, 1.0f) - d.l * i0, i0, i0);
+      } else {  // beyond what FP32 holds, or a quotient of which is: all in FP64
+        const double dd = warp_sum_f64(den), ad = warp_sum_f64(dz), bd = warp_sum_f64(ddl);
+        if (lane == j) {
+          den_j.h = CUDART_NAN_F;  // done
+          if (dd > 0.0) {
+            loss -= log(dd) + log_ref;
+            gz -= ad / dd;
+            gdl -= bd / dd;
+          } else {
+            ++sk;
+          }
+        }
+        if (!GRAD || !(dd > 0.0)) continue;
+        minus_inv = -static_cast<float>(1.0 / dd);
       }
-      if (!GRAD || !(d.h > 0.0f)) continue;
-      const float i0 = __frcp_rn(d.h);
-      const float minus_inv = -fmaf(fmaf(-d.h, i0, 1.0f) - d.l * i0, i0, i0);
       before = 0;
       for (int rb = 0; rb < nrows; rb += step) {
         if (nrows > step) setup(rb);
@@ -338,7 +366,7 @@ __global__ void __launch_bounds__(32 * kNllWarps) nll_kernel(
         const double inv = 1.0 / dd;
         gz -= (static_cast<double>(dz_j.h) + static_cast<double>(dz_j.l)) * inv;
         gdl -= (static_cast<double>(ddl_j.h) + static_cast<double>(ddl_j.l)) * inv;
-      } else {
+      } else if (den_j.h == den_j.h) {  // not done
         ++sk;
       }
     }
