@@ -129,7 +129,7 @@ struct jpet_strip {
   unsigned long long table_kernel_calls = 0;
   DevBuf<unsigned long long> box_pixels;
   DevBuf<double> nll_acc;            // loss, d/dsigma_z, d/dsigma_dl
-  DevBuf<float> nll_parts;           // partial gradient images
+  DevBuf<double> nll_parts;          // partial gradient images
   DevBuf<DevCounters> counters;
 
   int64_t n_events = 0;
@@ -1065,11 +1065,11 @@ int jpet_strip_nll_grad(jpet_strip_t* h, double sigma_z, double sigma_dl, const 
   JPET_CUDA(h, h->nll_acc.alloc(4), "cudaMalloc(likelihood)");
   const size_t n_parts = d_grad_rho ? nll_grad_parts(static_cast<int64_t>(n_pix)) * n_pix : 0;
   if (d_grad_rho) JPET_CUDA(h, h->nll_parts.alloc(n_parts), "cudaMalloc(gradient)");
-  float* parts = d_grad_rho ? h->nll_parts.p : nullptr;
+  double* parts = d_grad_rho ? h->nll_parts.p : nullptr;
   const float* rho = d_rho ? d_rho : h->rho.p;
   const float* sens = d_sens ? d_sens : h->sens_point.p;
   JPET_CUDA(h, cudaMemsetAsync(h->nll_acc.p, 0, 4 * sizeof(double), s), "memset");
-  if (parts) JPET_CUDA(h, cudaMemsetAsync(parts, 0, n_parts * sizeof(float), s), "memset");
+  if (parts) JPET_CUDA(h, cudaMemsetAsync(parts, 0, n_parts * sizeof(double), s), "memset");
   const NllConst k = make_nll_const(sigma_z, sigma_dl);
   auto* skipped = reinterpret_cast<unsigned long long*>(h->nll_acc.p + 3);
   JPET_CUDA(h, launch_nll(h->g, k, h->n_sorted, h->sorted_geom.p, h->sorted_box.p,

@@ -250,10 +250,10 @@ NllConst make_nll_const(double sigma_z, double sigma_dl);
 int nll_grad_parts(int64_t n_pix);
 cudaError_t launch_nll(const DevGeom& g, const NllConst& k, int32_t n, const float4* ev_geom,
                        const short4* ev_box, const uint16_t* table, int32_t stride,
-                       const float* rho, float* parts, double* acc, unsigned long long* skipped,
+                       const float* rho, double* parts, double* acc, unsigned long long* skipped,
                        cudaStream_t s);
 // acc[0] += sum s rho; grad = s + the partial images (grad may be null)
-cudaError_t launch_nll_finish(const float* sens, const float* rho, const float* parts, float* grad,
+cudaError_t launch_nll_finish(const float* sens, const float* rho, const double* parts, float* grad,
                               double* acc, int64_t n, cudaStream_t s);
 // The image of an iteration in the compensated and fixed-point modes:
 // rho = out + aux.lo (compensated) or rho = float(aux.q 2^-22) + out (fixed;
