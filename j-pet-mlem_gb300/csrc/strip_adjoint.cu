@@ -51,6 +51,7 @@
 #include <cfloat>
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 
 #include "strip_device.cuh"
 #include "strip_internal.h"
@@ -64,6 +65,13 @@ constexpr int kNllWarps = 4;     // warps per CTA
 constexpr int kNllCache = 1536;  // kernel values kept per event
 constexpr int kNllRows = 96;     // rows of a block (an event's set-up is then kept for the
                                  // gradient pass)
+// Rows of more than kNllWide pixels (two per lane): events of several thousand
+// pixels, of which the cache would hold a few.  Their kernel keeps none and has
+// larger blocks instead, and sweeps rows of any length.  2e5 events of up to 252
+// rows x 85 columns (0.5 mm): 16.6 ms with the cache and a second loop past a
+// row's first 64 pixels, 10.4 so (inner loop unrolled by 3; by 2 10.5, by 1 11.9).
+constexpr int kNllWide = 64;
+constexpr int kNllWideRows = 256;
 
 // ---- double-float arithmetic: h + l, |l| <= ulp(h) / 2 ---------------------------------
 struct Pair {
@@ -139,24 +147,28 @@ __device__ __forceinline__ Pair half_neg_log2_1p(Pair x) {
   return pair_mul(r, Pair{ch, cl});
 }
 
+template <bool WIDE>
 struct NllWarp {
-  float4 row[kNllRows];     // prefactor exponent, d/dipz and d/dipd terms, u at column 0
-  int4 at[kNllRows];        // pixels before the row | width << 16, image index of its first
+  static constexpr int kRows = WIDE ? kNllWideRows : kNllRows;
+  float4 row[kRows];        // prefactor exponent, d/dipz and d/dipd terms, u at column 0
+  int4 at[kRows];           // pixels before the row | width << 16, image index of its first
                             // pixel, first column (float bits), unused
-  float cache[kNllCache];   // kernel values
+  float cache[WIDE ? 1 : kNllCache];  // kernel values
 };
 
 // (five CTAs per SM where the row table is read, 96 registers: 3.22 ms for 5e5 events of
 // 1763 pixels, with the four of 120 registers 3.44; the kernels that compute the
-// intervals would spill)
-template <bool GRAD, bool TABLE>
-__global__ void __launch_bounds__(32 * kNllWarps, TABLE ? 5 : 1) nll_kernel(
+// intervals would spill.  Wide rows: 10.4 ms with five, 11.6 with four, the loss
+// alone 5.9 and 5.4)
+template <bool GRAD, bool TABLE, bool WIDE>
+__global__ void __launch_bounds__(32 * kNllWarps, (WIDE ? GRAD : TABLE) ? 5 : 1) nll_kernel(
     DevGeom g, NllConst k, int32_t n, int32_t group, const float4* __restrict__ ev_geom,
     const short4* __restrict__ ev_box, const uint16_t* __restrict__ table, int32_t stride,
     const float* __restrict__ rho, double* __restrict__ parts, int32_t n_parts, int64_t n_pix,
     double* __restrict__ acc, unsigned long long* skipped) {
-  __shared__ NllWarp shared[kNllWarps];
-  NllWarp& s = shared[threadIdx.x >> 5];
+  constexpr int kRows = NllWarp<WIDE>::kRows;
+  __shared__ NllWarp<WIDE> shared[kNllWarps];
+  NllWarp<WIDE>& s = shared[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int n_warps = (gridDim.x * blockDim.x) >> 5;
@@ -200,13 +212,11 @@ __global__ void __launch_bounds__(32 * kNllWarps, TABLE ? 5 : 1) nll_kernel(
       const float pa_c = 2.0f * sec2 * sec2;     // Pa = pa_c (py^2 + R^2)
       const float qa_c = 4.0f * sec2 * tn * tn;  // Qa = qa_c py^2
       const int nrows = by1 - by0;
-      // rows per block
-      const int step = nrows <= kNllRows ? kNllRows : 32;
       int n_rows = 0, total = 0, widest = 0;  // of the block last set up: rows with pixels
       auto setup = [&](int rb) {
         n_rows = total = widest = 0;
         __syncwarp();
-        for (int r0 = rb; r0 < min(rb + step, nrows); r0 += 32) {
+        for (int r0 = rb; r0 < min(rb + kRows, nrows); r0 += 32) {
           int first = 0, w = 0;
           const int iy = by0 + r0 + lane;
           if (r0 + lane < nrows) {
@@ -260,25 +270,25 @@ __global__ void __launch_bounds__(32 * kNllWarps, TABLE ? 5 : 1) nll_kernel(
       // pixels: two pixels per lane, as many lanes per row as then fit the widest,
       // two rows in flight, lanes past a row's end along without a branch.  A
       // lane's pixels are a row's lanes apart, so that neighbouring lanes read
-      // and add to neighbouring pixels.
+      // and add to neighbouring pixels.  Wide rows: 16 lanes each, 32 pixels at a
+      // time.
       auto walk = [&](auto&& f) {
-        const int sh = widest <= 8 ? 2 : widest <= 16 ? 3 : widest <= 32 ? 4 : 5;
+        const int sh = WIDE ? 4 : widest <= 8 ? 2 : widest <= 16 ? 3 : widest <= 32 ? 4 : 5;
         const int l = lane & ((1 << sh) - 1), on = 1 << sh;
         const float2 fl = make_float2(static_cast<float>(l), static_cast<float>(l + on));
-#pragma unroll 2
+#pragma unroll(WIDE ? 1 : 2)
         for (int r0 = 0; r0 < n_rows; r0 += 32 >> sh) {
           const int r = min(r0 + (lane >> sh), n_rows - 1);
           const int4 at = s.at[r];
           const int w = r == r0 + (lane >> sh) ? at.x >> 16 : 0;
-          f(r, at, l, fl, on, l < w, l + on < w);
-        }
-        if (widest > 64) {
-          for (int r = 0; r < n_rows; ++r) {
-            const int4 at = s.at[r];
-            const int w = at.x >> 16;
-            for (int i = lane + 64; i < w; i += 64)
-              f(r, at, i, make_float2(static_cast<float>(i), static_cast<float>(i + 32)), 32,
-                true, i + 32 < w);
+          if constexpr (WIDE) {
+#pragma unroll 3
+            for (int i = 0; i < widest; i += 32) {
+              const float fi = static_cast<float>(i);
+              f(r, at, i + l, __fadd2_rn(fl, make_float2(fi, fi)), 16, i + l < w, i + l + 16 < w);
+            }
+          } else {
+            f(r, at, l, fl, on, l < w, l + on < w);
           }
         }
       };
@@ -291,7 +301,7 @@ __global__ void __launch_bounds__(32 * kNllWarps, TABLE ? 5 : 1) nll_kernel(
       };
       float2 den = make_float2(0.0f, 0.0f), dz = den, ddl = den;
       int before = 0;  // pixels of the blocks before
-      for (int rb = 0; rb < nrows; rb += step) {
+      for (int rb = 0; rb < nrows; rb += kRows) {
         setup(rb);
         walk([&](int r, const int4 at, int i, float2 fi, int on, bool in0, bool in1) {
           const float4 row = s.row[r];
@@ -307,9 +317,11 @@ __global__ void __launch_bounds__(32 * kNllWarps, TABLE ? 5 : 1) nll_kernel(
           dz = __ffma2_rn(kr, __ffma2_rn(make_float2(-u.x, -u.y), u, make_float2(row.y, row.y)),
                           dz);
           ddl = __ffma2_rn(kr, make_float2(row.z, row.z), ddl);
-          const int c = before + (at.x & 0xffff) + i;
-          if (GRAD && in0 && c < kNllCache) s.cache[c] = kv.x;
-          if (GRAD && in1 && c + on < kNllCache) s.cache[c + on] = kv.y;
+          if constexpr (GRAD && !WIDE) {
+            const int c = before + (at.x & 0xffff) + i;
+            if (in0 && c < kNllCache) s.cache[c] = kv.x;
+            if (in1 && c + on < kNllCache) s.cache[c + on] = kv.y;
+          }
         });
         before = min(before + total, kNllCache);
       }
@@ -344,12 +356,13 @@ __global__ void __launch_bounds__(32 * kNllWarps, TABLE ? 5 : 1) nll_kernel(
         minus_inv = -static_cast<float>(1.0 / dd);
       }
       before = 0;
-      for (int rb = 0; rb < nrows; rb += step) {
-        if (nrows > step) setup(rb);
+      for (int rb = 0; rb < nrows; rb += kRows) {
+        if (nrows > kRows) setup(rb);
         walk([&](int r, const int4 at, int i, float2 fi, int on, bool in0, bool in1) {
-          const int c = before + (at.x & 0xffff) + i;
-          float2 kv = make_float2(s.cache[min(c, kNllCache - 1)],
-                                  s.cache[min(c + on, kNllCache - 1)]);
+          const int c = WIDE ? kNllCache : before + (at.x & 0xffff) + i;
+          float2 kv = make_float2(0.0f, 0.0f);
+          if constexpr (!WIDE)
+            kv = make_float2(s.cache[min(c, kNllCache - 1)], s.cache[min(c + on, kNllCache - 1)]);
           if (in0 && c + on >= kNllCache) {  // not kept (either pixel, or none in the row)
             const float first = __int_as_float(at.z);
             float2 u;
@@ -459,11 +472,15 @@ cudaError_t launch_nll(const DevGeom& g, const NllConst& k, int32_t n, const flo
   const int64_t n_pix = static_cast<int64_t>(g.n_y) * g.n_z;
   const int warps = (n + group - 1) / group;
   const int blocks = std::min((warps + kNllWarps - 1) / kNllWarps, 152 * 7 * 4);
-  auto* kern = parts ? (table ? nll_kernel<true, true> : nll_kernel<true, false>)
-                     : (table ? nll_kernel<false, true> : nll_kernel<false, false>);
-  kern<<<blocks, 32 * kNllWarps, 0, s>>>(g, k, n, group, ev_geom, ev_box, table, stride, rho, parts,
-                                         nll_grad_parts(n_pix), n_pix, acc, skipped);
-  return cudaGetLastError();
+  auto go = [&](auto wide) {
+    constexpr bool W = decltype(wide)::value;
+    auto* kern = parts ? (table ? nll_kernel<true, true, W> : nll_kernel<true, false, W>)
+                       : (table ? nll_kernel<false, true, W> : nll_kernel<false, false, W>);
+    kern<<<blocks, 32 * kNllWarps, 0, s>>>(g, k, n, group, ev_geom, ev_box, table, stride, rho,
+                                           parts, nll_grad_parts(n_pix), n_pix, acc, skipped);
+    return cudaGetLastError();
+  };
+  return row_span(g) >= kNllWide - 0.1 ? go(std::true_type{}) : go(std::false_type{});
 }
 
 cudaError_t launch_nll_finish(const float* sens, const float* rho, const double* parts, float* grad,

@@ -166,6 +166,11 @@ namespace {
 
 }  // namespace
 
+// Pixels that the longest in-ellipse row spans: it holds at most one more.
+double jpet::row_span(const DevGeom& g) {
+  return 2.0 * 3.0 * g.sigma_z / std::sqrt(2.0) / g.pixel_width;
+}
+
 // Scanner<float, short> constructor arithmetic (src/2d/strip/scanner.h:50-67)
 // and GaussianKernel<float> constants (gaussian_kernel.h:27-33), in float.
 DevGeom jpet::make_dev_geom(const jpet_strip_geom& in) {
@@ -232,11 +237,6 @@ int validate_geom(const jpet_strip_geom* geom, std::string& msg) {
 int widest_row(const DevGeom& g) {
   const double half = 3.0 * g.sigma_z / std::sqrt(2.0) / g.pixel_width;
   return 2 * static_cast<int>(half) + 3;
-}
-
-// Pixels that the longest in-ellipse row spans: it holds at most one more.
-double row_span(const DevGeom& g) {
-  return 2.0 * 3.0 * g.sigma_z / std::sqrt(2.0) / g.pixel_width;
 }
 
 // The batch-union kernel's batch shape for events of the given box rows (99.9 %

@@ -104,6 +104,8 @@ enum Semantics : int32_t { kCpuReference = 0, kGpuReference = 1 };
 // Scanner<float, short> / GaussianKernel<float> constants from the C-ABI geometry
 // (strip_capi.cu).
 DevGeom make_dev_geom(const jpet_strip_geom& in);
+// Pixels that the longest in-ellipse row spans: it holds at most one more (strip_capi.cu).
+double row_span(const DevGeom& g);
 // Message returned by jpet_strip_last_error(NULL) on this thread.
 void set_call_error(const std::string& msg);
 
