@@ -35,6 +35,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/jpet_hybrid.h"
@@ -1070,6 +1071,7 @@ struct jpet_hybrid {
   Buf<uint32_t> order_keys;  // event order: sort keys (input, output)
   Buf<int32_t> order;        // event order: event indices (input, output)
   int64_t n_tabled = 0;      // events of the table iteration; order[n + n_tabled ...] the rest
+  bool shared_infos = false; // a pixel info lies in the ranges of several LORs: no table
   int table_blocks = 0;
 };
 
@@ -1160,6 +1162,27 @@ int check_geom(const jpet_hybrid_geom* g) {
   return JPET_OK;
 }
 
+// Whether a pixel info lies in the ranges of two LORs (given weights allow it): its
+// voxel weights then depend on the event's LOR, which the voxel table cannot hold.
+bool ranges_overlap(const jpet_hybrid_geom& g, int64_t n_lors) {
+  uint64_t end = 0;
+  int64_t l = 0;
+  for (; l < n_lors; ++l) {  // in LOR order, as the reference's geometries have them
+    if (g.lor_pixel_info_begin[l] == g.lor_pixel_info_end[l]) continue;
+    if (g.lor_pixel_info_begin[l] < end) break;
+    end = g.lor_pixel_info_end[l];
+  }
+  if (l == n_lors) return false;
+  std::vector<std::pair<uint64_t, uint64_t>> r;
+  for (l = 0; l < n_lors; ++l)
+    if (g.lor_pixel_info_begin[l] < g.lor_pixel_info_end[l])
+      r.emplace_back(g.lor_pixel_info_begin[l], g.lor_pixel_info_end[l]);
+  std::sort(r.begin(), r.end());
+  for (size_t k = 1; k < r.size(); ++k)
+    if (r[k].first < r[k - 1].second) return true;
+  return false;
+}
+
 // Stable radix sort of (pixel index, info index): the infos of each pixel in
 // ascending info order.  Used to check that no LOR lists a pixel twice and, for
 // the computed sensitivity, to sum each pixel's weights sequentially in that
@@ -1227,7 +1250,7 @@ int prepare_table(jpet_hybrid* h) {
   const int64_t n = h->n_events, entries = h->c.n_infos * h->c.pitch;
   h->n_tabled = 0;
   if (!h->table.p) {
-    if (entries <= 0 || (h->c.pitch & 3) != 0 || h->used_voxels < entries / 8 || n > INT32_MAX / 2) return JPET_OK;
+    if (h->shared_infos || entries <= 0 || (h->c.pitch & 3) != 0 || h->used_voxels < entries / 8 || n > INT32_MAX / 2) return JPET_OK;
     size_t free_bytes = 0, total = 0;
     HYB_CUDA(h, cudaMemGetInfo(&free_bytes, &total), "memory info");
     if (static_cast<size_t>(entries) * sizeof(float) > free_bytes / 4) return JPET_OK;
@@ -1447,6 +1470,7 @@ int jpet_hybrid_create(const jpet_hybrid_geom* g, const jpet_hybrid_opts* opts_i
   h->table_blocks = std::max(1, per_sm) * h->n_sms;
 
   const int64_t n_lors = h->c.n_lors, n = h->c.n_infos;
+  h->shared_infos = ranges_overlap(*g, n_lors);
   const int64_t n_px = static_cast<int64_t>(h->c.n_columns) * h->c.n_rows;
   const int64_t n_vox = n_px * h->c.pitch;
   CREATE_CUDA(h->seg.alloc(3 * n_lors), "cudaMalloc");
