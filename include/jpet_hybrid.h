@@ -178,7 +178,12 @@ int jpet_hybrid_get_image(jpet_hybrid_t* h, float* rho);
 int jpet_hybrid_get_sensitivity(jpet_hybrid_t* h, float* sens);
 int jpet_hybrid_get_weights(jpet_hybrid_t* h, float* weights);
 
-/* n MLEM iterations on the device (asynchronous on the handle's stream). */
+/* n MLEM iterations on the device, asynchronous on the handle's stream.  When the
+ * iterations asked for pay for it (5 of 1e6 events on a 384-detector ring, 23 of
+ * 1.7e5), the handle first makes a table of its geometry's voxel weights, 4 bytes
+ * per pixel info and plane, of at most a quarter of the free device memory, and
+ * orders the events: that call allocates and waits for the stream.  Not inside a
+ * stream capture: a captured call uses what is there. */
 int jpet_hybrid_iterate(jpet_hybrid_t* h, int n);
 /* Counters of the last iteration (synchronises). */
 int jpet_hybrid_get_counters(jpet_hybrid_t* h, jpet_hybrid_counters* out);

@@ -1071,6 +1071,8 @@ struct jpet_hybrid {
   Buf<uint32_t> order_keys;  // event order: sort keys (input, output)
   Buf<int32_t> order;        // event order: event indices (input, output)
   int64_t n_tabled = 0;      // events of the table iteration; order[n + n_tabled ...] the rest
+  double not_saved = 0.0;    // what the iterations so far would have saved (table_saves)
+  bool table_refused = false, order_refused = false;  // for the held events
   bool shared_infos = false; // a pixel info lies in the ranges of several LORs: no table
   int table_blocks = 0;
 };
@@ -1240,47 +1242,73 @@ int sort_and_check_pixels(jpet_hybrid* h, bool sum) {
   return JPET_OK;
 }
 
-// The voxel-weight table and the event order of the iterations that read it.
-// The table costs about one evaluation per entry once per handle, an iteration
-// without it one per voxel of every event; so it is made when an iteration's
-// voxels are at least an eighth of its entries (1e6 events on the 384-detector
-// ring, 200 x 200 x 125 voxels: 3.1e9 of 4.1e9, 16.5 GB made in 9 ms) and it
-// takes at most a quarter of the free memory.
-int prepare_table(jpet_hybrid* h) {
-  const int64_t n = h->n_events, entries = h->c.n_infos * h->c.pitch;
-  h->n_tabled = 0;
-  if (!h->table.p) {
-    if (h->shared_infos || entries <= 0 || (h->c.pitch & 3) != 0 || h->used_voxels < entries / 8 || n > INT32_MAX / 2) return JPET_OK;
-    size_t free_bytes = 0, total = 0;
-    HYB_CUDA(h, cudaMemGetInfo(&free_bytes, &total), "memory info");
-    if (static_cast<size_t>(entries) * sizeof(float) > free_bytes / 4) return JPET_OK;
-    if (h->info_up.alloc(h->c.n_infos) != cudaSuccess || h->table.alloc(entries) != cudaSuccess) {
-      cudaGetLastError();  // fragmented memory: the iterations compute the weights
-      return JPET_OK;
-    }
-    const int blocks = h->n_sms * 8;
-    if (h->c.n_planes_half > 1)
-      voxel_table_kernel<kMultiPlane><<<blocks, 256, 0, h->stream>>>(
-          h->seg.p, h->pix.p, h->w.p, h->ib.p, h->ie.p, h->c, h->table.p, h->info_up.p);
-    else
-      voxel_table_kernel<kSens2D><<<blocks, 256, 0, h->stream>>>(
-          h->seg.p, h->pix.p, h->w.p, h->ib.p, h->ie.p, h->c, h->table.p, h->info_up.p);
-    HYB_CUDA(h, cudaGetLastError(), "voxel table");
+// What the voxel table saves and costs, in microseconds.  An iteration saves about
+// 1.35 ns per event and 0.88 ps per voxel: 1e6 events on the 384-detector ring (3.1e9
+// voxels) 10.3 -> 6.1 ms, 5e5 on a 96-detector one (2.8e8) 2.07 -> 1.14 ms.  The table
+// (4.2e9 entries, 16.9 GB, and 5.3e7) costs 3.6 ps an entry, allocation included, and
+// with the first event order 0.3 ms and 2 ns an event; another set's order 0.08 ms
+// and 0.15 ns an event.  So the table is made by the call that asks for enough
+// iterations; calls that ask for a few at a time have to pass twice that, as they may be
+// the last.  Set-up and k iterations without the table / with one made at once, ms:
+// 1e6 events k = 3 31.4 / 34.2, k = 5 53.7 / 46.4; 1.7e5 k = 5 9.2 / 20.7, k = 20 35.6 /
+// 36.7; on the 96-detector ring 1e5 events k = 3 1.51 / 1.55, k = 5 2.35 / 2.01, 3e4 events
+// k = 5 0.90 / 1.21, k = 20 2.89 / 2.35.
+double table_saves(const jpet_hybrid* h, int64_t iterations) {
+  return static_cast<double>(iterations) * (1.35e-3 * static_cast<double>(h->n_events) +
+                                            0.88e-6 * static_cast<double>(h->used_voxels));
+}
+double table_costs(const jpet_hybrid* h) {
+  const double n = static_cast<double>(h->n_events);
+  if (h->table.p) return 80.0 + 0.15e-3 * n;
+  return 300.0 + 2e-3 * n + 3.6e-6 * static_cast<double>(h->c.n_infos * h->c.pitch);
+}
+
+// The voxel-weight table, if this handle may have it (at most a quarter of the free
+// memory).
+int make_table(jpet_hybrid* h) {
+  const int64_t entries = h->c.n_infos * h->c.pitch;
+  h->table_refused = true;
+  size_t free_bytes = 0, total = 0;
+  HYB_CUDA(h, cudaMemGetInfo(&free_bytes, &total), "memory info");
+  if (static_cast<size_t>(entries) * sizeof(float) > free_bytes / 4) return JPET_OK;
+  if (h->info_up.alloc(h->c.n_infos) != cudaSuccess || h->table.alloc(entries) != cudaSuccess) {
+    cudaGetLastError();  // fragmented memory: the iterations compute the weights
+    return JPET_OK;
   }
-  if (n > INT32_MAX / 2) return JPET_OK;
-  HYB_CUDA(h, h->order_keys.alloc(2 * n), "cudaMalloc");
-  HYB_CUDA(h, h->order.alloc(2 * n), "cudaMalloc");
-  HYB_CUDA(h, h->tab_events.alloc(n), "cudaMalloc");
-  HYB_CUDA(h, cudaMemsetAsync(h->flag.p, 0, sizeof(int), h->stream), "memset");
-  event_order_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, h->stream>>>(
-      h->ev.p, static_cast<int32_t>(n), h->order_keys.p, h->order.p, h->flag.p);
-  HYB_CUDA(h, cudaGetLastError(), "event order");
+  const int blocks = h->n_sms * 8;
+  if (h->c.n_planes_half > 1)
+    voxel_table_kernel<kMultiPlane><<<blocks, 256, 0, h->stream>>>(
+        h->seg.p, h->pix.p, h->w.p, h->ib.p, h->ie.p, h->c, h->table.p, h->info_up.p);
+  else
+    voxel_table_kernel<kSens2D><<<blocks, 256, 0, h->stream>>>(
+        h->seg.p, h->pix.p, h->w.p, h->ib.p, h->ie.p, h->c, h->table.p, h->info_up.p);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) h->table.release();
+  HYB_CUDA(h, e, "voxel table");
+  // the iterations may run on another stream
+  HYB_CUDA(h, cudaStreamSynchronize(h->stream), "synchronize");
+  h->table_refused = false;
+  return JPET_OK;
+}
+
+// The event order of the table iterations.
+int order_events(jpet_hybrid* h) {
+  const int64_t n = h->n_events;
   size_t bytes = 0;
   HYB_CUDA(h, cub::DeviceRadixSort::SortPairs(nullptr, bytes, h->order_keys.p, h->order_keys.p + n,
                                               h->order.p, h->order.p + n, static_cast<int>(n), 0,
                                               32, h->stream),
            "sort size");
-  HYB_CUDA(h, h->temp.alloc(bytes), "cudaMalloc");
+  if (h->order_keys.alloc(2 * n) != cudaSuccess || h->order.alloc(2 * n) != cudaSuccess ||
+      h->tab_events.alloc(n) != cudaSuccess || h->temp.alloc(bytes) != cudaSuccess) {
+    cudaGetLastError();  // no room: the iterations compute the weights
+    h->order_refused = true;
+    return JPET_OK;
+  }
+  HYB_CUDA(h, cudaMemsetAsync(h->flag.p, 0, sizeof(int), h->stream), "memset");
+  event_order_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, h->stream>>>(
+      h->ev.p, static_cast<int32_t>(n), h->order_keys.p, h->order.p, h->flag.p);
+  HYB_CUDA(h, cudaGetLastError(), "event order");
   HYB_CUDA(h, cub::DeviceRadixSort::SortPairs(h->temp.p, bytes, h->order_keys.p,
                                               h->order_keys.p + n, h->order.p, h->order.p + n,
                                               static_cast<int>(n), 0, 32, h->stream),
@@ -1296,14 +1324,38 @@ int prepare_table(jpet_hybrid* h) {
         h->tab_events.p);
     HYB_CUDA(h, cudaGetLastError(), "table events");
   }
-  h->n_tabled = tabled;
   // the iterations may run on another stream
   HYB_CUDA(h, cudaStreamSynchronize(h->stream), "synchronize");
+  h->n_tabled = tabled;
+  h->not_saved = 0.0;
+  h->order_refused = tabled == 0;  // nothing to gain
   return JPET_OK;
+}
+
+// Makes the table and the event order where `asked` iterations of the held events
+// pay for them (never inside a stream capture: what is there by then is used).
+int prepare_table(jpet_hybrid* h, int64_t asked) {
+  const int64_t n = h->n_events, entries = h->c.n_infos * h->c.pitch;
+  if (n == 0 || h->n_tabled > 0 || h->order_refused || h->table_refused) return JPET_OK;
+  if (h->shared_infos || entries <= 0 || (h->c.pitch & 3) != 0 || n > INT32_MAX / 2)
+    return JPET_OK;
+  const double cost = table_costs(h), saved = table_saves(h, asked);
+  if (saved < cost && h->not_saved + saved < 2.0 * cost) return JPET_OK;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  HYB_CUDA(h, cudaStreamIsCapturing(h->stream, &capture), "capture status");
+  if (capture != cudaStreamCaptureStatusNone) return JPET_OK;
+  if (!h->table.p) {
+    const int rc = make_table(h);
+    if (rc != JPET_OK || !h->table.p) return rc;
+  }
+  return order_events(h);
 }
 
 int finish_events(jpet_hybrid* h, int64_t n) {
   h->n_events = n;
+  h->n_tabled = 0;
+  if (h->table.p) h->not_saved = 0.0;  // an event order serves one set
+  h->order_refused = h->table_refused = false;
   HYB_CUDA(h, cudaMemsetAsync(h->counters.p, 0, 3 * sizeof(unsigned long long), h->stream),
            "memset");
   HYB_CUDA(h, cudaMemsetAsync(h->flag.p, 0, sizeof(int), h->stream), "memset");
@@ -1327,7 +1379,45 @@ int finish_events(jpet_hybrid* h, int64_t n) {
   }
   h->used_pixels = static_cast<int64_t>(st[0]);
   h->used_voxels = static_cast<int64_t>(st[1]);
-  return n > 0 ? prepare_table(h) : JPET_OK;
+  return JPET_OK;
+}
+
+// n iterations; ahead: the iterations that the caller knows to follow, these included.
+int iterate(jpet_hybrid* h, int n, int64_t ahead) {
+  HYB_CUDA(h, cudaSetDevice(h->device), "cudaSetDevice");
+  const int rc = prepare_table(h, ahead);
+  if (rc != JPET_OK) return rc;
+  if (h->n_tabled == 0) h->not_saved += table_saves(h, n);
+  const int64_t n_vox = static_cast<int64_t>(h->c.n_columns) * h->c.n_rows * h->c.pitch;
+  for (int it = 0; it < n; ++it) {
+    HYB_CUDA(h, cudaMemsetAsync(h->out.p, 0, n_vox * sizeof(float), h->stream), "memset");
+    HYB_CUDA(h, cudaMemsetAsync(h->counters.p + 2, 0, sizeof(unsigned long long), h->stream),
+             "memset");
+    if (h->n_events > 0) {
+      const bool multi = h->c.n_planes_half > 1, sens3d = h->c.sens_depth > 1;
+      if (h->n_tabled > 0) {
+        auto* k = multi    ? iterate_table_kernel<kMultiPlane>
+                  : sens3d ? iterate_table_kernel<kSens3D>
+                           : iterate_table_kernel<kSens2D>;
+        k<<<h->table_blocks, kTabThreads, 0, h->stream>>>(
+            h->tab_events.p, static_cast<int32_t>(h->n_tabled), h->table.p, h->info_up.p, h->seg.p,
+            h->pix.p, h->w.p, h->sens.p, h->rho.p, h->out.p, h->c, h->counters.p + 2);
+        HYB_CUDA(h, cudaGetLastError(), "iterate");
+      }
+      const int64_t rest = h->n_events - h->n_tabled;
+      if (rest > 0) {
+        auto* k = multi    ? iterate_kernel<kMultiPlane>
+                  : sens3d ? iterate_kernel<kSens3D>
+                           : iterate_kernel<kSens2D>;
+        k<<<h->iterate_blocks, kThreads, 0, h->stream>>>(
+            h->ev.p, h->n_tabled > 0 ? h->order.p + h->n_events + h->n_tabled : nullptr, rest,
+            h->seg.p, h->pix.p, h->w.p, h->sens.p, h->rho.p, h->out.p, h->c, h->counters.p + 2);
+        HYB_CUDA(h, cudaGetLastError(), "iterate");
+      }
+    }
+    std::swap(h->rho, h->out);
+  }
+  return JPET_OK;
 }
 
 int translate(jpet_hybrid* h, const jpet_hybrid_response* d_resp, int64_t n) {
@@ -1664,37 +1754,7 @@ int jpet_hybrid_get_weights(jpet_hybrid_t* h, float* w) {
 int jpet_hybrid_iterate(jpet_hybrid_t* h, int n) {
   if (!h) return fail(nullptr, JPET_ERR_ARGUMENT, "handle is NULL");
   if (n < 0) return fail(h, JPET_ERR_ARGUMENT, "negative iteration count");
-  HYB_CUDA(h, cudaSetDevice(h->device), "cudaSetDevice");
-  const int64_t n_vox = static_cast<int64_t>(h->c.n_columns) * h->c.n_rows * h->c.pitch;
-  for (int it = 0; it < n; ++it) {
-    HYB_CUDA(h, cudaMemsetAsync(h->out.p, 0, n_vox * sizeof(float), h->stream), "memset");
-    HYB_CUDA(h, cudaMemsetAsync(h->counters.p + 2, 0, sizeof(unsigned long long), h->stream),
-             "memset");
-    if (h->n_events > 0) {
-      const bool multi = h->c.n_planes_half > 1, sens3d = h->c.sens_depth > 1;
-      if (h->n_tabled > 0) {
-        auto* k = multi    ? iterate_table_kernel<kMultiPlane>
-                  : sens3d ? iterate_table_kernel<kSens3D>
-                           : iterate_table_kernel<kSens2D>;
-        k<<<h->table_blocks, kTabThreads, 0, h->stream>>>(
-            h->tab_events.p, static_cast<int32_t>(h->n_tabled), h->table.p, h->info_up.p, h->seg.p,
-            h->pix.p, h->w.p, h->sens.p, h->rho.p, h->out.p, h->c, h->counters.p + 2);
-        HYB_CUDA(h, cudaGetLastError(), "iterate");
-      }
-      const int64_t rest = h->n_events - h->n_tabled;
-      if (rest > 0) {
-        auto* k = multi    ? iterate_kernel<kMultiPlane>
-                  : sens3d ? iterate_kernel<kSens3D>
-                           : iterate_kernel<kSens2D>;
-        k<<<h->iterate_blocks, kThreads, 0, h->stream>>>(
-            h->ev.p, h->n_tabled > 0 ? h->order.p + h->n_events + h->n_tabled : nullptr, rest,
-            h->seg.p, h->pix.p, h->w.p, h->sens.p, h->rho.p, h->out.p, h->c, h->counters.p + 2);
-        HYB_CUDA(h, cudaGetLastError(), "iterate");
-      }
-    }
-    std::swap(h->rho, h->out);
-  }
-  return JPET_OK;
+  return iterate(h, n, n);
 }
 
 int jpet_hybrid_get_counters(jpet_hybrid_t* h, jpet_hybrid_counters* c) {
@@ -1758,7 +1818,8 @@ int jpet_hybrid_run(const jpet_hybrid_geom* geom, const float* sensitivity,
       const int iteration = block * n_iterations_in_block + i;
       if (iteration < start_iteration) continue;
       if (progress) progress(iteration, 0, user);
-      if ((rc = jpet_hybrid_iterate(h, 1)) != JPET_OK) return done(rc);
+      const int64_t all = static_cast<int64_t>(n_blocks) * n_iterations_in_block;
+      if ((rc = iterate(h, 1, all - iteration)) != JPET_OK) return done(rc);
       if ((rc = jpet_hybrid_synchronize(h)) != JPET_OK) return done(rc);
       if (progress) progress(iteration, 1, user);
       if (!block && i < n_iterations_in_block - 1 &&
