@@ -297,7 +297,7 @@ def gb300_arm(args, wl, world, rank, local):
     rec.synchronize()
     counters = rec.counters()
     evals_per_iter = counters["n_kernel_calls"]
-    launches_per_iter = 1 + (1 if counters["n_oversize"] > 0 else 0)
+    launches_per_iter = 2 + (1 if counters["n_oversize"] > 0 else 0)
 
     clocks = ClockSampler(local)
     if world > 1:

@@ -311,8 +311,8 @@ int jpet_strip_batch_plan_of(const jpet_strip_batch_t* b, int32_t i, jpet_strip_
 /* n iterations of every instance: one graph launch (captured on first use for
  * each n), complete on return. */
 int jpet_strip_batch_iterate(jpet_strip_batch_t* b, int32_t n);
-/* Kernels per batched iteration (of all instances) after the first iterate (0
- * before). */
+/* Kernels per batched iteration (of all instances, their clears included) after
+ * the first iterate (0 before). */
 int jpet_strip_batch_launches_per_iteration(const jpet_strip_batch_t* b);
 
 /* ---- event generator (the phantom tool's Monte Carlo on the GPU) ----------

@@ -751,10 +751,10 @@ const DevGeom& handle_geom(const jpet_strip* h) { return h->g; }
 const Tiling& handle_tiling(const jpet_strip* h) { return h->tiling; }
 uint64_t handle_generation(const jpet_strip* h) { return h->generation; }
 const float* handle_image(const jpet_strip* h) { return h->rho.p; }
-// kernels of one iteration over the events (the clear before them not counted)
+// kernels of one FP32 iteration: the clear and those over the events
 int handle_launches(const jpet_strip* h) {
   const int parts = static_cast<int>(h->parts.size());  // with several, their records too
-  return (parts > 1 ? 2 * parts : h->n_chunks > 0 ? 1 : 0) + (h->n_oversize > 0 ? 1 : 0);
+  return 1 + (parts > 1 ? 2 * parts : h->n_chunks > 0 ? 1 : 0) + (h->n_oversize > 0 ? 1 : 0);
 }
 
 // Issues n iterations on the (capturing) stream and leaves the handle as it was:
