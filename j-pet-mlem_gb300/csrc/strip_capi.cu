@@ -379,7 +379,11 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
   // and 4 or 4 and 2 chunks: 2e6 events at 2 mm 1128, 1128, 1090; 3e6 1654, 1591,
   // 1577; 2e5 190, 190, 177; 1e6 at 5 mm 225, 225, 206.  With 2 and 2: 1e6 at 3 mm
   // 527 instead of 507; with 1 below 1024: 2e5 at 3 mm 160 instead of 136.  Chunks
-  // of 32 events: 2e4 at 5 mm 31 instead of 25.  The fixed-point mode (whose
+  // of 32 events: 2e4 at 5 mm 31 instead of 25.  Below one chunk of 64 events per SM
+  // they shrink further, to 8: each is a serial chain of batches, of one or two events
+  // in sets as sparse as these (1e3 events at 5 mm 39 us with 64, 28 with 32, 23 with
+  // 16, 18.5 with 8; 5e3 31, and 27 with 32), but not in the 96x40 shape, whose
+  // windows cost more (2e3 at sigma 14 / 55 33 and 35).  The fixed-point mode (whose
   // integer window sums must stay below 2^31) takes at most 512, the other
   // kernels 512.
   t.chunk_events = 512;
@@ -389,6 +393,8 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
     while (t.chunk_events > 64 &&
            n_nonempty / t.chunk_events < (t.chunk_events > 512 ? 4 : 2) * resident)
       t.chunk_events /= 2;
+    const int least = u.shape == kUnion96x40 ? 64 : 8;
+    while (t.chunk_events > least && n_nonempty / t.chunk_events < n_sms) t.chunk_events /= 2;
   }
   t.threads = o.block_threads > 0 ? o.block_threads : (rows4 ? 128 : 256);
   // order of a tile's events: for the batch-union kernel, tan buckets of 1/4 and
