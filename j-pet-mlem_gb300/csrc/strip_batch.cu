@@ -43,6 +43,7 @@ void handle_batch_done(jpet_strip* h, int n);
 int handle_reprepare(jpet_strip* h, int raster_shape, int block_threads, int tile,
                      const float* d_zu, const float* d_zd, const float* d_dl, int64_t n);
 const char* handle_error(const jpet_strip* h);
+void handle_set_beside(jpet_strip* h, int32_t n);
 }  // namespace jpet
 
 using namespace jpet;
@@ -196,7 +197,10 @@ int jpet_strip_batch_create(int32_t n, const jpet_strip_geom* geoms, const jpet_
   b->plan.assign(n, jpet_strip_batch_plan{});
   for (int i = 0; i < n; ++i) {
     const int rc = jpet_strip_create(&geoms[i], &o, &b->h[i]);
-    if (rc == JPET_OK) jpet_strip_set_stream(b->h[i], b->stream);
+    if (rc == JPET_OK) {
+      jpet_strip_set_stream(b->h[i], b->stream);
+      handle_set_beside(b->h[i], n);
+    }
     if (rc != JPET_OK) {
       jpet_strip_batch_destroy(b);
       return rc;

@@ -137,6 +137,7 @@ struct jpet_strip {
   int32_t n_oversize = 0;
   int32_t n_chunks = 0;
   int32_t n_tiles_nonempty = 0;
+  int32_t beside = 1;  // handles that iterate together (a batch's instances)
   unsigned long long total_box_pixels = 0;
   bool events_ready = false;
   int64_t iterations_done = 0;
@@ -248,7 +249,9 @@ int widest_row(const DevGeom& g) {
 // rows x 11 columns (5 mm pixels) 552 us in the 64x32 shape, 294 in 32x16; 1e6
 // events of 82 rows x 31 columns (2 mm, sigma 14 / 55), of which the 64x32
 // shape's windows and batches take one in ten, 23.0 ms there, 1.52 ms in 96x40
-// (1.64 with batches of 4 events and two CTAs per SM).
+// (1.64 with batches of 4 events and two CTAs per SM).  For 64x32n4 the count is
+// one more than its windows and records leave room for: the chunk rule below runs
+// faster with 4 than with 3 (5e5 events at 2 mm 337 and 383 us; mostly the same).
 //
 // Events whose rows no batch takes (40 columns from an even start) are rasterised
 // one by one, and its one CTA of 12 warps per SM does that slowest: 4e5 events of
@@ -286,7 +289,7 @@ int precision_code(int precision) {
 // the events (the tail takes the global-memory path), then the largest square
 // tile whose window (tile + box) fits the shared-memory budget.
 void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
-                   const std::vector<int32_t>& hh, int64_t n_nonempty, int n_sms,
+                   const std::vector<int32_t>& hh, int64_t n_nonempty, int n_sms, int beside,
                    size_t most_smem, int n_y, int n_z, int widest, double span, double tallest,
                    Tiling& t) {
   // window pixels per array (rho, out): 12288 (~100 KiB per CTA, 2 CTAs per SM)
@@ -379,13 +382,15 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
   // and 4 or 4 and 2 chunks: 2e6 events at 2 mm 1128, 1128, 1090; 3e6 1654, 1591,
   // 1577; 2e5 190, 190, 177; 1e6 at 5 mm 225, 225, 206.  With 2 and 2: 1e6 at 3 mm
   // 527 instead of 507; with 1 below 1024: 2e5 at 3 mm 160 instead of 136.  Chunks
-  // of 32 events: 2e4 at 5 mm 31 instead of 25.  Below one chunk of 64 events per SM
-  // they shrink further, to 8: each is a serial chain of batches, of one or two events
-  // in sets as sparse as these (1e3 events at 5 mm 39 us with 64, 28 with 32, 23 with
-  // 16, 18.5 with 8; 5e3 31, and 27 with 32), but not in the 96x40 shape, whose
-  // windows cost more (2e3 at sigma 14 / 55 33 and 35).  The fixed-point mode (whose
+  // of 32 events: 2e4 at 5 mm 31 instead of 25.  The fixed-point mode (whose
   // integer window sums must stay below 2^31) takes at most 512, the other
   // kernels 512.
+  // Below one chunk of 64 events per SM they shrink further, to 8: each is a serial
+  // chain of batches, of one or two events in sets as sparse as these (1e3 events
+  // at 5 mm 39 us with 64, 28 with 32, 23 with 16, 18.5 with 8; 5e3 31, and 27 with
+  // 32).  Not in the 96x40 shape, whose windows cost more (2e3 at sigma 14 / 55 33
+  // and 35), and in a batch only below a handle's share of the SMs (10 iterations of
+  // 100 instances of 2e3 events 6.0 ms, with short chunks 8.8).
   t.chunk_events = 512;
   if (union_k) {
     const int64_t resident = static_cast<int64_t>(u.ctas_per_sm) * std::max(n_sms, 1);
@@ -394,7 +399,8 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
            n_nonempty / t.chunk_events < (t.chunk_events > 512 ? 4 : 2) * resident)
       t.chunk_events /= 2;
     const int least = u.shape == kUnion96x40 ? 64 : 8;
-    while (t.chunk_events > least && n_nonempty / t.chunk_events < n_sms) t.chunk_events /= 2;
+    while (t.chunk_events > least && n_nonempty / t.chunk_events < n_sms / beside)
+      t.chunk_events /= 2;
   }
   t.threads = o.block_threads > 0 ? o.block_threads : (rows4 ? 128 : 256);
   // order of a tile's events: for the batch-union kernel, tan buckets of 1/4 and
@@ -527,9 +533,9 @@ int prepare_events(jpet_strip* h, const float* d_zu, const float* d_zd, const fl
   JPET_CUDA(h, cudaDeviceGetAttribute(&most_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                                       h->device),
             "cudaDeviceGetAttribute");
-  choose_tiling(h->opts, hw, hh, nonempty, n_sms, static_cast<size_t>(most_smem), h->g.n_y,
-                h->g.n_z, widest_row(h->g), row_span(h->g), 3.0 * h->g.sigma_dl / h->g.pixel_height,
-                h->tiling);
+  choose_tiling(h->opts, hw, hh, nonempty, n_sms, h->beside, static_cast<size_t>(most_smem),
+                h->g.n_y, h->g.n_z, widest_row(h->g), row_span(h->g),
+                3.0 * h->g.sigma_dl / h->g.pixel_height, h->tiling);
   h->tiling.fast_shape = std::max(h->tiling.fast_shape, fast_width_shape(h->g));
   {
     int64_t tail = static_cast<int64_t>(std::floor(0.001 * nonempty)), acc_h = 0;
@@ -792,6 +798,7 @@ int handle_reprepare(jpet_strip* h, int raster_shape, int block_threads, int til
 }
 
 const char* handle_error(const jpet_strip* h) { return h->last_error.c_str(); }
+void handle_set_beside(jpet_strip* h, int32_t n) { h->beside = n; }
 
 }  // namespace jpet
 
