@@ -526,21 +526,20 @@ __device__ __forceinline__ float atan2_poly(float y, float x) {
   return copysignf(p, y);
 }
 
-// weight = GaussianKernel::normalized(...) * pixel weight * rho of voxel
-// (pixel, plane col), reconstruction.h:327-363, with the plane's terms
-// dz = z - right, lp = L/2 + z, lm = L/2 - z.  exp(-b_ic_b / 2) is
-// 2^(exp_bpq (dz - dy tan)^2 + pa.z); the frame sensitivity's
-// atan(a) - atan(b) (gaussian_kernel.h:140-150) is evaluated as
-// atan2(a - b, 1 + a b), the same angle for every a, b; a non-positive kernel
-// value gives weight 0 as in the reference (reconstruction.h:335-341).
 // The frame sensitivity's angle (gaussian_kernel.h:140-150) of a pixel with
-// rm = 1 / (R - up), rp = 1 / (R + up) at lp = L/2 + z, lm = L/2 - z.
+// rm = 1 / (R - up), rp = 1 / (R + up) at lp = L/2 + z, lm = L/2 - z:
+// atan(a) - atan(b) as atan2(a - b, 1 + a b), the same angle for every a, b.
 __device__ __forceinline__ float frame_angle(float rm, float rp, float lp, float lm) {
   const float a = fminf(lm * rm, lp * rp);
   const float b = fmaxf(-lp * rm, -lm * rp);
   return atan2_poly(a - b, fmaf(a, b, 1.0f));
 }
 
+// weight = GaussianKernel::normalized(...) * pixel weight * rho of voxel
+// (pixel, plane col), reconstruction.h:327-363, with the plane's terms
+// dz = z - right, lp = L/2 + z, lm = L/2 - z.  exp(-b_ic_b / 2) is
+// 2^(exp_bpq (dz - dy tan)^2 + pa.z); a non-positive kernel value gives weight 0
+// as in the reference (reconstruction.h:335-341).
 template <int SM>
 __device__ __forceinline__ float plane_weight(const HybConst& c, const EvC& e, const float4 pa,
                                               const float4 pb, float dz, float lp, float lm,

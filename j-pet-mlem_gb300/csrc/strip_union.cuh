@@ -225,8 +225,6 @@ constexpr int kXChain = 2;  // split, and K' stepped along the row by R8
 // that the pairs of the jc tables stay aligned.
 __device__ __forceinline__ int u_centre(int wu) { return (wu >> 1) & ~1; }
 
-// Union rows and per-(event, row) records of one batch: 4 / RS threads per
-
 // A batch's records (zero, so no pixel, for events past its count and rows past
 // its union) and union rows.  rec: the batch's first event's records.
 template <class C, class DT>

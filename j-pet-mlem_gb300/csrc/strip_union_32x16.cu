@@ -1,5 +1,5 @@
 // Batch-union iteration (strip_union.cuh) for batches of up to
-// 32 rows x 16 columns: 5 mm pixels at sigma 10 / 42.
+// 32 rows x 16 columns: boxes of up to 30 rows with rows of up to about 11 pixels.
 #include "strip_union.cuh"
 
 namespace jpet {

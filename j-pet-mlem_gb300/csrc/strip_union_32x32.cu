@@ -1,5 +1,5 @@
 // Batch-union iteration (strip_union.cuh) for batches of up to
-// 32 rows x 32 columns: wide rows of short boxes (4 mm pixels at sigma_z 14).
+// 32 rows x 32 columns: boxes of up to 30 rows with rows of up to 28 pixels.
 #include "strip_union.cuh"
 
 namespace jpet {

@@ -1,5 +1,5 @@
 // Batch-union iteration (strip_union.cuh) for batches of up to
-// 64 rows x 16 columns: narrow rows of tall boxes (4 mm pixels at sigma 7 / 44).
+// 64 rows x 16 columns: boxes of up to 64 rows with rows of up to about 9 pixels.
 #include "strip_union.cuh"
 
 namespace jpet {

@@ -1,5 +1,6 @@
 // Batch-union iteration (strip_union.cuh) for batches of up to
-// 64 rows x 32 columns, 256 threads: 2 mm pixels at sigma 10 / 42, 1 mm at 5 / 20.
+// 64 rows x 32 columns, 256 threads: boxes of up to 64 rows with rows of up to 28
+// pixels, and events that no batch takes.
 #include "strip_union.cuh"
 
 namespace jpet {

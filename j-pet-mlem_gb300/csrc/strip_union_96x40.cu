@@ -1,5 +1,5 @@
 // Batch-union iteration (strip_union.cuh) for batches of up to
-// 96 rows x 40 columns: 2 mm pixels at sigma 14 / 60.
+// 96 rows x 40 columns: boxes of up to 96 rows with rows of up to 39 pixels.
 #include "strip_union.cuh"
 
 namespace jpet {
