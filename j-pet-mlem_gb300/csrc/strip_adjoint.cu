@@ -30,8 +30,8 @@
 // kernel values are kept for the gradient pass, which adds them with FP64
 // reductions to one of a few partial images (nll_finish_kernel sums those): in
 // float images, eight of them, the sum of 5e6 events of a point source was 4e-5 off
-// and that of 5e5 events of 1763 pixels 2.0e-7, for 18.9 instead of 22.0 ms and
-// 2.91 instead of 3.22 ms.
+// and that of 5e5 events of 1763 pixels 2.0e-7, for 18.9 instead of 21.8 ms and
+// 2.91 instead of 2.97 ms.
 //
 // This GPU's FP64 pipe is a sixty-fourth of its FP32 one, so FP64 is left where
 // one lane's instruction serves one event: a warp takes `group` events, lane j
@@ -69,7 +69,8 @@ constexpr int kNllRows = 96;     // rows of a block (an event's set-up is then k
 // pixels, of which the cache would hold a few.  Their kernel keeps none and has
 // larger blocks instead, and sweeps rows of any length.  2e5 events of up to 252
 // rows x 85 columns (0.5 mm): 16.6 ms with the cache and a second loop past a
-// row's first 64 pixels, 10.4 so (inner loop unrolled by 3; by 2 10.5, by 1 11.9).
+// row's first 64 pixels, 9.6 so (inner loop unrolled by 3; 10.4 before additions were
+// spared the conversion, where by 2 took 10.5 and by 1 11.9).
 constexpr int kNllWide = 64;
 constexpr int kNllWideRows = 256;
 
@@ -98,6 +99,21 @@ __device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
   Pair s = two_sum(a.h, b.h);
   s.l = __fadd_rn(s.l, __fadd_rn(a.l, b.l));
   return s;
+}
+// Adds v, a negative normal float unless ANY, to a double.  The conversion instruction
+// runs on the FP64 pipe, which one per addition kept 67 % busy (5e5 events of 1763
+// pixels 3.22 ms), so the double is made of the float's bits (2.97).  Smaller values
+// than normal ones are left out, as float reductions leave them.
+template <bool ANY>
+__device__ __forceinline__ void add_negative(double* p, float v, bool in) {
+  if (ANY) {
+    if (in) atomicAdd(p, static_cast<double>(v));
+  } else {
+    const uint32_t b = __float_as_uint(v);
+    if (in && v <= -FLT_MIN)
+      atomicAdd(p, __hiloint2double(static_cast<int>((b >> 3) + 0xA8000000u),
+                                    static_cast<int>(b << 29)));
+  }
 }
 // sum over the warp's lanes, in FP64
 __device__ __noinline__ double warp_sum_f64(float2 v) {
@@ -156,10 +172,10 @@ struct NllWarp {
   float cache[WIDE ? 1 : kNllCache];  // kernel values
 };
 
-// (five CTAs per SM where the row table is read, 96 registers: 3.22 ms for 5e5 events of
-// 1763 pixels, with the four of 120 registers 3.44; the kernels that compute the
-// intervals would spill.  Wide rows: 10.4 ms with five, 11.6 with four, the loss
-// alone 5.9 and 5.4)
+// (five CTAs per SM where the row table is read, 96 registers: for 5e5 events of 1763
+// pixels 3.22 ms against 3.44 with the four of 120 registers; the kernels that compute
+// the intervals would spill.  Wide rows 10.5 ms against 11.6, but the loss alone 5.9
+// against 5.4.  All four measured with the conversion in add_negative)
 template <bool GRAD, bool TABLE, bool WIDE>
 __global__ void __launch_bounds__(32 * kNllWarps, (WIDE ? GRAD : TABLE) ? 5 : 1) nll_kernel(
     DevGeom g, NllConst k, int32_t n, int32_t group, const float4* __restrict__ ev_geom,
@@ -330,6 +346,7 @@ __global__ void __launch_bounds__(32 * kNllWarps, (WIDE ? GRAD : TABLE) ? 5 : 1)
       ddl = make_float2(ddl.x * k.dipd_dsdl, ddl.y * k.dipd_dsdl);
       const Pair a = pair_warp_sum(dz), b = pair_warp_sum(ddl);
       float minus_inv;
+      bool any = false;  // -K / den may be any float
       // (the sum of the three is not finite if one of them is not)
       if (fabsf(d.h) + fabsf(a.h) + fabsf(b.h) <= FLT_MAX && !(d.h > 0.0f && d.h < FLT_MIN)) {
         if (lane == j) {
@@ -354,27 +371,35 @@ __global__ void __launch_bounds__(32 * kNllWarps, (WIDE ? GRAD : TABLE) ? 5 : 1)
         }
         if (!GRAD || !(dd > 0.0)) continue;
         minus_inv = -static_cast<float>(1.0 / dd);
+        any = true;
       }
-      before = 0;
-      for (int rb = 0; rb < nrows; rb += kRows) {
-        if (nrows > kRows) setup(rb);
-        walk([&](int r, const int4 at, int i, float2 fi, int on, bool in0, bool in1) {
-          const int c = WIDE ? kNllCache : before + (at.x & 0xffff) + i;
-          float2 kv = make_float2(0.0f, 0.0f);
-          if constexpr (!WIDE)
-            kv = make_float2(s.cache[min(c, kNllCache - 1)], s.cache[min(c + on, kNllCache - 1)]);
-          if (in0 && c + on >= kNllCache) {  // not kept (either pixel, or none in the row)
-            const float first = __int_as_float(at.z);
-            float2 u;
-            const float2 v = value(s.row[r], __fadd2_rn(make_float2(first, first), fi), u);
-            if (c >= kNllCache) kv.x = v.x;
-            kv.y = v.y;
-          }
-          if (in0) atomicAdd(&grad[at.y + i], static_cast<double>(kv.x * minus_inv));
-          if (in1) atomicAdd(&grad[at.y + i + on], static_cast<double>(kv.y * minus_inv));
-        });
-        before = min(before + total, kNllCache);
-      }
+      auto gradient = [&](auto any_float) {
+        constexpr bool ANY = decltype(any_float)::value;
+        before = 0;
+        for (int rb = 0; rb < nrows; rb += kRows) {
+          if (nrows > kRows) setup(rb);
+          walk([&](int r, const int4 at, int i, float2 fi, int on, bool in0, bool in1) {
+            const int c = WIDE ? kNllCache : before + (at.x & 0xffff) + i;
+            float2 kv = make_float2(0.0f, 0.0f);
+            if constexpr (!WIDE)
+              kv = make_float2(s.cache[min(c, kNllCache - 1)], s.cache[min(c + on, kNllCache - 1)]);
+            if (in0 && c + on >= kNllCache) {  // not kept (either pixel, or none in the row)
+              const float first = __int_as_float(at.z);
+              float2 u;
+              const float2 v = value(s.row[r], __fadd2_rn(make_float2(first, first), fi), u);
+              if (c >= kNllCache) kv.x = v.x;
+              kv.y = v.y;
+            }
+            add_negative<ANY>(&grad[at.y + i], kv.x * minus_inv, in0);
+            add_negative<ANY>(&grad[at.y + i + on], kv.y * minus_inv, in1);
+          });
+          before = min(before + total, kNllCache);
+        }
+      };
+      if (any)
+        gradient(std::true_type{});
+      else
+        gradient(std::false_type{});
       __syncwarp();  // the next event's set-up overwrites the rows
     }
     if (lane < cnt) {
