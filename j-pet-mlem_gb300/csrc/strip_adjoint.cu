@@ -30,7 +30,7 @@
 // kernel values are kept for the gradient pass, which adds them with FP64
 // reductions to one of a few partial images (nll_finish_kernel sums those): in
 // float images, eight of them, the sum of 5e6 events of a point source was 4e-5 off
-// and that of 5e5 events of 1763 pixels 2.0e-7, for 18.9 instead of 21.8 ms and
+// and that of 5e5 events of 1763 pixels 2.0e-7, for 18.9 instead of 19.7 ms and
 // 2.91 instead of 2.97 ms.
 //
 // This GPU's FP64 pipe is a sixty-fourth of its FP32 one, so FP64 is left where
@@ -479,16 +479,20 @@ NllConst make_nll_const(double sigma_z, double sigma_dl) {
 }
 
 // Partial gradient images: where many events share a pixel, additions to one image
-// wait for each other (5e6 events of a point source at 2 mm: 36.6 ms with one image,
-// 28.1 with two, 24.0 with four); four images of up to 2^20 pixels, 32 MB, stay in L2.
-int nll_grad_parts(int64_t n_pix) {
-  return n_pix <= (int64_t(1) << 20) ? 4 : n_pix <= (int64_t(1) << 21) ? 2 : 1;
+// wait for each other (5e6 events of a point source at 2 mm, widths 10 / 42 and 14 / 55: 35
+// and 54 ms with one image, 21.5 and 35 with 4, 19.8 and 35 with 8, 19.7 and 26.7 with 16, as
+// with 32); sets of fewer events do with 4, and so do their clearing and adding up.
+// Together they stay in L2: 32 MB.
+int nll_grad_parts(int64_t n_pix, int64_t n_events) {
+  int parts = n_events >= (int64_t(1) << 20) ? 16 : 4;
+  while (parts > 1 && parts * n_pix > (int64_t(1) << 22)) parts /= 2;
+  return parts;
 }
 
 cudaError_t launch_nll(const DevGeom& g, const NllConst& k, int32_t n, const float4* ev_geom,
                        const short4* ev_box, const uint16_t* table, int32_t stride,
-                       const float* rho, double* parts, double* acc, unsigned long long* skipped,
-                       cudaStream_t s) {
+                       const float* rho, double* parts, int32_t n_parts, double* acc,
+                       unsigned long long* skipped, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   // events per warp: up to 32, so that the FP64 of a lane serves an event, but
   // enough warps to fill the SMs (152 x 28)
@@ -502,15 +506,16 @@ cudaError_t launch_nll(const DevGeom& g, const NllConst& k, int32_t n, const flo
     auto* kern = parts ? (table ? nll_kernel<true, true, W> : nll_kernel<true, false, W>)
                        : (table ? nll_kernel<false, true, W> : nll_kernel<false, false, W>);
     kern<<<blocks, 32 * kNllWarps, 0, s>>>(g, k, n, group, ev_geom, ev_box, table, stride, rho,
-                                           parts, nll_grad_parts(n_pix), n_pix, acc, skipped);
+                                           parts, n_parts, n_pix, acc, skipped);
     return cudaGetLastError();
   };
   return row_span(g) >= kNllWide - 0.1 ? go(std::true_type{}) : go(std::false_type{});
 }
 
-cudaError_t launch_nll_finish(const float* sens, const float* rho, const double* parts, float* grad,
-                              double* acc, int64_t n, cudaStream_t s) {
-  nll_finish_kernel<<<152 * 4, 256, 0, s>>>(sens, rho, parts, nll_grad_parts(n), grad, acc, n);
+cudaError_t launch_nll_finish(const float* sens, const float* rho, const double* parts,
+                              int32_t n_parts, float* grad, double* acc, int64_t n,
+                              cudaStream_t s) {
+  nll_finish_kernel<<<152 * 4, 256, 0, s>>>(sens, rho, parts, n_parts, grad, acc, n);
   return cudaGetLastError();
 }
 

@@ -1076,23 +1076,23 @@ int jpet_strip_nll_grad(jpet_strip_t* h, double sigma_z, double sigma_dl, const 
   cudaStream_t s = h->stream;
   const size_t n_pix = static_cast<size_t>(h->g.n_y) * h->g.n_z;
   JPET_CUDA(h, h->nll_acc.alloc(4), "cudaMalloc(likelihood)");
-  const size_t n_parts = d_grad_rho ? nll_grad_parts(static_cast<int64_t>(n_pix)) * n_pix : 0;
-  if (d_grad_rho) JPET_CUDA(h, h->nll_parts.alloc(n_parts), "cudaMalloc(gradient)");
+  const int32_t n_parts = nll_grad_parts(static_cast<int64_t>(n_pix), h->n_events);
+  if (d_grad_rho) JPET_CUDA(h, h->nll_parts.alloc(n_parts * n_pix), "cudaMalloc(gradient)");
   double* parts = d_grad_rho ? h->nll_parts.p : nullptr;
   const float* rho = d_rho ? d_rho : h->rho.p;
   const float* sens = d_sens ? d_sens : h->sens_point.p;
   JPET_CUDA(h, cudaMemsetAsync(h->nll_acc.p, 0, 4 * sizeof(double), s), "memset");
-  if (parts) JPET_CUDA(h, cudaMemsetAsync(parts, 0, n_parts * sizeof(double), s), "memset");
+  if (parts) JPET_CUDA(h, cudaMemsetAsync(parts, 0, n_parts * n_pix * sizeof(double), s), "memset");
   const NllConst k = make_nll_const(sigma_z, sigma_dl);
   auto* skipped = reinterpret_cast<unsigned long long*>(h->nll_acc.p + 3);
   JPET_CUDA(h, launch_nll(h->g, k, h->n_sorted, h->sorted_geom.p, h->sorted_box.p,
                           h->use_fast ? h->row_table.p : nullptr, h->tiling.row_stride, rho, parts,
-                          h->nll_acc.p, skipped, s),
+                          n_parts, h->nll_acc.p, skipped, s),
             "likelihood kernel launch");
   JPET_CUDA(h, launch_nll(h->g, k, h->n_oversize, h->over_geom.p, h->over_box.p, nullptr, 0, rho,
-                          parts, h->nll_acc.p, skipped, s),
+                          parts, n_parts, h->nll_acc.p, skipped, s),
             "likelihood kernel launch");
-  JPET_CUDA(h, launch_nll_finish(sens, rho, parts, d_grad_rho, h->nll_acc.p,
+  JPET_CUDA(h, launch_nll_finish(sens, rho, parts, n_parts, d_grad_rho, h->nll_acc.p,
                                  static_cast<int64_t>(n_pix), s),
             "likelihood finish launch");
   double host[4];

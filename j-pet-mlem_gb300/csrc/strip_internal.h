@@ -246,17 +246,18 @@ struct NllConst {
 };
 NllConst make_nll_const(double sigma_z, double sigma_dl);
 // acc[0] -= sum_e log den_e, acc[1..2] -= sum_e (d den_e / d sigma) / den_e,
-// and, unless parts is NULL, -sum_e K_e / den_e into nll_grad_parts(n_pix) partial
-// images (cleared by the caller); table (with its stride): the events' row table
+// and, unless parts is NULL, -sum_e K_e / den_e into n_parts partial images
+// (cleared by the caller); table (with its stride): the events' row table
 // (launch_row_tables), or NULL
-int nll_grad_parts(int64_t n_pix);
+int nll_grad_parts(int64_t n_pix, int64_t n_events);
 cudaError_t launch_nll(const DevGeom& g, const NllConst& k, int32_t n, const float4* ev_geom,
                        const short4* ev_box, const uint16_t* table, int32_t stride,
-                       const float* rho, double* parts, double* acc, unsigned long long* skipped,
-                       cudaStream_t s);
+                       const float* rho, double* parts, int32_t n_parts, double* acc,
+                       unsigned long long* skipped, cudaStream_t s);
 // acc[0] += sum s rho; grad = s + the partial images (grad may be null)
-cudaError_t launch_nll_finish(const float* sens, const float* rho, const double* parts, float* grad,
-                              double* acc, int64_t n, cudaStream_t s);
+cudaError_t launch_nll_finish(const float* sens, const float* rho, const double* parts,
+                              int32_t n_parts, float* grad, double* acc, int64_t n,
+                              cudaStream_t s);
 // The image of an iteration in the compensated and fixed-point modes:
 // rho = out + aux.lo (compensated) or rho = float(aux.q 2^-22) + out (fixed;
 // out holds the contributions of events taken by the reference-order paths).
