@@ -852,8 +852,9 @@ def hybrid_summary(local, n_events=10_000_000, steps=5, warmup=2, cpu_seconds=10
         r.synchronize()
         set_s = time.perf_counter() - t0
         st = r.statistics()
-        for _ in range(warmup):
-            r(1)
+        # asks for as many iterations as the timed call, so that the handle makes its
+        # table of voxel weights for both or for neither
+        r(max(warmup, steps))
         r.synchronize()
         a = torch.cuda.Event(enable_timing=True)
         b = torch.cuda.Event(enable_timing=True)
