@@ -41,8 +41,8 @@
 // FMA).  5e5 events of 1763 pixels (2 mm, support 14 / 55): 8.0 ms with FP64 row
 // terms and per-event FP64 on one lane (FP64 pipe 70-81 % busy) and float
 // atomics on windows in shared memory, 3.65 ms with all that (FP64 pipe 3 %), bound
-// by instruction issue (63 % of the slots, 52 instructions a pixel for both
-// passes); 2.92 ms with two pixels a lane in packed arithmetic (rows unrolled by
+// by instruction issue (63 % of the slots, 52 instructions a pixel in either
+// pass); 2.92 ms with two pixels a lane in packed arithmetic (rows unrolled by
 // 2; by 1, 3 and 4: 3.31, 3.04 and 3.00).
 #include <cuda_runtime.h>
 #include <math_constants.h>
