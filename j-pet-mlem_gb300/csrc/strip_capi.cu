@@ -319,7 +319,7 @@ void choose_tiling(const jpet_strip_opts& o, const std::vector<int32_t>& hw,
   // batch shape of the batch-union kernel
   const int rows999 = pct(hh, 0.999);
   UnionLimits u = union_limits(o, rows999, widest, span);
-  if (u.shape == kUnion96x40 && rows999 > kUnionRows) {
+  if (union_k && u.shape == kUnion96x40 && rows999 > kUnionRows) {
     // Boxes taller than any batch: one by one in the 64x32 shape's windows where
     // those hold them, else in the large-box kernel, with batches of the others
     // in the 96x40 shape.  4e5 events of up to 105 rows (2 mm, sigma 8 / 70, 62 %
