@@ -87,9 +87,9 @@ typedef struct jpet_strip_geom {
                                 bytes written at set-up (0.5 to 1.5 KB per event, above
                                 1 GB at most half of the free memory: what does not fit is
                                 written again part by part in every iteration).  An image
-                                pixel that is infinite or not a number takes out all events
-                                of a batch whose union holds it (the other variants: the
-                                events whose ellipse does) */
+                                pixel that is infinite or not a number can take out all
+                                events of a batch whose union holds it (the other variants:
+                                the events whose ellipse does) */
 #define JPET_VARIANT_EXACT 1 /* every pixel evaluated in the reference's operation order */
 #define JPET_VARIANT_WARP 2  /* one warp per event, shared-memory atomics */
 #define JPET_VARIANT_ROWS 3  /* row-owned kernel: image rows owned by warps, one event at a
